@@ -195,7 +195,7 @@ def _model(name, dtype):
 
 class _Live:
     """A program's open requests and what its next step brings; they are closed with it."""
-    count = 0
+    count = steps = 0
 
     def __init__(self, model):
         self.model, self.engine, self.requests, self.entries = model, model.engine, [], []
@@ -249,11 +249,11 @@ def prepare(case, seed):
         return {"case": case, "model": model, "tokens": tokens}
     live = _Live(model)
     jobs = [[live.open(), past, 0] for past, _ in tokens]
-    # contexts are fed as a server feeds them, in portions under a budget; the portions' lengths differ, as prompts' do
-    turn = int(seed) % 1000
+    # contexts are fed as a server feeds them, in portions under a budget; the portions' lengths differ, as prompts' do (the
+    # engine keeps a few shapes of step that recur; these are not to be among them)
     while any(at < len(past) for _, past, at in jobs):
-        turn += 1
-        room, batch = 2048 + turn % 997, []
+        _Live.steps += 1
+        room, batch = 2048 + _Live.steps % 997, []
         for job in jobs:
             n = min(room, len(job[1]) - job[2])
             if n > 0:
