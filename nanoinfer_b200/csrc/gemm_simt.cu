@@ -1,6 +1,5 @@
-// The general matrix product of the engine: C[M,N] = A[M,K] . W[N,K]^T (+ bias), any M, N, K,
-// 32-bit accumulation on the CUDA cores. It is the true 32-bit path (no reduced-precision matrix
-// mode) and the fallback of the bfloat16 path for shapes the tensor-core kernel refuses.
+// The general matrix product of the bfloat16 path: C[M,N] = A[M,K] . W[N,K]^T (+ bias), any M, N, K, 32-bit accumulation
+// on the CUDA cores. It takes the shapes that the tensor-core kernels refuse (the 32-bit path has gemm_f32.cu).
 //
 // Every output element is accumulated by one thread over k = 0..K-1 in ascending order, so a row's
 // result does not depend on how many other rows the call has (the reference guarantees the same:
@@ -128,16 +127,14 @@ static int launch_simt(const void* A, const void* W, const float* bias, void* ou
 // A [M, K] with row stride lda; W [N, K] (SWIGLU: [2N, K], gate rows then up rows); out [M, N] with
 // row stride ldo. epi: 0 store, 1 add into float, 2 store float, 3 swiglu, 5 the gated form with the constants glu, 6 geglu.
 NIB_API int nib_gemm_simt(const void* A, const void* W, const float* bias, void* out, int M, int N, int K,
-                          int lda, int ldo, int epi, int dtype, const NibGlu* glu, cudaStream_t stream) {
+                          int lda, int ldo, int epi, const NibGlu* glu, cudaStream_t stream) {
     NIB_REQUIRE(M >= 0 && N > 0 && K > 0 && lda >= K && ldo >= N, "gemm: bad sizes M=%d N=%d K=%d lda=%d ldo=%d", M, N, K, lda, ldo);
     NIB_REQUIRE(!epi_dual(epi) || bias == nullptr, "gemm: the gated epilogues take no bias");
     NIB_REQUIRE(epi != EPI_GLU || glu != nullptr, "gemm: the gated epilogue needs its constants");
     const NibGlu constants = glu != nullptr ? *glu : NibGlu{};
     if (M == 0) return 0;
     NIB_REQUIRE(ceil_div(M, 64) <= 65535, "gemm: M=%d is too large for one launch", M);
-    if (dtype == NIB_F32) return launch_simt<float>(A, W, bias, out, M, N, K, lda, ldo, epi, constants, stream);
-    if (dtype == NIB_BF16) return launch_simt<__nv_bfloat16>(A, W, bias, out, M, N, K, lda, ldo, epi, constants, stream);
-    NIB_REQUIRE(false, "gemm: unknown dtype %d", dtype);
+    return launch_simt<__nv_bfloat16>(A, W, bias, out, M, N, K, lda, ldo, epi, constants, stream);
 }
 
 // ---------------------------------------------------------------------------------- block-diagonal product, few tokens

@@ -117,7 +117,7 @@ class Kernels:
         except OSError as e:
             raise KernelError(f"cannot load the kernel library {lib_path}: {e}") from e
         self._lib.nib_last_error.restype = ctypes.c_char_p
-        for name in ("nib_embed", "nib_rmsnorm", "nib_rope_store", "nib_gemm_simt", "nib_attention_generic",
+        for name in ("nib_embed", "nib_rmsnorm", "nib_rope_store", "nib_gemm_simt", "nib_gemm_f32", "nib_attention_generic",
                      "nib_gemm_smallm", "nib_gemm_smallm_supported", "nib_gemm_tc", "nib_gemm_tc_splitk",
                      "nib_gemm_tc_pair", "nib_gemm_tc_supported", "nib_gemm_tc_error", "nib_attention_mma_supported",
                      "nib_attention_prefill_mma", "nib_attention_decode_mma", "nib_attention_decode_tma",
@@ -399,9 +399,9 @@ class Kernels:
                 _ptr(self._ws_scratch), _ptr(self._ws_counters), c_longlong(self._ws_scratch.numel()),
                 c_longlong(self._ws_counters.numel()), glu, self._stream()), "linear (tensor cores)")
             return
-        self._check(self._lib.nib_gemm_simt(_ptr(a), _ptr(w), _ptr(bias32), _ptr(out), c_int(m), c_int(n), c_int(k),
-                                            c_int(a.stride(0)), c_int(out.stride(0)), c_int(epi), c_int(_DT[a.dtype]), glu,
-                                            self._stream()), "linear")
+        product = self._lib.nib_gemm_simt if a.dtype == torch.bfloat16 else self._lib.nib_gemm_f32
+        self._check(product(_ptr(a), _ptr(w), _ptr(bias32), _ptr(out), c_int(m), c_int(n), c_int(k), c_int(a.stride(0)),
+                            c_int(out.stride(0)), c_int(epi), glu, self._stream()), "linear")
 
     def gemm_tc_error(self) -> int:
         """The error word of the tensor-core GEMM's bounded waits (0 = none); synchronises and clears it."""
@@ -548,7 +548,7 @@ class Kernels:
                 _ptr(qkv), c_int(qkv.stride(0)), _ptr(out), _ptr(ctx.positions), _ptr(ctx.req_index), _ptr(block_table),
                 c_int(bt_stride), c_int(page_size), _ptr(k_pages), _ptr(v_pages), c_int(num_pages),
                 c_int(m), c_int(heads), c_int(kv_heads), c_int(head_dim), c_float(scale), c_int(window),
-                c_int(_DT[qkv.dtype]), self._stream()), "attention")
+                c_int(_DT[qkv.dtype]), c_int(max(ctx.host.ctx_lens, default=0)), self._stream()), "attention")
             return
         q_lens, ctx_lens = ctx.host.q_lens, ctx.host.ctx_lens
         n_req = len(q_lens)

@@ -781,3 +781,66 @@ def test_qkv_projection_with_rotation_and_cache_write(K, heads, kv_heads, hd, ro
     keep = torch.ones(pages, dtype=torch.bool, device="cuda")
     keep[page_of[1]] = False
     assert torch.equal(kp3[keep], kr[keep]) and not kp3[page_of[1]].any()
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 5, 8, 9, 16, 17, 64, 65, 300])
+@pytest.mark.parametrize("n,k", [(8, 4), (9, 127), (64, 128), (65, 129), (100, 1280), (40, 1284), (33, 2600), (4736, 256), (24, 4864), (16, 18944)])
+def test_f32_product_edges(K, m, n, k):
+    """The 32-bit products at the edges of their chunks (128 of k), tiles (8, 16 and 64 rows), clusters and shared memory, also
+    with operands that are not 16-byte aligned: values, what lies behind them, and rows that are the same bits whatever the
+    number of rows."""
+    a_flat, w_flat = rnd((m * k + 1,), torch.float32, 70), rnd((n * k + 1,), torch.float32, 71, scale=0.05)
+    bias = rnd((n,), torch.float32, 72)
+    for off in (0, 1):
+        a, w = a_flat[off:off + m * k].view(m, k), w_flat[off:off + n * k].view(n, k)
+        want = _ref_linear_f64(a, w, bias)
+        room = torch.full((m * n + 70,), 7.0, device="cuda")
+        out = room[:m * n].view(m, n)
+        K.linear(a, w, bias, out, "f32")
+        assert_close(out, want, torch.float32, f"offset {off}")
+        assert (room[m * n:] == 7.0).all()
+        some = torch.empty(min(m, 2), n, device="cuda")
+        K.linear(a[m - some.shape[0]:], w, bias, some, "f32")
+        assert torch.equal(some, out[m - some.shape[0]:])
+        res = rnd((m, n), torch.float32, 73)
+        acc = res.clone()
+        K.linear(a, w, None, acc, "add")
+        assert_close(acc, res.double() + _ref_linear_f64(a, w, None), torch.float32, f"add, offset {off}")
+
+
+@pytest.mark.parametrize("m", [1, 4, 7, 16, 17, 130])
+@pytest.mark.parametrize("inter,k", [(3, 96), (8, 896), (70, 1300), (1500, 130), (20, 6000)])
+def test_f32_gated_product_edges(K, m, inter, k):
+    a, w = rnd((m, k), torch.float32, 74), rnd((2 * inter, k), torch.float32, 75, scale=0.03)
+    out, ref, one = (torch.empty(r, inter, device="cuda") for r in (m, m, 1))
+    K.linear_swiglu(a, w, out)
+    REF.linear_swiglu(a, w, ref)
+    assert_close(out, ref, torch.float32, "swiglu")
+    K.linear_swiglu(a[m - 1:], w, one)
+    assert torch.equal(one[0], out[m - 1])
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,kv_heads,hd,page,window", [
+    (14, 2, 64, 16, 0), (9, 1, 40, 8, 0), (3, 3, 5, 4, 0), (4, 2, 256, 16, 0), (14, 2, 64, 16, 129), (8, 2, 100, 16, 33), (16, 1, 64, 8, 700)])
+def test_general_attention_segments(K, dtype, heads, kv_heads, hd, page, window):
+    """The general kernel at the edges of its blocks (32 keys), segments (128) and rounds (up to eight segments), of groups
+    larger than a CTA's eight heads, and with windows that begin inside a segment; a token alone gets the same bits as in a
+    batch of others (where another number of warps shares its keys)."""
+    K = K.with_options(force_general_attention=True)
+    before = [0, 31, 126, 127, 128, 255, 1023, 1100, 2047, 0]
+    q_lens = [1] * 9 + [40]
+    ctx, bt = make_paged_batch(q_lens, before, page, 8400 // page + 10, "cuda", seed=4)
+    kp, vp = _fill_cache(ctx, bt, page, bt.max().item() + 1, kv_heads, hd, dtype, 76)
+    m = sum(q_lens)
+    qkv = rnd((m, (heads + 2 * kv_heads) * hd), dtype, 78)
+    out, ref = (torch.empty(m, heads * hd, dtype=dtype, device="cuda") for _ in range(2))
+    scale = 1.0 / math.sqrt(hd)
+    K.attention(qkv, out, heads, kv_heads, hd, scale, window, ctx, bt, page, kp, vp)
+    REF.attention(qkv, ref, heads, kv_heads, hd, scale, window, ctx, bt, page, kp, vp)
+    assert_close(out, ref, dtype, "general attention")
+    for i in (0, 3, 8):
+        alone, bt1 = make_paged_batch([1], [before[i]], page, 1 + before[i] // page, "cuda", seed=4)
+        one = torch.empty(1, heads * hd, dtype=dtype, device="cuda")
+        K.attention(qkv[i:i + 1].contiguous(), one, heads, kv_heads, hd, scale, window, alone, bt[i:i + 1].contiguous(), page, kp, vp)
+        assert torch.equal(one[0], out[i])
