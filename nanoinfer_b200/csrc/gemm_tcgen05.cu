@@ -254,7 +254,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     __shared__ volatile int s_failed;
 
     pdl_launch_dependents();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) nib_trace_mark(trace, trace_cap, NIB_TK_GEMM_TC, EPI, 0);
     const int f_tiles = (n_out + BLOCK_F - 1) / BLOCK_F, t_tiles = (tokens + TOK - 1) / TOK;
     const int items = f_tiles * t_tiles * splits;       // work item = (output tile, split of K), splits fastest
@@ -275,77 +275,79 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const unsigned tmem_base = *tmem_slot;
+    const unsigned tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     pdl_wait();         // from here on the kernel reads what earlier kernels wrote (activations, the residual stream)
     if (threadIdx.x == 0) nib_trace_mark(trace, trace_cap, NIB_TK_GEMM_TC, EPI, 1);
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
         // ---------------- producer: TMA loads of W (and the up rows) and A tiles, stage after stage across tiles
-        int it = 0, issued = 0;
-        for (int item = blockIdx.x; item < items && !s_failed; item += gridDim.x) {
+        int it = 0;
+        bool ok = true;
+        for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
             const int tile = item / splits, split = item - tile * splits;
             const int f0 = (tile % f_tiles) * BLOCK_F, t0 = (tile / f_tiles) * TOK;
             const int kb_end = min(k_blocks, (split + 1) * kb_per_split);
             for (int kb = split * kb_per_split; kb < kb_end; ++kb, ++it) {
                 const int s = it % C::STAGES;
-                if (!mbar_wait(&empty_bar[s], ((it / C::STAGES) & 1) ^ 1)) {
-                    atomicCAS(&g_tc_error, 0, (1 << 16) | (int)blockIdx.x);
-                    s_failed = 1;
-                    break;
-                }
+                ok = warp_wait(&empty_bar[s], ((it / C::STAGES) & 1) ^ 1);
+                if (!ok) break;
                 unsigned char* st = smem + s * C::STAGE_BYTES;
-                mbar_expect_tx(&full_bar[s], C::STAGE_BYTES);
-                tma_load_2d(st, &map_w, &full_bar[s], kb * BLOCK_K, f0);
-                if (DUAL) tma_load_2d(st + C::W_BYTES, &map_w, &full_bar[s], kb * BLOCK_K, n_out + f0);
-                tma_load_2d(st + (DUAL ? 2 : 1) * C::W_BYTES, &map_a, &full_bar[s], kb * BLOCK_K, t0);
-                issued = it + 1;
+                if (elect_one()) {
+                    mbar_expect_tx(&full_bar[s], C::STAGE_BYTES);
+                    tma_load_2d(st, &map_w, &full_bar[s], kb * BLOCK_K, f0);
+                    if (DUAL) tma_load_2d(st + C::W_BYTES, &map_w, &full_bar[s], kb * BLOCK_K, n_out + f0);
+                    tma_load_2d(st + (DUAL ? 2 : 1) * C::W_BYTES, &map_a, &full_bar[s], kb * BLOCK_K, t0);
+                }
+                __syncwarp();
             }
         }
-        if (s_failed) {
+        if (!ok && lane == 0) {
+            if (!s_failed) atomicCAS(&g_tc_error, 0, (1 << 16) | (int)blockIdx.x);
+            s_failed = 1;
             // copies already issued still target this CTA's shared memory: wait for them, bounded
-            for (int i = max(0, issued - C::STAGES); i < issued; ++i)
+            for (int i = max(0, it - C::STAGES); i < it; ++i)
                 mbar_wait(&full_bar[i % C::STAGES], (i / C::STAGES) & 1);
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
         // ---------------- MMA issuer
         constexpr unsigned idesc = SWAP ? instr_desc(TOK, BLOCK_F) : instr_desc(BLOCK_F, TOK);
-        int it = 0, local = 0;
-        for (int item = blockIdx.x; item < items && !s_failed; item += gridDim.x, ++local) {
+        int it = 0, local = 0, code = 0;
+        for (int item = blockIdx.x; item < items; item += gridDim.x, ++local) {
             const int buf = local & 1;
             const int split = item % splits;
             const int kb_begin = split * kb_per_split, kb_end = min(k_blocks, kb_begin + kb_per_split);
             // the epilogue has drained this buffer (two tiles ago)
-            if (!mbar_wait(&acc_empty_bar[buf], ((local >> 1) & 1) ^ 1)) {
-                atomicCAS(&g_tc_error, 0, (4 << 16) | (int)blockIdx.x);
-                s_failed = 1;
-                break;
-            }
+            if (!warp_wait(&acc_empty_bar[buf], ((local >> 1) & 1) ^ 1)) { code = 4; break; }
             tc_fence_after();
             const unsigned acc = tmem_base + buf * C::ACC_COLS;
             for (int kb = kb_begin; kb < kb_end; ++kb, ++it) {
                 const int s = it % C::STAGES;
-                if (!mbar_wait(&full_bar[s], (it / C::STAGES) & 1)) {
-                    atomicCAS(&g_tc_error, 0, (2 << 16) | (int)blockIdx.x);
-                    s_failed = 1;
-                    break;
-                }
+                if (!warp_wait(&full_bar[s], (it / C::STAGES) & 1)) { code = 2; break; }
                 tc_fence_after();
                 const unsigned st = smem_u32(smem + s * C::STAGE_BYTES);
                 const unsigned long long w_desc = desc_kmajor(st);
                 const unsigned long long u_desc = desc_kmajor(st + C::W_BYTES);
                 const unsigned long long a_desc = desc_kmajor(st + (DUAL ? 2 : 1) * C::W_BYTES);
+                if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
-                    const unsigned long long adv = (unsigned long long)((k * UMMA_K * 2) >> 4);   // 32 bytes per step
-                    const bool accumulate = (kb > kb_begin) || (k > 0);
-                    if (SWAP) tc_mma(acc, a_desc + adv, w_desc + adv, idesc, accumulate);
-                    else tc_mma(acc, w_desc + adv, a_desc + adv, idesc, accumulate);
-                    if (DUAL) tc_mma(acc + TOK, u_desc + adv, a_desc + adv, idesc, accumulate);
+                    for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
+                        const unsigned long long adv = (unsigned long long)((k * UMMA_K * 2) >> 4);   // 32 bytes per step
+                        const bool accumulate = (kb > kb_begin) || (k > 0);
+                        if (SWAP) tc_mma(acc, a_desc + adv, w_desc + adv, idesc, accumulate);
+                        else tc_mma(acc, w_desc + adv, a_desc + adv, idesc, accumulate);
+                        if (DUAL) tc_mma(acc + TOK, u_desc + adv, a_desc + adv, idesc, accumulate);
+                    }
+                    tc_commit(&empty_bar[s]);        // the stage is free when these MMAs have read it
                 }
-                tc_commit(&empty_bar[s]);        // the stage is free when these MMAs have read it
+                __syncwarp();
             }
-            if (s_failed) break;
-            tc_commit(&acc_full_bar[buf]);       // the accumulator is complete when all MMAs are done
+            if (code != 0) break;
+            if (elect_one()) tc_commit(&acc_full_bar[buf]);       // the accumulator is complete when all MMAs are done
+            __syncwarp();
+        }
+        if (code != 0 && lane == 0) {
+            if (!s_failed) atomicCAS(&g_tc_error, 0, (code << 16) | (int)blockIdx.x);
+            s_failed = 1;
         }
     } else if (warp >= 2) {
         // ---------------- epilogue: TMEM -> registers -> global, one output feature per thread
@@ -587,7 +589,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_m, const __grid_constan
     __shared__ volatile int s_failed;
 
     pdl_launch_dependents();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     if (threadIdx.x == 0) nib_trace_mark(trace, trace_cap, NIB_TK_GEMM_PAIR, EPI, 0);
     const unsigned rank = cluster_rank();                       // 0: issues the MMAs and owns the shared barriers
     const int n_tiles = (n_out + FEAT - 1) / FEAT, m_tiles = (tokens + PAIR_M - 1) / PAIR_M;
@@ -614,14 +616,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_m, const __grid_constan
     __syncthreads();
     cluster_sync();            // the peer's barriers exist before anything signals them
     tc_fence_after();
-    const unsigned tmem_base = *tmem_slot;
+    const unsigned tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     pdl_wait();
     if (threadIdx.x == 0) nib_trace_mark(trace, trace_cap, NIB_TK_GEMM_PAIR, EPI, 1);
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
         // ---------------- producer (in both CTAs): this CTA's 128 token rows and its half of the weight rows
         int it = 0;
-        for (int item = cluster_id; item < items && !s_failed; item += n_clusters) {
+        bool ok = true;
+        for (int item = cluster_id; item < items && ok; item += n_clusters) {
             const int tile = item / splits, split = item - tile * splits;
             const int f0 = (tile % n_tiles) * FEAT, t0 = (tile / n_tiles) * PAIR_M + (int)rank * BLOCK_F;
             // weight rows: half of the tile's features, or (gate/up) the gate rows here and the up rows in the peer
@@ -629,53 +632,57 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_m, const __grid_constan
             const int kb_end = min(k_blocks, (split + 1) * kb_per_split);
             for (int kb = split * kb_per_split; kb < kb_end; ++kb, ++it) {
                 const int s = it % C::STAGES;
-                if (!mbar_wait(&empty_bar[s], ((it / C::STAGES) & 1) ^ 1)) {
-                    atomicCAS(&g_tc_error, 0, (5 << 16) | (int)blockIdx.x);
-                    s_failed = 1;
-                    break;
-                }
+                ok = warp_wait(&empty_bar[s], ((it / C::STAGES) & 1) ^ 1);
+                if (!ok) break;
                 unsigned char* st = smem + s * C::STAGE_BYTES;
                 const unsigned bar0 = peer_smem(&full_bar[s], 0);
-                if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * C::STAGE_BYTES);
-                tma_load_2d_pair(st, &map_m, bar0, kb * BLOCK_K, t0);
-                tma_load_2d_pair(st + C::M_BYTES, &map_n, bar0, kb * BLOCK_K, w0);
+                if (elect_one()) {
+                    if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * C::STAGE_BYTES);
+                    tma_load_2d_pair(st, &map_m, bar0, kb * BLOCK_K, t0);
+                    tma_load_2d_pair(st + C::M_BYTES, &map_n, bar0, kb * BLOCK_K, w0);
+                }
+                __syncwarp();
             }
         }
-    } else if (warp == 1 && lane == 0 && rank == 0) {
+        if (!ok && lane == 0) {
+            if (!s_failed) atomicCAS(&g_tc_error, 0, (5 << 16) | (int)blockIdx.x);
+            s_failed = 1;
+        }
+    } else if (warp == 1 && rank == 0) {
         // ---------------- MMA issuer: one thread of the even CTA, for both
         constexpr unsigned idesc = instr_desc(PAIR_M, NT);
-        int it = 0, local = 0;
-        for (int item = cluster_id; item < items && !s_failed; item += n_clusters, ++local) {
+        int it = 0, local = 0, code = 0;
+        for (int item = cluster_id; item < items; item += n_clusters, ++local) {
             const int buf = local & 1;
             const int split = item % splits;
             const int kb_begin = split * kb_per_split, kb_end = min(k_blocks, kb_begin + kb_per_split);
-            if (!mbar_wait(&acc_empty_bar[buf], ((local >> 1) & 1) ^ 1)) {
-                atomicCAS(&g_tc_error, 0, (6 << 16) | (int)blockIdx.x);
-                s_failed = 1;
-                break;
-            }
+            if (!warp_wait(&acc_empty_bar[buf], ((local >> 1) & 1) ^ 1)) { code = 6; break; }
             tc_fence_after();
             const unsigned acc = tmem_base + buf * NT;
             for (int kb = kb_begin; kb < kb_end; ++kb, ++it) {
                 const int s = it % C::STAGES;
-                if (!mbar_wait(&full_bar[s], (it / C::STAGES) & 1)) {
-                    atomicCAS(&g_tc_error, 0, (7 << 16) | (int)blockIdx.x);
-                    s_failed = 1;
-                    break;
-                }
+                if (!warp_wait(&full_bar[s], (it / C::STAGES) & 1)) { code = 7; break; }
                 tc_fence_after();
                 const unsigned st = smem_u32(smem + s * C::STAGE_BYTES);
                 const unsigned long long m_desc = desc_kmajor(st);
                 const unsigned long long n_desc = desc_kmajor(st + C::M_BYTES);
+                if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
-                    const unsigned long long adv = (unsigned long long)((k * UMMA_K * 2) >> 4);
-                    tc_mma_pair(acc, m_desc + adv, n_desc + adv, idesc, (kb > kb_begin) || (k > 0));
+                    for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
+                        const unsigned long long adv = (unsigned long long)((k * UMMA_K * 2) >> 4);
+                        tc_mma_pair(acc, m_desc + adv, n_desc + adv, idesc, (kb > kb_begin) || (k > 0));
+                    }
+                    tc_commit_pair(&empty_bar[s]);       // frees the stage in both CTAs
                 }
-                tc_commit_pair(&empty_bar[s]);       // frees the stage in both CTAs
+                __syncwarp();
             }
-            if (s_failed) break;
-            tc_commit_pair(&acc_full_bar[buf]);      // the accumulators of both CTAs are complete
+            if (code != 0) break;
+            if (elect_one()) tc_commit_pair(&acc_full_bar[buf]);      // the accumulators of both CTAs are complete
+            __syncwarp();
+        }
+        if (code != 0 && lane == 0) {
+            if (!s_failed) atomicCAS(&g_tc_error, 0, (code << 16) | (int)blockIdx.x);
+            s_failed = 1;
         }
     } else if (warp >= 2) {
         // ---------------- epilogue (in both CTAs): one token row per thread, half of the tile's features per warp

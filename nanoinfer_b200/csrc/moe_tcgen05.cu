@@ -84,7 +84,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     __shared__ int s_row[4][TOK];        // ... and the row each writes (-1: none)
 
     pdl_launch_dependents();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int f_tiles = (n_out + BLOCK_F - 1) / BLOCK_F;
     const int k_blocks = (k_dim + BLOCK_K - 1) / BLOCK_K;
 
@@ -103,7 +103,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const unsigned tmem_base = *tmem_slot;
+    const unsigned tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     pdl_wait();         // from here on the kernel reads what earlier kernels wrote (the table, the rows)
     int nt = __ldcg(n_tiles);
     if (nt > max_tiles) nt = max_tiles;
@@ -112,10 +112,11 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     const int items = nt * f_tiles * splits;
     const bool reduce = scatter == 2 || splits > 1;
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
         // ---------------- producer: TMA loads of the expert's weight rows and of the tile's rows, stage after stage
-        int it = 0, issued = 0;
-        for (int item = blockIdx.x; item < items && !s_failed; item += gridDim.x) {
+        int it = 0;
+        bool ok = true;
+        for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
             const int split = item % splits, rest = item / splits;
             const int tile = rest / f_tiles, f0 = (rest - tile * f_tiles) * BLOCK_F;
             const int expert = __ldg(tiles + 3 * tile), row0 = __ldg(tiles + 3 * tile + 1);
@@ -123,67 +124,68 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
             const int kb_end = min(k_blocks, (split + 1) * kb_per_split);
             for (int kb = split * kb_per_split; kb < kb_end; ++kb, ++it) {
                 const int s = it % C::STAGES;
-                if (!mbar_wait(&empty_bar[s], ((it / C::STAGES) & 1) ^ 1)) {
-                    atomicCAS(&g_moe_tc_error, 0, (1 << 16) | (int)blockIdx.x);
-                    s_failed = 1;
-                    break;
-                }
+                ok = warp_wait(&empty_bar[s], ((it / C::STAGES) & 1) ^ 1);
+                if (!ok) break;
                 unsigned char* st = smem + s * C::STAGE_BYTES;
-                mbar_expect_tx(&full_bar[s], C::STAGE_BYTES);
-                tma_load_2d(st, &map_w, &full_bar[s], kb * BLOCK_K, wrow);
-                if (DUAL) tma_load_2d(st + C::W_BYTES, &map_w, &full_bar[s], kb * BLOCK_K, wrow + n_out);
-                tma_load_2d(st + (DUAL ? 2 : 1) * C::W_BYTES, &map_a, &full_bar[s], kb * BLOCK_K, row0);
-                issued = it + 1;
+                if (elect_one()) {
+                    mbar_expect_tx(&full_bar[s], C::STAGE_BYTES);
+                    tma_load_2d(st, &map_w, &full_bar[s], kb * BLOCK_K, wrow);
+                    if (DUAL) tma_load_2d(st + C::W_BYTES, &map_w, &full_bar[s], kb * BLOCK_K, wrow + n_out);
+                    tma_load_2d(st + (DUAL ? 2 : 1) * C::W_BYTES, &map_a, &full_bar[s], kb * BLOCK_K, row0);
+                }
+                __syncwarp();
             }
         }
-        if (s_failed) {
+        if (!ok && lane == 0) {
+            if (!s_failed) atomicCAS(&g_moe_tc_error, 0, (1 << 16) | (int)blockIdx.x);
+            s_failed = 1;
             // copies already issued still target this CTA's shared memory: wait for them, bounded
-            for (int i = max(0, issued - C::STAGES); i < issued; ++i)
+            for (int i = max(0, it - C::STAGES); i < it; ++i)
                 mbar_wait(&full_bar[i % C::STAGES], (i / C::STAGES) & 1);
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
         // ---------------- MMA issuer
         constexpr unsigned idesc = SWAP ? instr_desc(TOK, BLOCK_F) : instr_desc(BLOCK_F, TOK);
-        int it = 0, local = 0;
-        for (int item = blockIdx.x; item < items && !s_failed; item += gridDim.x, ++local) {
+        int it = 0, local = 0, code = 0;
+        for (int item = blockIdx.x; item < items; item += gridDim.x, ++local) {
             const int buf = local & 1;
             // the epilogue has drained this buffer (two tiles ago)
-            if (!mbar_wait(&acc_empty_bar[buf], ((local >> 1) & 1) ^ 1)) {
-                atomicCAS(&g_moe_tc_error, 0, (4 << 16) | (int)blockIdx.x);
-                s_failed = 1;
-                break;
-            }
+            if (!warp_wait(&acc_empty_bar[buf], ((local >> 1) & 1) ^ 1)) { code = 4; break; }
             tc_fence_after();
             const unsigned acc = tmem_base + buf * C::ACC_COLS;
             const int kb_begin = (item % splits) * kb_per_split, kb_end = min(k_blocks, kb_begin + kb_per_split);
             for (int kb = kb_begin; kb < kb_end; ++kb, ++it) {
                 const int s = it % C::STAGES;
-                if (!mbar_wait(&full_bar[s], (it / C::STAGES) & 1)) {
-                    atomicCAS(&g_moe_tc_error, 0, (2 << 16) | (int)blockIdx.x);
-                    s_failed = 1;
-                    break;
-                }
+                if (!warp_wait(&full_bar[s], (it / C::STAGES) & 1)) { code = 2; break; }
                 tc_fence_after();
                 const unsigned st = smem_u32(smem + s * C::STAGE_BYTES);
                 const unsigned long long w_desc = desc_kmajor(st);
                 const unsigned long long u_desc = desc_kmajor(st + C::W_BYTES);
                 const unsigned long long a_desc = desc_kmajor(st + (DUAL ? 2 : 1) * C::W_BYTES);
+                if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
-                    const unsigned long long adv = (unsigned long long)((k * UMMA_K * 2) >> 4);   // 32 bytes per step
-                    const bool accumulate = (kb > kb_begin) || (k > 0);
-                    if (SWAP) {
-                        tc_mma(acc, a_desc + adv, w_desc + adv, idesc, accumulate);
-                        if (DUAL) tc_mma(acc + BLOCK_F, a_desc + adv, u_desc + adv, idesc, accumulate);
-                    } else {
-                        tc_mma(acc, w_desc + adv, a_desc + adv, idesc, accumulate);
-                        if (DUAL) tc_mma(acc + TOK, u_desc + adv, a_desc + adv, idesc, accumulate);
+                    for (int k = 0; k < BLOCK_K / UMMA_K; ++k) {
+                        const unsigned long long adv = (unsigned long long)((k * UMMA_K * 2) >> 4);   // 32 bytes per step
+                        const bool accumulate = (kb > kb_begin) || (k > 0);
+                        if (SWAP) {
+                            tc_mma(acc, a_desc + adv, w_desc + adv, idesc, accumulate);
+                            if (DUAL) tc_mma(acc + BLOCK_F, a_desc + adv, u_desc + adv, idesc, accumulate);
+                        } else {
+                            tc_mma(acc, w_desc + adv, a_desc + adv, idesc, accumulate);
+                            if (DUAL) tc_mma(acc + TOK, u_desc + adv, a_desc + adv, idesc, accumulate);
+                        }
                     }
+                    tc_commit(&empty_bar[s]);        // the stage is free when these MMAs have read it
                 }
-                tc_commit(&empty_bar[s]);        // the stage is free when these MMAs have read it
+                __syncwarp();
             }
-            if (s_failed) break;
-            tc_commit(&acc_full_bar[buf]);       // the accumulator is complete when all MMAs are done
+            if (code != 0) break;
+            if (elect_one()) tc_commit(&acc_full_bar[buf]);       // the accumulator is complete when all MMAs are done
+            __syncwarp();
+        }
+        if (code != 0 && lane == 0) {
+            if (!s_failed) atomicCAS(&g_moe_tc_error, 0, (code << 16) | (int)blockIdx.x);
+            s_failed = 1;
         }
     } else if (warp >= 2) {
         // ---------------- epilogue: TMEM -> registers -> global, one output feature per thread

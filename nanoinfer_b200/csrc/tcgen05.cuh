@@ -9,6 +9,19 @@ namespace nibt {
 
 using nibp::smem_u32;
 
+// ---- one thread of a converged warp. The tensor core and the copy engine take their operands from the warp's uniform
+// registers. A role that a whole warp runs, in loops whose bounds, waits and addresses are the warp's and not a thread's, with
+// only the instructions themselves behind elect_one(), keeps them there; a role that lane 0 runs alone has every operand of
+// every instruction moved over first (about 150 cycles for one tcgen05.mma: more than the instruction takes).
+__device__ __forceinline__ bool elect_one() {
+    unsigned is;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(is));
+    return is != 0;
+}
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+// a wait of the whole warp, with one answer
+__device__ __forceinline__ bool warp_wait(unsigned long long* bar, unsigned parity) { return __all_sync(0xffffffffu, nibp::mbar_wait(bar, parity)); }
+
 // ---- tensor memory: allocated and freed by one whole warp; the address arrives in shared memory
 __device__ __forceinline__ void tmem_alloc(unsigned* dst_smem, unsigned cols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(dst_smem)), "r"(cols) : "memory");
@@ -57,6 +70,14 @@ __device__ __forceinline__ void tc_mma_pair(unsigned d_tmem, unsigned long long 
                  ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(acc) : "memory");
 }
 
+// ---- D[tmem] (+)= A[tmem] . B[smem]^T: A has a row per lane, two bfloat16 of K to a column (the even one below)
+__device__ __forceinline__ void tc_mma_ts(unsigned d_tmem, unsigned a_tmem, unsigned long long b_desc, unsigned idesc, bool accumulate) {
+    const unsigned acc = accumulate ? 1u : 0u;
+    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                 " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+                 ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(acc) : "memory");
+}
+
 // ---- a thread's TMEM lane to and from registers. The values of a load may be used only after tmem_wait_ld();
 // issue every load of a batch first and wait once: a load's latency is hundreds of cycles.
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
@@ -82,6 +103,12 @@ __device__ __forceinline__ void tmem_ld32_async(unsigned addr, unsigned (&r)[32]
                    "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
                    "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
                  : "r"(addr));
+}
+__device__ __forceinline__ void tmem_st16(unsigned addr, const unsigned (&r)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n"
+                 ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+                   "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+                 : "memory");
 }
 __device__ __forceinline__ void tmem_st32(unsigned addr, const unsigned (&r)[32]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
