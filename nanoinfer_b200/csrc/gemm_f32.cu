@@ -12,7 +12,7 @@
 //   16-byte copies, sent before the wait for the kernel before it); then a thread per (row, chunk) walks its chain, eight
 //   rows side by side in a warp (rows lie one 16-byte unit off a multiple of eight apart: no bank conflicts; the tokens'
 //   values are broadcast). A long K is shared by the CTAs of a cluster, whose chunk sums the first one adds up in order.
-// * gemm_f32_tile_kernel, more tokens: bound by the multiply-adds. Tiles of 64 x 64, 8 x 4 outputs a thread, the next 16 k
+// * gemm_f32_tile_kernel, more tokens: bound by the multiply-adds. Tiles of 64 x 64, 4 x 4 outputs a thread, the next 16 k
 //   fetched into registers under this block's arithmetic. Few tiles: the chunks are shared by the CTAs of a cluster.
 //
 // Measured on B200 at the 0.5B widths, a step of one token / a prompt of 128: see the figures beside the launch rules below.
@@ -162,44 +162,35 @@ gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, c
 }
 
 // ------------------------------------------------------------------------------------------------ more tokens
-constexpr int BM = 64, BN = 64, BK = 16, TM = 8, TN = 4, TILE_THREADS = 128, TILE_PITCH = 68;
+constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4, TILE_THREADS = 256, TILE_PITCH = 68;
 
-// A thread's share of a 64 x 16 block of a row-major matrix: two runs of four k of one row, zeros outside.
-struct Fetched { float4 v[2]; };
-__device__ __forceinline__ Fetched fetch_block(const float* src, size_t stride, int rows, int k, int K, bool wide) {
-    Fetched f;
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int r = (threadIdx.x >> 2) + 32 * i, kk = k + 4 * (threadIdx.x & 3);
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (r < rows && kk < K) {
-            const float* p = src + (size_t)r * stride + kk;
-            if (wide) {
-                v = *reinterpret_cast<const float4*>(p);
-            } else {
-                v.x = p[0];
-                if (kk + 1 < K) v.y = p[1];
-                if (kk + 2 < K) v.z = p[2];
-                if (kk + 3 < K) v.w = p[3];
-            }
+// A thread's share of a 64 x 16 block of a row-major matrix: four k of one row, zeros outside.
+__device__ __forceinline__ float4 fetch_block(const float* src, size_t stride, int rows, int k, int K, bool wide) {
+    const int r = threadIdx.x >> 2, kk = k + 4 * (threadIdx.x & 3);
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (r < rows && kk < K) {
+        const float* p = src + (size_t)r * stride + kk;
+        if (wide) {
+            v = *reinterpret_cast<const float4*>(p);
+        } else {
+            v.x = p[0];
+            if (kk + 1 < K) v.y = p[1];
+            if (kk + 2 < K) v.z = p[2];
+            if (kk + 3 < K) v.w = p[3];
         }
-        f.v[i] = v;
     }
-    return f;
+    return v;
 }
-__device__ __forceinline__ void put_block(float (*dst)[TILE_PITCH], const Fetched& f) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int r = (threadIdx.x >> 2) + 32 * i, kk = 4 * (threadIdx.x & 3);
-        dst[kk][r] = f.v[i].x;
-        dst[kk + 1][r] = f.v[i].y;
-        dst[kk + 2][r] = f.v[i].z;
-        dst[kk + 3][r] = f.v[i].w;
-    }
+__device__ __forceinline__ void put_block(float (*dst)[TILE_PITCH], const float4& v) {
+    const int r = threadIdx.x >> 2, kk = 4 * (threadIdx.x & 3);
+    dst[kk][r] = v.x;
+    dst[kk + 1][r] = v.y;
+    dst[kk + 2][r] = v.z;
+    dst[kk + 3][r] = v.w;
 }
 
 template <int EPI, bool SPLIT>
-__global__ void __launch_bounds__(TILE_THREADS)
+__global__ void __launch_bounds__(TILE_THREADS, 2)
 gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, const float* __restrict__ bias, float* __restrict__ out,
                      int M, int N, int K, int lda, int ldo, int chunks_per_cta, int wide, const NibGlu glu) {
     constexpr bool DUAL = epi_dual(EPI);
@@ -233,10 +224,10 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
 
     pdl_launch_dependents();
     int k = c_lo * CHUNK;
-    Fetched fw = fetch_block(w_src, K, w_rows, k, k_hi, wide), fu;
+    float4 fw = fetch_block(w_src, K, w_rows, k, k_hi, wide), fu;
     if (DUAL) fu = fetch_block(u_src, K, w_rows, k, k_hi, wide);
     pdl_wait();
-    Fetched fa = fetch_block(a_src, lda, a_rows, k, k_hi, wide);
+    float4 fa = fetch_block(a_src, lda, a_rows, k, k_hi, wide);
     int buf = 0;
     for (int c = c_lo; c < c_hi; ++c) {
 #pragma unroll 1
@@ -255,7 +246,6 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
             for (int kk = 0; kk < BK; ++kk) {
                 float a[TM], w[TN], u[TN];
                 *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(&As[buf][kk][ty * TM]);
-                *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(&As[buf][kk][ty * TM + 4]);
                 *reinterpret_cast<float4*>(w) = *reinterpret_cast<const float4*>(&Ws[buf][kk][tx * TN]);
                 if (DUAL) *reinterpret_cast<float4*>(u) = *reinterpret_cast<const float4*>(&Us[DUAL ? buf : 0][DUAL ? kk : 0][tx * TN]);
 #pragma unroll
@@ -293,7 +283,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, c
             for (int s = 0; s < ranks; ++s) {
                 const int n = min(chunks_per_cta, all_chunks - s * chunks_per_cta);
                 const unsigned peer = peer_smem(part + i * BN + j, s);
-#pragma unroll 2
+#pragma unroll 4
                 for (int c = 0; c < n; ++c) {
                     const float4 p = ld_peer_f32x4(peer + 4u * (unsigned)(c * ACCS * BM * BN));
                     v[0] += p.x; v[1] += p.y; v[2] += p.z; v[3] += p.w;
@@ -391,7 +381,11 @@ int launch_f32(const Args& a) {
         }
     }
     const int tiles = ceil_div(a.N, BN) * ceil_div(a.M, BM);
-    int ranks = max(1, min(min(8, chunks), ceil_div(2 * 148, tiles)));
+    // CTAs that share the chunks of a tile: as many as keep all CTAs on the GPU at once, two an SM; with more tiles than SMs none,
+    // unless their last turn would leave most SMs idle (152 tiles of 7 chunks on 148 SMs: 105 us with a CTA a tile, 94 with seven)
+    int ranks = 2 * 148 / tiles;
+    if (tiles > 148 && ceil_div(tiles, 148) * 148 > tiles + tiles / 2) ranks = 8;
+    ranks = max(1, min(min(8, chunks), ranks));
     const int cpc = ceil_div(chunks, ranks);
     ranks = ceil_div(chunks, cpc);
     const size_t smem = sizeof(float) * (size_t)cpc * (DUAL ? 2 : 1) * BM * BN;
