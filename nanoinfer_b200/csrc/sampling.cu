@@ -173,13 +173,14 @@ constexpr float FIX_ONE = 1099511627776.0f;  // 2^40
 // A mass into the three histograms of 14-bit chunks. 64-bit adds to shared memory are loops of compare-and-swap, and
 // the first radix pass (the key's top 8 bits: sign and exponent of the scaled logit) puts almost every element of a
 // row into a handful of bins: a thousand threads queueing there with such loops made a pure top-p row cost two
-// milliseconds. 32-bit adds to one address are combined by the hardware. A row's masses sum to 2^40, so every
-// chunk's sum over up to 2^17 elements stays below 2^32.
-__device__ __forceinline__ void mass_add(unsigned (*m)[256], unsigned bin, unsigned long long q) {
+// milliseconds. A row's masses sum to 2^40, so every chunk's sum over up to 2^17 elements stays below 2^32. Lanes that add
+// to one bin queue too, so there are COPIES of every histogram, a lane uses its own and each lies a bank further on.
+constexpr int COPIES = 8, BINS = 257;       // (bins of a copy, with the bank in between)
+__device__ __forceinline__ void mass_add(unsigned (*m)[COPIES * BINS], unsigned at, unsigned long long q) {
     const unsigned a = (unsigned)(q & 0x3fffull), b = (unsigned)((q >> 14) & 0x3fffull), c = (unsigned)(q >> 28);
-    if (a) atomicAdd(&m[0][bin], a);
-    if (b) atomicAdd(&m[1][bin], b);
-    if (c) atomicAdd(&m[2][bin], c);
+    if (a) atomicAdd(&m[1][at], a);
+    if (b) atomicAdd(&m[2][at], b);
+    if (c) atomicAdd(&m[3][at], c);
 }
 
 // ---- the sampling kernel: a cluster of CS CTAs per row. One SM working through a row of 152K logits a dozen times was
@@ -188,7 +189,8 @@ __device__ __forceinline__ void mass_add(unsigned (*m)[256], unsigned bin, unsig
 // memory between cluster barriers. Everything that decides a token is either an integer sum (histograms of counts
 // and of fixed-point masses: any order gives the same) or a float sum in a fixed order (threads, warps, lanes and CTAs
 // in ascending order), so a row's token depends on the row alone.
-constexpr int ST = 256;      // threads of a CTA
+constexpr int ST = 256;      // chunks of a CTA's slice: what is summed in order is summed by so many threads
+constexpr int NT = 512;      // threads of a CTA
 constexpr int CS = 8;        // CTAs of the cluster that shares a row
 
 __device__ __forceinline__ unsigned ld_peer_u32(unsigned addr) {
@@ -202,71 +204,91 @@ __device__ __forceinline__ unsigned long long ld_peer_u64(unsigned addr) {
     return v;
 }
 
-// f(x) for every scaled logit x = l[i] / temperature of the CTA's slice [begin, end) of a row, in no particular order:
-// 16-byte loads, two of them in flight per thread, where the slice allows (a thread with one 4-byte load in flight waits
-// out the whole latency of the memory system for every element). begin is a multiple of 4.
-template <typename F>
-__device__ __forceinline__ void for_each_scaled(const float* __restrict__ l, int begin, int end, float inv_t, F&& f) {
-    const int tid = threadIdx.x;
-    int done = begin;
-    if ((reinterpret_cast<uintptr_t>(l) & 15) == 0) {
-        const float4* l4 = reinterpret_cast<const float4*>(l + begin);
-        const int n4 = (end - begin) >> 2;
-        int i = tid;
-        for (; i + ST < n4; i += 2 * ST) {
-            const float4 a = l4[i], b = l4[i + ST];
-            f(a.x * inv_t); f(a.y * inv_t); f(a.z * inv_t); f(a.w * inv_t);
-            f(b.x * inv_t); f(b.y * inv_t); f(b.z * inv_t); f(b.w * inv_t);
-        }
-        if (i < n4) {
-            const float4 a = l4[i];
-            f(a.x * inv_t); f(a.y * inv_t); f(a.z * inv_t); f(a.w * inv_t);
-        }
-        done = begin + 4 * n4;
+// The scaled logits l[i] / temperature of a CTA's slice of a row, as the kernel's passes read them: from shared memory, where
+// the first pass has left them (a dozen passes over global memory, two loads in flight a thread, took half of the kernel's
+// time), or, for a vocabulary whose slice does not fit, from global memory each time. Element i of the slice; ``vec``: the
+// row starts on 16 bytes.
+template <bool KEPT>
+struct Slice {
+    const float* p;         // KEPT: shared memory, scaled; else the slice's first logit
+    int n;
+    float inv_t;
+    bool vec;
+    __device__ __forceinline__ float at(int i) const { return KEPT ? p[i] : p[i] * inv_t; }
+    __device__ __forceinline__ float4 at4(int i4) const {
+        float4 v = reinterpret_cast<const float4*>(p)[i4];
+        if (!KEPT) { v.x *= inv_t; v.y *= inv_t; v.z *= inv_t; v.w *= inv_t; }
+        return v;
     }
-    for (int i = done + tid; i < end; i += ST) f(l[i] * inv_t);
-}
-
-// f(i, x) for i = begin .. end - 1 in ascending order (a thread's chunk of a row), until f returns false. 16-byte loads,
-// all of a group of 16 elements issued before the first is used, where begin is a multiple of 4 and the row is aligned.
-template <typename F>
-__device__ __forceinline__ void for_chunk(const float* __restrict__ l, int begin, int end, float inv_t, F&& f) {
-    int i = begin;
-    if ((begin & 3) == 0 && (reinterpret_cast<uintptr_t>(l) & 15) == 0) {
-        for (; i + 16 <= end; i += 16) {
-            float4 v[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = *reinterpret_cast<const float4*>(l + i + 4 * j);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                if (!f(i + 4 * j, v[j].x * inv_t)) return;
-                if (!f(i + 4 * j + 1, v[j].y * inv_t)) return;
-                if (!f(i + 4 * j + 2, v[j].z * inv_t)) return;
-                if (!f(i + 4 * j + 3, v[j].w * inv_t)) return;
+    // f(x) for every element, in no particular order, by all threads of the CTA
+    template <typename F>
+    __device__ __forceinline__ void each(F&& f) const {
+        int done = 0;
+        if (KEPT || vec) {
+            const int n4 = n >> 2;
+#pragma unroll 2
+            for (int i = threadIdx.x; i < n4; i += blockDim.x) {
+                const float4 v = at4(i);
+                f(v.x); f(v.y); f(v.z); f(v.w);
+            }
+            done = 4 * n4;
+        }
+        for (int i = done + threadIdx.x; i < n; i += blockDim.x) f(at(i));
+    }
+    // the same by threads 0..ST-1, each its elements in ascending order: groups of four ST groups apart where the row starts
+    // on 16 bytes, elements ST apart otherwise
+    template <typename F>
+    __device__ __forceinline__ void each_in_order(F&& f) const {
+        if (threadIdx.x >= ST) return;
+        int done = 0;
+        if (vec) {
+            const int n4 = n >> 2;
+            for (int i = threadIdx.x; i < n4; i += ST) {
+                const float4 v = at4(i);
+                f(v.x); f(v.y); f(v.z); f(v.w);
+            }
+            done = 4 * n4;
+        }
+        for (int i = done + threadIdx.x; i < n; i += ST) f(at(i));
+    }
+    // f(i, x) for i = begin .. end - 1 in ascending order (a thread's chunk; begin is a multiple of 4), until f returns false
+    template <typename F>
+    __device__ __forceinline__ void chunk(int begin, int end, F&& f) const {
+        int i = begin;
+        if (KEPT || vec) {
+            for (; i + 4 <= end; i += 4) {
+                const float4 v = at4(i >> 2);
+                if (!f(i, v.x)) return;
+                if (!f(i + 1, v.y)) return;
+                if (!f(i + 2, v.z)) return;
+                if (!f(i + 3, v.w)) return;
             }
         }
+        for (; i < end; ++i)
+            if (!f(i, at(i))) return;
     }
-    for (; i < end; ++i)
-        if (!f(i, l[i] * inv_t)) return;
-}
+};
 
 // The unnormalised probability of a scaled logit d = x - max <= 0, the same function wherever the kernel needs it. The
 // fast exponential (2 ulp) is plenty for a draw.
 __device__ __forceinline__ float weight(float d) { return __expf(d); }
 
-// temperature > 0 for every row given to this kernel. grid: CS CTAs (one cluster) per row.
-__global__ void __launch_bounds__(ST)
+// temperature > 0 for every row given to this kernel. grid: CS CTAs (one cluster) per row. Dynamic shared memory: the
+// histograms' copies and, KEPT, the slice.
+template <bool KEPT>
+__global__ void __launch_bounds__(NT)
 sample_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p, const float* __restrict__ uniform,
               int* __restrict__ out) {
     using namespace nibp;
-    __shared__ float scratch[ST / 32];
-    __shared__ unsigned hist[256];                  // this CTA's histogram of a radix pass
-    // ... and its masses as three histograms of 14-bit chunks: mass = m0 + m1 * 2^14 + m2 * 2^28
-    __shared__ unsigned mass3[3][256];
-    __shared__ unsigned tot_hist[256];              // CTA 0: the cluster's sums
+    extern __shared__ __align__(16) float dyn[];
+    unsigned (*copies)[COPIES * BINS] = reinterpret_cast<unsigned (*)[COPIES * BINS]>(dyn);      // counts, then masses as three histograms
+    float* kept = dyn + 4 * COPIES * BINS;          // of 14-bit chunks: mass = m1 + m2 * 2^14 + m3 * 2^28
+    __shared__ float scratch[NT / 32];
+    __shared__ unsigned pub[2][4][256];             // this CTA's histograms of a radix pass, for the cluster; the passes take turns
+    __shared__ unsigned tot_hist[256];              // the cluster's sums
     __shared__ unsigned long long tot_mass[256];
-    __shared__ unsigned dec_prefix, dec_remaining;  // CTA 0: what a radix pass decided, read by every CTA
+    __shared__ unsigned dec_prefix, dec_remaining;  // what a radix pass decided (every CTA decides for itself, alike)
     __shared__ unsigned long long dec_above;
     __shared__ float x_max, x_z, x_total;           // what this CTA tells the others
     __shared__ int x_ties;
@@ -281,56 +303,98 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
     const float inv_t = 1.0f / temperature[row];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
-    // a thread's chunk of the row (vocabulary order: rank, then thread), a multiple of 4 long so that chunks start on 16 bytes
+    // a thread's chunk of the row (vocabulary order: rank, then thread), a multiple of 4 long so that chunks start on 16 bytes;
+    // begin and end count from the slice's first element
     const int per = ((vocab + CS * ST - 1) / (CS * ST) + 3) & ~3;
-    const int begin = min(vocab, ((int)rank * ST + tid) * per), end = min(vocab, begin + per);
-    const int s_begin = min(vocab, (int)rank * ST * per), s_end = min(vocab, s_begin + ST * per);
+    const int s_begin = min(vocab, (int)rank * ST * per), s_n = min(vocab, s_begin + ST * per) - s_begin;
+    const int begin = tid < ST ? min(s_n, tid * per) : 0, end = tid < ST ? min(s_n, begin + per) : 0;
+    const bool vec = (reinterpret_cast<uintptr_t>(l) & 15) == 0;
+    const Slice<KEPT> slice{KEPT ? kept : l + s_begin, s_n, inv_t, vec};
 
-    auto cta_reduce = [&](float v, bool is_max) -> float {      // over the CTA, in a fixed order
+    auto cta_reduce = [&](float v, bool is_max, int warps) -> float {      // over the CTA's first warps, in a fixed order
         v = is_max ? warp_max(v) : warp_sum(v);
         if (lane == 0) scratch[warp] = v;
         __syncthreads();
         float r = scratch[0];
-        for (int i = 1; i < ST / 32; ++i) r = is_max ? fmaxf(r, scratch[i]) : r + scratch[i];
+        for (int i = 1; i < warps; ++i) r = is_max ? fmaxf(r, scratch[i]) : r + scratch[i];
         __syncthreads();
         return r;
     };
 
-    // ---- the row's maximum
+    // ---- the row's maximum; KEPT: what is read for it stays
     float mx = -INFINITY;
-    for_each_scaled(l, s_begin, s_end, inv_t, [&](float x) { mx = fmaxf(mx, x); });
-    mx = cta_reduce(mx, true);
+    if (KEPT) {
+        const float* src = l + s_begin;
+        int done = 0;
+        if (vec) {
+            const int n4 = s_n >> 2;
+#pragma unroll 8
+            for (int i = tid; i < n4; i += NT) {
+                float4 v = reinterpret_cast<const float4*>(src)[i];
+                v.x *= inv_t; v.y *= inv_t; v.z *= inv_t; v.w *= inv_t;
+                reinterpret_cast<float4*>(kept)[i] = v;
+                mx = fmaxf(fmaxf(fmaxf(mx, v.x), fmaxf(v.y, v.z)), v.w);
+            }
+            done = 4 * n4;
+        }
+#pragma unroll 8
+        for (int i = done + tid; i < s_n; i += NT) {
+            const float x = src[i] * inv_t;
+            kept[i] = x;
+            mx = fmaxf(mx, x);
+        }
+    } else {
+        slice.each([&](float x) { mx = fmaxf(mx, x); });
+    }
+    mx = cta_reduce(mx, true, NT / 32);
     if (tid == 0) x_max = mx;
     cluster_sync();
     for (unsigned r = 0; r < CS; ++r) mx = fmaxf(mx, ld_peer_f32(peer_smem(&x_max, r)));
 
-    // One radix pass over the slice: histogram (and masses), summed over the cluster by CTA 0, whose thread 0 then
-    // chooses the digit (``choose``) and leaves the decision where every CTA reads it after the second barrier.
+    // One radix pass over the slice: histogram (and masses), told to the cluster; every CTA sums them up and chooses the
+    // digit (``choose``, warp 0). A pass tells its results in the buffer of the pass before the last one: whoever is past the
+    // last pass's barrier has read that.
+    int pass = 0;
+    const unsigned copy = (lane & (COPIES - 1)) * BINS;
     auto radix_pass = [&](bool with_mass, auto&& add, auto&& choose) {
-        for (int b = tid; b < 256; b += ST) { hist[b] = 0u; mass3[0][b] = mass3[1][b] = mass3[2][b] = 0u; }
+        unsigned (*mine)[256] = pub[pass++ & 1];
+        const int used = with_mass ? 4 : 1;
+        for (int i = tid; i < used * COPIES * BINS; i += NT) copies[0][i] = 0u;
         __syncthreads();
-        for_each_scaled(l, s_begin, s_end, inv_t, add);
+        slice.each(add);
         __syncthreads();
-        cluster_sync();
-        if (rank == 0) {
-            for (int b = tid; b < 256; b += ST) {
-                unsigned n = 0u;
-                unsigned long long m = 0ull;
-                for (unsigned r = 0; r < CS; ++r) {
-                    n += ld_peer_u32(peer_smem(&hist[b], r));
-                    if (with_mass)
-                        m += (unsigned long long)ld_peer_u32(peer_smem(&mass3[0][b], r)) +
-                             ((unsigned long long)ld_peer_u32(peer_smem(&mass3[1][b], r)) << 14) +
-                             ((unsigned long long)ld_peer_u32(peer_smem(&mass3[2][b], r)) << 28);
-                }
-                tot_hist[b] = n;
-                tot_mass[b] = m;
-            }
-            __syncthreads();
-            if (tid < 32) choose();          // warp 0: lane j looks at the bins 8j..8j+7
+        for (int i = tid; i < used * 256; i += NT) {
+            const int h = i >> 8, b = i & 255;
+            unsigned sum = 0u;
+#pragma unroll
+            for (int c = 0; c < COPIES; ++c) sum += copies[h][c * BINS + b];
+            mine[h][b] = sum;
         }
         cluster_sync();
+        if (tid < 256) {
+            unsigned v[CS], n = 0u;
+#pragma unroll
+            for (unsigned r = 0; r < CS; ++r) v[r] = ld_peer_u32(peer_smem(&mine[0][tid], r));
+#pragma unroll
+            for (unsigned r = 0; r < CS; ++r) n += v[r];
+            tot_hist[tid] = n;
+        } else if (with_mass) {
+            const int b = tid - 256;
+            unsigned v[3][CS];
+            unsigned long long m = 0ull;
+#pragma unroll
+            for (unsigned r = 0; r < CS; ++r)
+#pragma unroll
+                for (int h = 0; h < 3; ++h) v[h][r] = ld_peer_u32(peer_smem(&mine[1 + h][b], r));
+#pragma unroll
+            for (unsigned r = 0; r < CS; ++r) m += (unsigned long long)v[0][r] + ((unsigned long long)v[1][r] << 14) + ((unsigned long long)v[2][r] << 28);
+            tot_mass[b] = m;
+        }
+        __syncthreads();
+        if (tid < 32) choose();          // warp 0: lane j looks at the bins 8j..8j+7
+        __syncthreads();
     };
+    static_assert(NT == 512, "the first 256 threads sum the counts, the others the masses");
 
     // ---- top-k: key of the k-th largest scaled logit (0 keeps everything)
     unsigned kth_key = 0u;
@@ -342,7 +406,7 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
             radix_pass(false,
                        [&](float x) {
                            const unsigned key = key_of(x);
-                           if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1u);
+                           if ((key & mask) == prefix) atomicAdd(&copies[0][copy + ((key >> shift) & 255u)], 1u);
                        },
                        [&]() {
                            // the highest bin b >= 1 with (elements in bins >= b) >= remaining, else bin 0; what is still to
@@ -373,18 +437,18 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
                                dec_remaining = has ? r : remaining - (all - tot_hist[0]);
                            }
                        });
-            prefix = ld_peer_u32(peer_smem(&dec_prefix, 0));
-            remaining = ld_peer_u32(peer_smem(&dec_remaining, 0));
+            prefix = dec_prefix;
+            remaining = dec_remaining;
         }
         kth_key = prefix;
     }
 
     // ---- normaliser over what top-k kept: threads, warps, CTAs in ascending order
     float z = 0.f;
-    for_each_scaled(l, s_begin, s_end, inv_t, [&](float x) {
+    slice.each_in_order([&](float x) {
         if (key_of(x) >= kth_key) z += weight(x - mx);
     });
-    z = cta_reduce(z, false);
+    z = cta_reduce(z, false, ST / 32);
     if (tid == 0) x_z = z;
     cluster_sync();
     z = 0.f;
@@ -405,8 +469,9 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
                        [&](float x) {
                            const unsigned key = key_of(x);
                            if (key >= kth_key && (key & mask) == prefix) {
-                               mass_add(mass3, (key >> shift) & 255u, (unsigned long long)(weight(x - mx) * fix_over_z));
-                               atomicAdd(&hist[(key >> shift) & 255u], 1u);
+                               const unsigned at = copy + ((key >> shift) & 255u);
+                               mass_add(copies, at, (unsigned long long)(weight(x - mx) * fix_over_z));
+                               atomicAdd(&copies[0][at], 1u);
                            }
                        },
                        [&]() {
@@ -449,8 +514,8 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
                                dec_above = chosen_above;
                            }
                        });
-            prefix = ld_peer_u32(peer_smem(&dec_prefix, 0));
-            above0 = ld_peer_u64(peer_smem(&dec_above, 0));
+            prefix = dec_prefix;
+            above0 = dec_above;
         }
         p_key = prefix;
         if (p_key < kth_key) p_key = kth_key;
@@ -467,8 +532,8 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
     long long tie_rank = 0;
     if (ties_kept >= 0) {
         int my_ties = 0;
-        for_chunk(l, begin, end, inv_t, [&](int, float x) { my_ties += key_of(x) == p_key; return true; });
-        tie_count[tid] = my_ties;
+        slice.chunk(begin, end, [&](int, float x) { my_ties += key_of(x) == p_key; return true; });
+        if (tid < ST) tie_count[tid] = my_ties;
         __syncthreads();
         if (tid < 32) {
             constexpr int G = ST / 32;
@@ -486,13 +551,13 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
         }
         __syncthreads();
         cluster_sync();
-        tie_rank = tie_count[tid];
+        tie_rank = tie_count[tid & (ST - 1)];
         for (unsigned r = 0; r < rank; ++r) tie_rank += (int)ld_peer_u32(peer_smem(&x_ties, r));
     }
     float csum = 0.f;
     {
         long long tr = tie_rank;
-        for_chunk(l, begin, end, inv_t, [&](int, float x) {
+        slice.chunk(begin, end, [&](int, float x) {
             const unsigned key = key_of(x);
             bool keep = key >= p_key;
             if (keep && ties_kept >= 0 && key == p_key) keep = (tr++) < ties_kept;
@@ -500,7 +565,7 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
             return true;
         });
     }
-    chunk_sum[tid] = csum;
+    if (tid < ST) chunk_sum[tid] = csum;
     __syncthreads();
     // The sums in a fixed order, in three levels: lane j of warp 0 adds the sums of the CTA's chunks 8j..8j+7 in order and
     // the 32 lane totals in order; the CTAs' totals are added in rank order. The CTA whose chunks hold the drawn point
@@ -575,7 +640,7 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
             float run = scratch[0];
             long long tr = tie_rank;
             int chosen = -1, last_kept = -1;
-            for_chunk(l, begin, end, inv_t, [&](int i, float x) {
+            slice.chunk(begin, end, [&](int i, float x) {
                 const unsigned key = key_of(x);
                 bool keep = key >= p_key;
                 if (keep && ties_kept >= 0 && key == p_key) keep = (tr++) < ties_kept;
@@ -585,7 +650,7 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
                 if (run > target) { chosen = i; return false; }
                 return true;
             });
-            out[row] = chosen >= 0 ? chosen : (last_kept >= 0 ? last_kept : 0);
+            out[row] = chosen >= 0 ? s_begin + chosen : (last_kept >= 0 ? s_begin + last_kept : 0);
         }
     }
     cluster_sync();         // nobody leaves while a peer may still read its shared memory
@@ -596,9 +661,15 @@ NIB_API int nib_sample(const float* logits, int rows, int vocab, const float* te
     NIB_REQUIRE(rows >= 0 && vocab > 0, "sample: bad sizes");
     if (rows == 0) return 0;
     NIB_REQUIRE((long long)vocab <= (1LL << 17) * 8, "sample: a row of %d logits is more than the fixed-point histograms hold", vocab);
+    const int per = (ceil_div(vocab, CS * ST) + 3) & ~3;
+    const size_t hist = sizeof(unsigned) * 4 * COPIES * BINS, slice = sizeof(float) * (size_t)ST * per;
+    const bool kept = hist + slice <= 200 * 1024;
+    const size_t smem = hist + (kept ? slice : 0);
+    if (kept) NIB_CUDA(cudaFuncSetAttribute(sample_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(rows * CS);
-    cfg.blockDim = dim3(ST);
+    cfg.blockDim = dim3(NT);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -607,7 +678,7 @@ NIB_API int nib_sample(const float* logits, int rows, int vocab, const float* te
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    NIB_CUDA(cudaLaunchKernelEx(&cfg, sample_kernel, logits, vocab, temperature, top_k, top_p, uniform, out));
+    NIB_CUDA(cudaLaunchKernelEx(&cfg, kept ? sample_kernel<true> : sample_kernel<false>, logits, vocab, temperature, top_k, top_p, uniform, out));
     NIB_LAUNCH_CHECK();
     return 0;
 }

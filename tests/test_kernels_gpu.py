@@ -844,3 +844,30 @@ def test_general_attention_segments(K, dtype, heads, kv_heads, hd, page, window)
         one = torch.empty(1, heads * hd, dtype=dtype, device="cuda")
         K.attention(qkv[i:i + 1].contiguous(), one, heads, kv_heads, hd, scale, window, alone, bt[i:i + 1].contiguous(), page, kp, vp)
         assert torch.equal(one[0], out[i])
+
+
+@pytest.mark.parametrize("vocab", [3, 2048, 2049, 32000, 151936, 151937, 389120, 389121, 700000])
+def test_sampling_slices(K, vocab):
+    """Slices of a row that are kept in shared memory and those that do not fit (more than 389,120 logits), rows that do not start
+    on 16 bytes, slices that are empty: the drawn token is the plain pipeline's wherever the number drawn is not within rounding
+    (1e-4 of the mass) of the border between two tokens, and a row's token does not depend on the rows beside it."""
+    rows = 5
+    logits = 2.0 * rnd((rows, vocab), torch.float32, 95)
+    logits[:, :: max(1, vocab // 37)] += 5.0
+    temperature = torch.tensor([0.7, 1.0, 0.8, 1.3, 0.9], device="cuda")
+    top_k = torch.tensor([0, 0, 40, 7, 1], dtype=torch.int32, device="cuda")
+    top_p = torch.tensor([1.0, 0.9, 1.0, 0.8, 1.0], device="cuda")
+    uniform = torch.tensor([0.31, 0.77, 0.12, 0.58, 0.5], device="cuda")
+    out, alone = (torch.empty(n, dtype=torch.int32, device="cuda") for n in (rows, 1))
+    K.sample(logits, temperature, top_k, top_p, uniform, out)
+    from plain_qwen2 import sampling_distribution
+    import numpy as np
+    for r in range(rows):
+        probs = sampling_distribution(logits[r].double().cpu().numpy(), [], float(temperature[r]), int(top_k[r]), float(top_p[r]), 1.0)
+        cdf = np.cumsum(probs) / probs.sum()
+        t, u = int(out[r]), float(uniform[r])
+        assert probs[t] > 0, (r, t)
+        assert (cdf[t - 1] if t else 0.0) - 1e-4 <= u <= cdf[t] + 1e-4, (r, t, u)
+        K.sample(logits[r:r + 1].clone(), temperature[r:r + 1], top_k[r:r + 1], top_p[r:r + 1], uniform[r:r + 1], alone)
+        # (a row that starts on 16 bytes adds up its normaliser in another order than one that does not)
+        assert int(alone[0]) == t or vocab % 4, (r, t)
