@@ -163,17 +163,19 @@ class Sampler:
         logit at temperature 1: of the elements that are kept (the maxima) the first in vocabulary order is taken,
         which is what the argmax kernel gives."""
         n = len(rows)
-        par = np.empty((4, n), dtype=np.float32)
-        par[0] = [1.0 if r.params.greedy else r.params.temperature for r in rows]
-        par[1].view(np.int32)[:] = [1 if r.params.greedy else r.params.k for r in rows]
-        par[2] = [1.0 if r.params.greedy else r.params.p for r in rows]
-        par[3] = [0.0 if r.params.greedy else uniform_for(r.seed, r.generated) for r in rows]
-        if torch.device(dev).type == "cuda":
-            if stage is None:
-                _, stage = self._pinned_pair(n)
-            stage[:4 * n].numpy()[:] = par.reshape(-1)
+        temperature, top_k, top_p, uniform = [1.0] * n, [1] * n, [1.0] * n, [0.0] * n
+        for i, r in enumerate(rows):
+            p = r.params
+            if not p.greedy:
+                temperature[i], top_k[i], top_p[i], uniform[i] = p.temperature, p.k, p.p, uniform_for(r.seed, r.generated)
+        on_gpu = torch.device(dev).type == "cuda"
+        if on_gpu and stage is None:
+            _, stage = self._pinned_pair(n)
+        host = stage[:4 * n] if on_gpu else torch.empty(4 * n, dtype=torch.float32)
+        par = host.numpy().reshape(4, n)
+        par[0], par[1].view(np.int32)[:], par[2], par[3] = temperature, top_k, top_p, uniform
+        d = host
+        if on_gpu:
             d = torch.empty(4 * n, dtype=torch.float32, device=dev)
-            d.copy_(stage[:4 * n], non_blocking=True)
-        else:
-            d = torch.from_numpy(par.reshape(-1).copy())
+            d.copy_(host, non_blocking=True)
         return d[:n], d[n:2 * n].view(torch.int32), d[2 * n:3 * n], d[3 * n:]
