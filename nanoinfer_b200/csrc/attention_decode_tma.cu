@@ -31,9 +31,11 @@
 // Formula as in attention_generic.cu (cpp/src/ops.cpp:206-270). The reference's decode attention is a
 // SIMT split-KV kernel with a combine pass (cpp/src/cuda/cuda_backend.cu:578-640, :331-352).
 #include "attention_common.cuh"
-#include "pipeline.cuh"
+#include "tcgen05.cuh"
 
 using namespace nibp;
+using nibt::elect_one;
+using nibt::uniform_warp;
 
 extern "C" int nib_attention_combine(const float* part_o, const float* part_ml, void* out, int rows, int splits,
                                      int head_dim, cudaStream_t stream);
@@ -85,7 +87,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
 
     pdl_launch_dependents();
     const int split = blockIdx.x, token = blockIdx.y, kvh = blockIdx.z;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31, g = lane >> 2, t = lane & 3;
     if (tid == 0) nib_trace_mark(trace, trace_cap, NIB_TK_ATTN_DECODE, 0, 0);
     const int p = ctx_lens[token] - 1;                     // the token's own position; -1: a padding row
     const int lo = window > 0 ? max(0, p - window + 1) : 0;
@@ -115,9 +117,10 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
 #pragma unroll
     for (int nh = 0; nh < NH; ++nh) { m_run[nh][0] = m_run[nh][1] = -INFINITY; l_part[nh][0] = l_part[nh][1] = 0.f; }
     if (warp == WARPS) {
-        // ---------------- producer warp: lane i fetches page i of every tile (K and V), lane 0 arms the
-        // stage's barrier. The block-table entry of the next tile is read while this one waits for its
-        // stage. Keys and values of earlier positions were written by earlier steps, so their tiles are
+        // ---------------- producer warp: lane i looks page i of every tile up, one thread arms the stage's barrier and sends
+        // for the pages' keys and values (lanes that sent for a page each took turns, 150 cycles an instruction: 2,500 for a
+        // tile of eight pages, the whole kernel's pace). The block-table entry of the next tile is read while this one waits for
+        // its stage. Keys and values of earlier positions were written by earlier steps, so their tiles are
         // fetched at once, before the step's earlier kernels have finished. The tile that holds p holds this
         // step's own key and value, written by the kernel before this one: with own_kv the consumers take
         // them from the activation buffer instead (below) and no fetch waits; without, that tile's does.
@@ -137,21 +140,24 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __g
             const int z = z_next;
             z_next = plane_of(j + 1);
             if (!own_kv && t_begin + j == t_last && !waited) { pdl_wait(); waited = true; }
-            int ok = 1;
-            if (lane == 0) {
-                if (j >= stages) ok = !s_failed && mbar_wait(&empty[st], ((j / stages) - 1) & 1);
-                if (ok) mbar_expect_tx(&full[st], C::STAGE);
-                else if (!s_failed) { atomicCAS(&g_dec_error, 0, (2 << 16) | (int)(blockIdx.x & 0xffff)); s_failed = 1; }
+            if (j >= stages && !__all_sync(0xffffffffu, mbar_wait(&empty[st], ((j / stages) - 1) & 1))) {
+                if (lane == 0 && !s_failed) { atomicCAS(&g_dec_error, 0, (2 << 16) | (int)(blockIdx.x & 0xffff)); s_failed = 1; }
+                break;
             }
-            ok = __shfl_sync(0xffffffffu, ok, 0);
-            if (!ok) break;
-            if (lane < pages_per_tile) {
-                unsigned char* kd = smem + st * C::STAGE + ((lane << page_shift) * 128);
+            if (elect_one()) mbar_expect_tx(&full[st], C::STAGE);
+            __syncwarp();
+            unsigned char* kd = smem + st * C::STAGE;
+            for (int i = 0; i < pages_per_tile; ++i) {
+                const int zi = __shfl_sync(0xffffffffu, z, i);
+                if (elect_one()) {
 #pragma unroll
-                for (int s = 0; s < C::SUB; ++s) {
-                    tma_load_3d(kd + s * SUBTILE, &map_k, &full[st], s * 64, 0, z);
-                    tma_load_3d(kd + C::TILE + s * SUBTILE, &map_v, &full[st], s * 64, 0, z);
+                    for (int s = 0; s < C::SUB; ++s) {
+                        tma_load_3d(kd + s * SUBTILE, &map_k, &full[st], s * 64, 0, zi);
+                        tma_load_3d(kd + C::TILE + s * SUBTILE, &map_v, &full[st], s * 64, 0, zi);
+                    }
                 }
+                __syncwarp();
+                kd += page_size * 128;
             }
             issued = j + 1;
         }

@@ -627,7 +627,13 @@ class Kernels:
                       head_dim: int = 128) -> int:
         """Into how many CTAs the keys of a decoding token are split. The kernel with TMA page loads keeps
         several tiles in flight per CTA: about 256 CTAs in all (measured best from 1 to 64 requests), at
-        least four of its tiles (128 keys for heads of 64, else 64) each. The cp.async kernel: two key tiles per CTA (both are in flight at once, so a
+        least four of its tiles (128 keys for heads of 64, else 64) each. While that leaves SMs without work, up to eight CTAs
+        that merge in one cluster and a tile each will do, as long as every CTA has an SM (one token of 777 keys, heads of 64:
+        3.7 us with eight, 6.7 with one; 4 tokens of 1,500: 4.8 and 6.9 with two; 24 tokens of up to 1,500: 7.0 with two, 7.4
+        with four, 11.6 with one), but not with a window, whose few tiles come at any context. More than one cluster of eight
+        a token and kv head, and with it a second kernel, only where eight leave SMs idle
+        (heads of 128, 8 tokens of 4,096: 11.4 us with 8, 13.0 with 16; 1 token: 9.3 and 8.9). The cp.async kernel: two key tiles
+        per CTA (both are in flight at once, so a
         CTA waits for memory once), as long as that does not make more CTAs than fill the GPU about eight
         times."""
         if self.options.fixed_decode_splits:
@@ -635,9 +641,15 @@ class Kernels:
         keys = min(max_ctx, window) if window > 0 else max_ctx
         tiles = -(-keys // 64) + 1
         if tma:
-            want = max(1, round(256 / max(1, n_tokens * kv_heads)))
+            units = max(1, n_tokens * kv_heads)
+            want = max(1, round(256 / units))
             tile_keys = 128 if head_dim == 64 else 64           # the kernel's tile
-            n = max(1, min(want, -(-keys // tile_keys) // 4, 64))
+            tiles = -(-keys // tile_keys)
+            n = max(1, min(want, tiles // 4, 64))
+            if window <= 0 and units <= self.sm_count:
+                n = max(n, min(8, 1 << (self.sm_count // units).bit_length() - 1, 1 << (tiles - 1).bit_length()))
+            if n > 8 and 8 * units >= 128:
+                n = 8
             return _cluster_splits(n)
         most = max(1, (8 * self.sm_count) // max(1, n_tokens * kv_heads))
         return max(1, min(-(-tiles // 2), most, 64))
