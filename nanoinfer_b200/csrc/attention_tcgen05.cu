@@ -2,21 +2,27 @@
 // bfloat16 and head sizes 64 and 128.
 //
 // A CTA owns a tile of up to 128 rows, where a row is one (token, query head of the kv group): the keys and
-// values of a kv head are read once for all the query heads that share it. For every block of 128 (heads of
-// 128: 64) keys:
-//         S = Q . K^T         (tcgen05.mma, accumulator S in tensor memory, two buffers)
+// values of a kv head are read once for all the query heads that share it. For every block of 128 keys:
+//         S = Q . K^T         (tcgen05.mma, accumulator S in tensor memory)
 //         P = exp2(S*scale - max), row sums       (a thread per row: no exchange between threads)
-//         O += P . V          (tcgen05.mma, P from shared memory (two buffers), V as the MN-major operand; O
-//                              stays in tensor memory over all blocks)
-// The scores of block j+1 are multiplied while the softmax of block j runs, and P.V of block j while the softmax
-// of block j+1 runs: the softmax warps, which bound the kernel (exponentials), never wait for the tensor core.
+//         O += P . V          (tcgen05.mma, P from tensor memory, V as the MN-major operand; O stays in tensor memory
+//                              over all blocks)
+// TWO CTAs share an SM (256 columns of tensor memory, half of the shared memory and of the registers each): while one
+// waits for its scores, its keys, its first block or its next tile, the other's softmax has the exponential unit, which
+// bounds the kernel (16 a clock and SM: 1,024 cycles for a tile's block; the two products take 512 at heads of 64, 1,024 at
+// heads of 128). Heads of 64: scores, probabilities and output have columns of their own, so the scores of block j+1 are
+// multiplied as soon as those of block j are in registers. Heads of 128: the probabilities overwrite the scores they come
+// from, and keys and values have one stage each, whose next copies run under the softmax. Against one CTA an SM with two
+// threads a row, probabilities through shared memory and blocks of 64 keys at heads of 128 (us a launch, that one
+// first): 2,048 tokens of 14 query and 2 key heads of 64, 27 and 29; 601 + 461 + 320 tokens of them, 13.7 and 11.8; 4,096 tokens
+// behind 4,096, 207 and 150; 2,048 behind 14,336, 12 and 2 heads of 128, 596 and 217; 2 x 4,096, 28 and 4 heads of 128, 806 and 235.
 // The running maximum that the exponents refer to is only replaced when the row's maximum grew by more than
 // 2^8; only then is the row of O rescaled (read from tensor memory, multiplied, written back). At the end O is
 // read once and divided by the sum.
 // Q, K and V tiles arrive by TMA (cp.async.bulk.tensor, 128-byte swizzle): Q through a 3-D map over
 // (head dim, heads of the group, tokens), K and V through a 3-D map over the page pool, one box per
 // page of the block table; a page the request does not hold is fetched from an out-of-range coordinate
-// and arrives as zeros. Roles: warp 0 = TMA producer, warp 1 = MMA issuer and TMEM owner, warps 4..7 =
+// and arrives as zeros. Roles: warp 0 = TMA producer, warp 1 = MMA issuer and TMEM owner, warps 2..5 =
 // softmax and output. Every wait is bounded; a wait that runs out records an error word, the CTA stops,
 // drains its copies, frees its TMEM and returns.
 //
@@ -31,6 +37,7 @@
 // Formula as in attention_generic.cu (cpp/src/ops.cpp:206-270); the reference's prefill attention is a
 // SIMT kernel with 32-key shared-memory slabs (cpp/src/cuda/cuda_backend.cu:489-575).
 #include "tcgen05.cuh"
+#include <type_traits>
 
 using namespace nibp;
 using namespace nibt;
@@ -38,7 +45,8 @@ using namespace nibt;
 namespace {
 
 constexpr int ROWS = 128;        // rows of a tile (UMMA M): TMEM lanes
-constexpr int THREADS = 384;     // TMA warp, MMA warp, two idle warps; eight softmax warps (two threads per row, half of a block's keys each)
+constexpr int THREADS = 192;     // TMA warp, MMA warp, four softmax warps (a thread per row)
+constexpr int KEYS = 128;        // keys per block (UMMA N of S, K of P.V)
 constexpr float LOG2E = 1.4426950408889634f;
 
 __device__ int g_attn_error = 0;
@@ -53,6 +61,7 @@ __device__ __forceinline__ bool mbar_spin(unsigned long long* bar, unsigned pari
     }
     return false;
 }
+__device__ __forceinline__ bool warp_spin(unsigned long long* bar, unsigned parity) { return __all_sync(0xffffffffu, mbar_spin(bar, parity)); }
 __device__ __forceinline__ unsigned pack2(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<unsigned*>(&v);
@@ -62,25 +71,62 @@ __device__ __forceinline__ float ex2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// Keys per block: 128 for heads of 64; 64 for heads of 128, where two query tiles, the key and value stages and two
-// tiles of probabilities of 128 keys would not fit the shared memory of an SM.
-template <int HD> constexpr int keys_of() { return HD == 64 ? 128 : 64; }
-
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float y;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+    return y;
+}
+// Two floats side by side: one instruction of the fused multiply-add unit works on both.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 two(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void split(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// 2^x of two numbers in the multiply-add unit, for -126 <= x < 127: x = n + f with n the nearest whole number (the low bits of
+// x + 1.5 * 2^23), 2^f on [-1/2, 1/2] by a polynomial of degree 5 (Remez exchange for the relative error: 7.5e-8, 2.1e-7 as
+// evaluated here; ex2.approx allows itself 2.4e-7), n added to the exponent.
+__device__ __forceinline__ void exp2_fma(f32x2 x, float& p0, float& p1) {
+    float x0, x1;
+    split(x, x0, x1);
+    x = two(fmaxf(x0, -126.f), fmaxf(x1, -126.f));
+    const f32x2 magic = two(12582912.f, 12582912.f);
+    const f32x2 n = add2(x, magic);
+    const f32x2 f = fma2(add2(n, two(-12582912.f, -12582912.f)), two(-1.f, -1.f), x);
+    f32x2 p = fma2(two(1.3276472454890609e-3f, 1.3276472454890609e-3f), f, two(9.675540961325169e-3f, 9.675540961325169e-3f));
+    p = fma2(p, f, two(5.550713092088699e-2f, 5.550713092088699e-2f));
+    p = fma2(p, f, two(0.24022120237350464f, 0.24022120237350464f));
+    p = fma2(p, f, two(0.6931469440460205f, 0.6931469440460205f));
+    p = fma2(p, f, two(1.0000001192092896f, 1.0000001192092896f));
+    float n0, n1;
+    split(n, n0, n1);
+    split(p, p0, p1);
+    p0 = __int_as_float(__float_as_int(p0) + (__float_as_int(n0) << 23));
+    p1 = __int_as_float(__float_as_int(p1) + (__float_as_int(n1) << 23));
+}
 template <int HD> struct Cfg {
-    static constexpr int KEYS = keys_of<HD>();                // keys per block (UMMA N of S, K of P.V)
     static constexpr int SUB = HD / 64;                       // sub-tiles of 64 elements (128 bytes) along the head dim
-    static constexpr int PSUB = KEYS / 64;                    // sub-tiles of 64 keys of a tile of probabilities
     static constexpr int SUBTILE = 128 * 128;                 // bytes of a [128 rows x 64 elements] sub-tile
     static constexpr int Q_BYTES = SUB * SUBTILE;             // the tile of queries
     static constexpr int KV_BYTES = KEYS * HD * 2;            // one block of keys (or values)
-    static constexpr int P_BYTES = PSUB * SUBTILE;            // [128 rows x KEYS]
-    static constexpr int STAGES = 2;
-    static constexpr int OFF_Q = 0, OFF_K = Q_BYTES, OFF_V = OFF_K + STAGES * KV_BYTES, OFF_P = OFF_V + STAGES * KV_BYTES;
-    static constexpr int OFF_BAR = OFF_P + 2 * P_BYTES;
-    static constexpr int OFF_XCH = OFF_BAR + 256;             // what the two threads of a row tell each other: [3][2][128] floats
-    static constexpr int SMEM = OFF_XCH + 3 * 2 * 128 * 4 + 1024;
-    static constexpr int COL_S = 0, COL_O = 2 * KEYS;         // two buffers of scores, then the output
-    static constexpr int TMEM_COLS = (2 * KEYS + HD) <= 256 ? 256 : 512;
+    static constexpr int STAGES = HD == 64 ? 2 : 1;
+    static constexpr int OFF_Q = 0, OFF_K = Q_BYTES, OFF_V = OFF_K + STAGES * KV_BYTES, OFF_BAR = OFF_V + STAGES * KV_BYTES;
+    static constexpr int SMEM = OFF_BAR + 256 + 1024;
+    static constexpr bool P_OWN = HD == 64;                   // the probabilities have columns of their own
+    static constexpr int COL_S = 0, COL_P = P_OWN ? KEYS : 0, COL_O = P_OWN ? KEYS + KEYS / 2 : KEYS;
+    static constexpr int TMEM_COLS = 256;
+    static_assert(COL_O + HD <= TMEM_COLS, "two CTAs share an SM's tensor memory");
 };
 
 // The running maximum of a row is replaced by a larger one only when it grew by more than this (in log2 units):
@@ -88,18 +134,22 @@ template <int HD> struct Cfg {
 // Meanwhile probabilities are at most 2^8, harmless in bfloat16 and in the 32-bit sums.
 constexpr float RESCALE_ABOVE = 8.0f;
 
-// grid: (row tiles, requests, kv heads)
+// Of 16 pairs of exponentials, how many go to the multiply-add unit: at heads of 128, 2,048 tokens behind 14,336 (12 query and 2
+// key heads), 0 / 3 / 6 of them took 243 / 223 / 270 us, at heads of 64, 4,096 behind 4,096, 150 / 150 / 166.
+template <int HD> constexpr int EMULATED = HD == 128 ? 3 : 0;
+
+// grid: row tiles x requests x kv heads, the kv head fastest: the tiles that see the most keys start first
 template <int HD, bool FLEX>
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__(THREADS, 2)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                             const __grid_constant__ CUtensorMap map_v, __nv_bfloat16* __restrict__ out,
                             const int* __restrict__ q_start, const int* __restrict__ ctx_lens,
-                            const int* __restrict__ block_table, int bt_stride, int page_size, int num_pages,
+                            const int* __restrict__ block_table, int bt_stride, int page_size, int num_pages, int n_req,
                             int heads, int kv_heads, float scale, int window, unsigned long long* trace, int trace_cap,
                             float softcap, int chunk, const float* __restrict__ sinks, float out_scale, int keep_first,
                             const float* __restrict__ gate, int ld_gate) {
     using C = Cfg<HD>;
-    constexpr int KEYS = C::KEYS, STAGES = C::STAGES;
+    constexpr int STAGES = C::STAGES;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned long long* bars = reinterpret_cast<unsigned long long*>(smem + C::OFF_BAR);
@@ -108,24 +158,24 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     unsigned long long* k_empty = bars + 3;
     unsigned long long* v_full = bars + 5;
     unsigned long long* v_empty = bars + 7;
-    // One barrier per BUFFER (of scores in tensor memory, of probabilities in shared memory): a buffer's next phase
-    // cannot complete before its last one was seen, which a single barrier shared by both buffers would not ensure.
-    unsigned long long* s_full = bars + 9;        // [2] the scores of a block are in buffer b
-    unsigned long long* p_full = bars + 11;       // [2] 256 arrivals: the probabilities of a block are in buffer b
-    unsigned long long* o_done = bars + 13;       // [2] P.V of the block whose probabilities were in buffer b has been added
-    unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 15);
-    unsigned long long* pair_bar = bars + 16;     // [4] the two softmax warps of a lane quadrant meet here (one arrival each)
+    // phase j of each of these belongs to block j; no phase can complete before the one before it was seen
+    unsigned long long* s_full = bars + 9;        // the scores are in tensor memory
+    unsigned long long* s_empty = bars + 10;      // P_OWN: ... and in registers (an arrival per softmax warp)
+    unsigned long long* p_full = bars + 11;       // [2] the probabilities of a half of the keys are in tensor memory (an arrival per softmax warp)
+    unsigned long long* o_done = bars + 13;       // P.V has been added
+    unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 14);
     __shared__ volatile int s_failed;
 
     pdl_launch_dependents();
     if (threadIdx.x == 0) nib_trace_mark(trace, trace_cap, NIB_TK_ATTN_PREFILL, 0, 0);
-    const int req = blockIdx.y, kvh = blockIdx.z;
     const int n_rep = heads / kv_heads;
     const int tpt = ROWS / n_rep;                         // tokens per tile
     const int rows_tile = tpt * n_rep;
+    const int kvh = blockIdx.x % kv_heads, req = (blockIdx.x / kv_heads) % n_req, tile = blockIdx.x / (kv_heads * n_req);
+    const int n_tiles = gridDim.x / (kv_heads * n_req);
     const int row_begin = q_start[req], q_len = q_start[req + 1] - row_begin;
     // tiles late in the portion see the most keys: they start first
-    const int tok0 = (gridDim.x - 1 - blockIdx.x) * tpt;  // first token of this tile within the request's portion
+    const int tok0 = (n_tiles - 1 - tile) * tpt;          // first token of this tile within the request's portion
     if (tok0 >= q_len) return;
     const int n_tok = min(tpt, q_len - tok0);
     const int ctx = ctx_lens[req];
@@ -137,7 +187,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     const int n_kept = FLEX ? min((keep_first + KEYS - 1) / KEYS, b_begin) : 0;      // key blocks with kept tokens before the window's first
     const int n_blk = n_kept + hi_cta / KEYS - b_begin + 1;
     auto block_at = [&](int j) { return FLEX && j < n_kept ? j : b_begin + j - n_kept; };
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int* bt = block_table + (size_t)req * bt_stride;
 
     if (threadIdx.x == 0) {
@@ -146,14 +196,15 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         prefetch_tensormap(&map_k);
         prefetch_tensormap(&map_v);
         mbar_init(q_full, 1);
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < STAGES; ++i) {
             mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1);
             mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);
-            mbar_init(&s_full[i], 1);
-            mbar_init(&p_full[i], 256);
-            mbar_init(&o_done[i], 1);
         }
-        for (int i = 0; i < 4; ++i) mbar_init(&pair_bar[i], 2);
+        mbar_init(s_full, 1);
+        mbar_init(s_empty, 4);
+        mbar_init(&p_full[0], 4);
+        mbar_init(&p_full[1], 4);
+        mbar_init(o_done, 1);
         mbar_fence_init();
     }
     if (warp == 1) {
@@ -163,138 +214,133 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const unsigned tmem_base = *tmem_slot;
+    // The producer's look-ups: a lane's block-table entry of block j, or -1 where there is no page to fetch. The entry of block
+    // j+1 is asked for while block j is being sent for and is looked at only a block later (the first before the wait for the
+    // kernel before this one: no kernel writes the table): the look-up's latency (more than half a microsecond) must not stand
+    // between two blocks' copies.
+    const int pages_per_block = KEYS / page_size;
+    const int oob = num_pages * kv_heads;             // a coordinate outside the pool: the box arrives as zeros
+    auto entry_of = [&](int j) -> int {
+        const int key = block_at(j) * KEYS + lane * page_size;
+        if (lane >= pages_per_block || key > hi_cta || (key + page_size <= lo_cta && !(FLEX && key < keep_first))) return -1;
+        return __ldg(bt + key / page_size);
+    };
+    const int entry_first = warp == 0 ? entry_of(0) : -1;
+    const unsigned tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     pdl_wait();
     if (threadIdx.x == 0) nib_trace_mark(trace, trace_cap, NIB_TK_ATTN_PREFILL, 0, 1);
 
     if (warp == 0) {
-        // ---------------- producer: lane 0 fetches Q and arms the barriers; lane i fetches page i of every block of
-        // keys (its block-table entry is read one block ahead, so that the look-up of a page never stands between
-        // two copies)
-        if (lane == 0) {
+        // ---------------- producer: one thread fetches Q, arms the barriers and fetches the pages of every block of keys;
+        // lane i looks page i up, one block ahead, so that the look-up of a page never stands between two copies
+        if (elect_one()) {
             mbar_expect_tx(q_full, (unsigned)(rows_tile * 128 * C::SUB));
 #pragma unroll
             for (int s = 0; s < C::SUB; ++s)
                 tma_load_3d(smem + C::OFF_Q + s * C::SUBTILE, &map_q, q_full, s * 64, kvh * n_rep, row_begin + tok0);
         }
-        const int pages_per_block = KEYS / page_size;
-        const int oob = num_pages * kv_heads;             // a coordinate outside the pool: the box arrives as zeros
-        // This lane's block-table entry of block j, or -1 where it has no page to fetch there. The entry of block j+1 is
-        // asked for while block j is being sent for and is looked at only a block later: the look-up's latency (more
-        // than half a microsecond) must not stand between two blocks' copies.
-        auto entry_of = [&](int j) -> int {
-            const int key = block_at(j) * KEYS + lane * page_size;
-            if (lane >= pages_per_block || key > hi_cta || (key + page_size <= lo_cta && !(FLEX && key < keep_first))) return -1;
-            return __ldg(bt + key / page_size);
-        };
-        int entry_next = entry_of(0);
+        __syncwarp();
+        int entry_next = entry_first;
         int issued = 0;
-        for (int j = 0; j < n_blk; ++j) {
+        bool ok = true;
+        for (int j = 0; j < n_blk && ok; ++j) {
             const int st = j % STAGES;
             const int entry = entry_next;
             if (j + 1 < n_blk) entry_next = entry_of(j + 1);
             const int z = (entry >= 0 && entry < num_pages) ? entry * kv_heads + kvh : oob;      // third coordinate of the page
-            // keys first (the scores of this block are wanted a whole block ahead), values when their stage is free
+            // keys first (the scores are wanted before the values), values when their stage is free
             const unsigned par = ((j / STAGES) & 1) ^ 1;
-            int ok = 1;
 #pragma unroll
             for (int kv = 0; kv < 2; ++kv) {
-                unsigned long long* empty = kv ? &v_empty[st] : &k_empty[st];
                 unsigned long long* full = kv ? &v_full[st] : &k_full[st];
-                if (lane == 0) {
-                    ok = !s_failed && mbar_wait(empty, par);
-                    if (ok) mbar_expect_tx(full, C::KV_BYTES);
-                    else if (!s_failed) { atomicCAS(&g_attn_error, 0, (1 << 16) | (int)(blockIdx.x & 0xffff)); s_failed = 1; }
-                }
-                ok = __shfl_sync(0xffffffffu, ok, 0);
+                ok = __all_sync(0xffffffffu, mbar_spin(kv ? &v_empty[st] : &k_empty[st], par));
                 if (!ok) break;
-                if (lane < pages_per_block) {
+                if (elect_one()) mbar_expect_tx(full, C::KV_BYTES);
+                __syncwarp();
+                unsigned char* to = smem + (kv ? C::OFF_V : C::OFF_K) + st * C::KV_BYTES;
+                for (int i = 0; i < pages_per_block; ++i) {
+                    const int zi = __shfl_sync(0xffffffffu, z, i);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int s = 0; s < C::SUB; ++s)
-                        tma_load_3d(smem + (kv ? C::OFF_V : C::OFF_K) + st * C::KV_BYTES + s * (KEYS * 128) + lane * page_size * 128,
-                                    kv ? &map_v : &map_k, full, s * 64, 0, z);
+                        for (int s = 0; s < C::SUB; ++s)
+                            tma_load_3d(to + s * (KEYS * 128) + i * page_size * 128, kv ? &map_v : &map_k, full, s * 64, 0, zi);
+                    }
+                    __syncwarp();
                 }
+                issued = 2 * j + kv + 1;
             }
-            if (!ok) break;
-            issued = j + 1;
         }
+        if (!ok && lane == 0 && !s_failed) { atomicCAS(&g_attn_error, 0, (1 << 16) | (int)(blockIdx.x & 0xffff)); s_failed = 1; }
         if (s_failed && lane == 0) {
             // copies already issued still target this CTA's shared memory: wait for them, bounded
             mbar_wait(q_full, 0);
-            for (int j = max(0, issued - STAGES); j < issued; ++j) {
+            for (int j = max(0, issued / 2 - STAGES); j < (issued + 1) / 2; ++j) {
                 mbar_wait(&k_full[j % STAGES], (j / STAGES) & 1);
-                mbar_wait(&v_full[j % STAGES], (j / STAGES) & 1);
+                if (2 * j + 1 < issued) mbar_wait(&v_full[j % STAGES], (j / STAGES) & 1);
             }
         }
-    } else if (warp == 1 && lane == 0) {
-        // ---------------- MMA issuer: S(0); then for every block j: S(j+1) into the other buffer of scores at once (so
-        // the softmax of block j+1 never waits for the tensor core), and O += P(j) . V(j) when P(j) is there.
+    } else if (warp == 1) {
+        // ---------------- MMA issuer. Products run in the order of issue, so where the probabilities lie on the scores
+        // the next scores are issued behind the P.V that reads them.
         constexpr unsigned idesc_s = instr_desc(ROWS, KEYS, false);
         constexpr unsigned idesc_o = instr_desc(ROWS, HD, true);
         const unsigned q_addr = smem_u32(smem + C::OFF_Q);
-        auto issue_qk = [&](int j) {
+        auto issue_qk = [&](int j) -> bool {
+            if (!warp_spin(&k_full[j % STAGES], (j / STAGES) & 1)) return false;
+            if (C::P_OWN && j > 0 && !warp_spin(s_empty, (j - 1) & 1)) return false;
+            tc_fence_after();
             const unsigned k_addr = smem_u32(smem + C::OFF_K + (j % STAGES) * C::KV_BYTES);
+            if (elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < HD / 16; ++kk) {
-                const unsigned long long adv = (unsigned long long)(((kk & 3) * 32) >> 4);
-                tc_mma(tmem_base + C::COL_S + (j & 1) * KEYS, desc_kmajor(q_addr + (kk >> 2) * C::SUBTILE) + adv,
-                       desc_kmajor(k_addr + (kk >> 2) * (KEYS * 128)) + adv, idesc_s, kk > 0);
+                for (int kk = 0; kk < HD / 16; ++kk) {
+                    const unsigned long long adv = (unsigned long long)(((kk & 3) * 32) >> 4);
+                    tc_mma(tmem_base + C::COL_S, desc_kmajor(q_addr + (kk >> 2) * C::SUBTILE) + adv,
+                           desc_kmajor(k_addr + (kk >> 2) * (KEYS * 128)) + adv, idesc_s, kk > 0);
+                }
+                tc_commit(s_full);
+                tc_commit(&k_empty[j % STAGES]);
             }
-            tc_commit(&s_full[j & 1]);
-            tc_commit(&k_empty[j % STAGES]);
+            __syncwarp();
+            return true;
         };
-        auto issue_pv = [&](int j) {
-            const unsigned p_addr = smem_u32(smem + C::OFF_P + (j & 1) * C::P_BYTES);
+        auto issue_pv = [&](int j) -> bool {
+            if (!warp_spin(&v_full[j % STAGES], (j / STAGES) & 1)) return false;
             const unsigned v_addr = smem_u32(smem + C::OFF_V + (j % STAGES) * C::KV_BYTES);
 #pragma unroll
-            for (int kk = 0; kk < KEYS / 16; ++kk) {
-                // P: sub-tile kk/4 (64 keys each), 32 bytes per step inside it; V: 16 keys = 2048 bytes further down,
-                // the second 64 elements of the head dim KEYS*128 bytes further on
-                const unsigned long long a = desc_kmajor(p_addr + (kk >> 2) * C::SUBTILE) + (unsigned long long)(((kk & 3) * 32) >> 4);
-                const unsigned long long b = desc_mnmajor(v_addr + kk * 16 * 128, KEYS * 128);
-                tc_mma(tmem_base + C::COL_O, a, b, idesc_o, j > 0 || kk > 0);
-            }
-            tc_commit(&o_done[j & 1]);
-            tc_commit(&v_empty[j % STAGES]);
-        };
-        bool ok = mbar_spin(q_full, 0) && mbar_spin(&k_full[0], 0);
-        if (!ok) { atomicCAS(&g_attn_error, 0, (2 << 16) | (int)(blockIdx.x & 0xffff)); s_failed = 1; }
-        if (ok) { tc_fence_after(); issue_qk(0); }
-        for (int j = 0; j < n_blk && ok; ++j) {
-            if (j + 1 < n_blk) {
-                // the other buffer of scores is free: the probabilities of block j-1 were complete before its P.V
-                ok = mbar_spin(&k_full[(j + 1) % STAGES], ((j + 1) / STAGES) & 1);
-                if (!ok) break;
+            for (int half = 0; half < 2; ++half) {          // of the keys, as their probabilities come
+                if (!warp_spin(&p_full[half], j & 1)) return false;
                 tc_fence_after();
-                issue_qk(j + 1);
+                if (elect_one()) {
+#pragma unroll
+                    for (int kk = half * (KEYS / 32); kk < (half + 1) * (KEYS / 32); ++kk) {
+                        // P: 16 keys are 8 columns; V: 16 keys = 2048 bytes further down, the second 64 elements of the head
+                        // dim KEYS*128 bytes further on
+                        const unsigned long long b = desc_mnmajor(v_addr + kk * 16 * 128, KEYS * 128);
+                        tc_mma_ts(tmem_base + C::COL_O, tmem_base + C::COL_P + kk * 8, b, idesc_o, j > 0 || kk > 0);
+                    }
+                    if (half == 1) {
+                        tc_commit(o_done);
+                        tc_commit(&v_empty[j % STAGES]);
+                    }
+                }
+                __syncwarp();
             }
-            ok = mbar_spin(&p_full[j & 1], (j >> 1) & 1) && mbar_spin(&v_full[j % STAGES], (j / STAGES) & 1);
-            if (!ok) break;
-            tc_fence_after();
-            issue_pv(j);
-        }
-        if (!ok && !s_failed) { atomicCAS(&g_attn_error, 0, (3 << 16) | (int)(blockIdx.x & 0xffff)); s_failed = 1; }
-    } else if (warp >= 4) {
-        // ---------------- softmax and output: two threads own a row, in warps that may read the same TMEM lanes
-        // (32*(warp%4)...): each takes half of a block's keys and half of the output row's columns. They tell each other
-        // the maximum of their halves (and at the end the sum) through shared memory, meeting at a barrier of their two
-        // warps. Rows past the tile's last (the tile holds a whole number of tokens) see what the last row sees; nothing
-        // of them is stored.
-        constexpr int HK = KEYS / 2;                      // keys of a block per thread
-        const int quad = warp & 3, half = (warp - 4) >> 2, row = quad * 32 + lane;
-        const unsigned lane_addr = tmem_base + ((unsigned)(quad * 32) << 16);
-        const unsigned o_addr = lane_addr + C::COL_O + half * (HD / 2);
-        float* xch = reinterpret_cast<float*>(smem + C::OFF_XCH);        // [3][2][128]
-        // the meeting of the two warps of a quadrant: an mbarrier, so that the wait is bounded like every other (a warp
-        // that has given up never arrives, and its partner then gives up too instead of waiting for ever)
-        unsigned pair_phase = 0;
-        auto pair_sync = [&]() -> bool {
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&pair_bar[quad]);
-            const bool met = mbar_spin(&pair_bar[quad], pair_phase & 1);
-            ++pair_phase;
-            return __all_sync(0xffffffffu, met);
+            return true;
         };
+        bool ok = warp_spin(q_full, 0) && issue_qk(0);
+        for (int j = 0; j < n_blk && ok; ++j) {
+            if (C::P_OWN && j + 1 < n_blk) ok = issue_qk(j + 1);
+            ok = ok && issue_pv(j);
+            if (!C::P_OWN && j + 1 < n_blk) ok = ok && issue_qk(j + 1);
+        }
+        if (!ok && lane == 0 && !s_failed) { atomicCAS(&g_attn_error, 0, (3 << 16) | (int)(blockIdx.x & 0xffff)); s_failed = 1; }
+    } else if (warp >= 2) {
+        // ---------------- softmax and output: a thread owns a row, in the warp that may read its TMEM lane
+        // (32*(warp%4)...). Rows past the tile's last (the tile holds a whole number of tokens) see what the last row
+        // sees; nothing of them is stored.
+        const int quad = warp & 3, row = quad * 32 + lane;
+        const unsigned lane_addr = tmem_base + ((unsigned)(quad * 32) << 16);
+        const unsigned o_addr = lane_addr + C::COL_O;
         const bool live = row < n_tok * n_rep;
         const int ti = min(row / n_rep, n_tok - 1), head = kvh * n_rep + (row % n_rep);
         const int hi = pos0 + ti;
@@ -304,54 +350,52 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         // capped scores are turned into base-2 units where they are read, so the factor on them afterwards is one
         const float scale2 = capped ? 1.0f : scale * LOG2E;
         const float cap_in = capped ? 2.0f * scale / softcap : 0.f, cap_out = softcap * LOG2E;
-        float m_cur = -INFINITY, l_run = 0.f;       // the maximum that the exponents refer to, and this thread's part of the sum
+        float m_cur = -INFINITY, l_run = 0.f;       // the maximum that the exponents refer to, and the row's sum
         bool ok = true;
-        for (int j = 0; j < n_blk && ok; ++j) {
-            const int b = j & 1;
-            ok = !s_failed && mbar_spin(&s_full[b], (j >> 1) & 1);
-            ok = __all_sync(0xffffffffu, ok);
+#pragma unroll 1
+        for (int j = 0; j < n_blk; ++j) {
+            ok = warp_spin(s_full, j & 1);
             if (!ok) break;
             tc_fence_after();
             const int key0 = block_at(j) * KEYS;
             // the same branch for the whole warp: a warp that took both would do the work twice
             const bool all_visible = __all_sync(0xffffffffu, key0 >= lo && key0 + KEYS - 1 <= hi);
-            // this thread's scores of the block: all loads are issued, then waited for once (a load from tensor memory
-            // takes hundreds of cycles). Four maxima side by side, so that no instruction waits for the one before it.
-            const unsigned s_addr = lane_addr + C::COL_S + b * KEYS + half * HK;
-            unsigned raw[HK / 32][32];
+            // the row's scores of the block: all loads are issued, then waited for once (a load from tensor memory
+            // takes hundreds of cycles)
+            unsigned raw[KEYS / 32][32];
 #pragma unroll
-            for (int c = 0; c < HK / 32; ++c) tmem_ld32_async(s_addr + c * 32, raw[c]);
+            for (int c = 0; c < KEYS / 32; ++c) tmem_ld32_async(lane_addr + C::COL_S + c * 32, raw[c]);
             tmem_wait_ld();
+            if (C::P_OWN) {         // the next scores may take their place
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(s_empty);
+            }
             if (capped) {
                 // c tanh(x / c) = c (1 - 2 / (1 + e^(2x/c))), off by a few 1e-7 in absolute terms
 #pragma unroll
-                for (int c = 0; c < HK / 32; ++c)
+                for (int c = 0; c < KEYS / 32; ++c)
 #pragma unroll
                     for (int i = 0; i < 32; ++i)
                         raw[c][i] = __float_as_uint(cap_out * (1.0f - __fdividef(2.0f, 1.0f + __expf(cap_in * __uint_as_float(raw[c][i])))));
             }
-            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+            if (!all_visible) {
 #pragma unroll
-            for (int c = 0; c < HK / 32; ++c) {
-                if (all_visible) {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(raw[c][i]));
-                } else {
+                for (int c = 0; c < KEYS / 32; ++c)
 #pragma unroll
                     for (int i = 0; i < 32; ++i) {
-                        const int key = key0 + half * HK + c * 32 + i;
+                        const int key = key0 + c * 32 + i;
                         if (!((key >= lo || (FLEX && key < keep_first)) && key <= hi)) raw[c][i] = 0xff800000u;      // -inf: its probability will be 0
-                        mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(raw[c][i]));
                     }
-                }
             }
-            // the row's maximum over both halves (the slot of block j is written again at block j + 2, after the barrier
-            // of block j + 1, which the other thread reaches only when it has read this one)
-            float mine = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-            xch[(b * 2 + half) * 128 + row] = mine;
-            ok = pair_sync();
-            if (!ok) break;
-            const float mx = fmaxf(mine, xch[(b * 2 + (half ^ 1)) * 128 + row]) * scale2;      // scale2 > 0
+            // four maxima side by side, so that no instruction waits for the one before it
+            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+            for (int c = 0; c < KEYS / 32; ++c)
+#pragma unroll
+                for (int i = 0; i < 32; i += 2)
+                    mx4[(i >> 1) & 3] = max3(mx4[(i >> 1) & 3], __uint_as_float(raw[c][i]), __uint_as_float(raw[c][i + 1]));
+            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale2;      // scale2 > 0
             float corr = 1.f;
             bool grow = false;
             if (m_cur == -INFINITY) {
@@ -363,92 +407,94 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 grow = true;
             }
             const float m_use = (m_cur == -INFINITY) ? 0.f : m_cur;
-            if (j > 0 && __any_sync(0xffffffffu, grow)) {
-                // rare: the output row is rescaled in tensor memory (each thread its half of the columns), once P.V of
-                // the block before has been added. Both threads of a row decide alike: they see the same maxima.
-                ok = mbar_spin(&o_done[(j - 1) & 1], ((j - 1) >> 1) & 1);
-                ok = __all_sync(0xffffffffu, ok);
+            const bool rescale = j > 0 && __any_sync(0xffffffffu, grow);
+            if (j > 0 && (C::P_OWN || rescale)) {
+                // P.V of the block before has been added: it has read its probabilities, and the output row is at rest
+                ok = warp_spin(o_done, (j - 1) & 1);
                 if (!ok) break;
                 tc_fence_after();
-#pragma unroll
-                for (int c = 0; c < HD / 64; ++c) {
-                    unsigned ov[32];
-                    tmem_ld32_async(o_addr + c * 32, ov);
+            }
+            if (rescale) {      // rare: the output row is rescaled in tensor memory
+#pragma unroll 1
+                for (int c = 0; c < HD; c += 16) {
+                    unsigned ov[16];
+                    tmem_ld16_async(o_addr + c, ov);
                     tmem_wait_ld();
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * corr);
-                    tmem_st32(o_addr + c * 32, ov);
+                    for (int i = 0; i < 16; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * corr);
+                    tmem_st16(o_addr + c, ov);
                 }
+            }
+            // the probabilities into tensor memory (two keys a column), their sum (four partial sums). Of 16 pairs the
+            // exponential unit takes 16 - EMULATED, the multiply-add unit the others (not where scores are masked: 2^-inf).
+            const f32x2 scale_2 = two(scale2, scale2), less_m = two(-m_use, -m_use);
+            f32x2 sum2[2] = {two(0.f, 0.f), two(0.f, 0.f)};
+            auto tell = [&](int half) {
                 tmem_wait_st();
-            }
-            if (j >= 2) {
-                // this buffer of probabilities was read by P.V of block j-2
-                ok = mbar_spin(&o_done[b], ((j - 2) >> 1) & 1);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-            }
-            // the probabilities into shared memory, their sum (four partial sums)
-            unsigned char* p_row = smem + C::OFF_P + b * C::P_BYTES + (row >> 3) * 1024 + (row & 7) * 128;
-            float sum4[4] = {0.f, 0.f, 0.f, 0.f};
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&p_full[half]);
+            };
+            auto probabilities = [&](auto emulated) {
+                constexpr int EMU = decltype(emulated)::value;
 #pragma unroll
-            for (int c = 0; c < HK / 32; ++c) {
-                unsigned pk[16];
+                for (int c = 0; c < KEYS / 32; ++c) {
+                    unsigned pk[16];
 #pragma unroll
-                for (int i = 0; i < 32; i += 2) {
-                    const float p0 = ex2(fmaf(__uint_as_float(raw[c][i]), scale2, -m_use));         // ex2(-inf) = 0
-                    const float p1 = ex2(fmaf(__uint_as_float(raw[c][i + 1]), scale2, -m_use));
-                    sum4[(i >> 1) & 3] += p0 + p1;
-                    pk[i >> 1] = pack2(p0, p1);
+                    for (int i = 0; i < 16; ++i) {
+                        const f32x2 x = fma2(two(__uint_as_float(raw[c][2 * i]), __uint_as_float(raw[c][2 * i + 1])), scale_2, less_m);
+                        float p0, p1;
+                        if ((i * EMU) / 16 != ((i + 1) * EMU) / 16) {
+                            exp2_fma(x, p0, p1);
+                        } else {
+                            split(x, p0, p1);
+                            p0 = ex2(p0);                                   // ex2(-inf) = 0
+                            p1 = ex2(p1);
+                        }
+                        sum2[i & 1] = add2(sum2[i & 1], two(p0, p1));
+                        pk[i] = pack2(p0, p1);
+                    }
+                    // a half of the keys is complete: its P.V may start. The first half is told once the next keys'
+                    // exponentials are under way, so that nothing waits for its stores.
+                    if (c == KEYS / 64) tell(0);
+                    tmem_st16(lane_addr + C::COL_P + c * 16, pk);
+                    if (c == KEYS / 32 - 1) tell(1);
                 }
-                const int cg = half * (HK / 32) + c;                        // the chunk of 32 keys within the block
-                unsigned char* sub = p_row + (cg >> 1) * C::SUBTILE;       // 64 keys per sub-tile
-#pragma unroll
-                for (int q4 = 0; q4 < 4; ++q4) {
-                    const int chunk = ((cg & 1) << 2) + q4;                 // 16-byte chunk within the 128-byte row
-                    *reinterpret_cast<uint4*>(sub + ((chunk ^ (row & 7)) << 4)) =
-                        make_uint4(pk[4 * q4], pk[4 * q4 + 1], pk[4 * q4 + 2], pk[4 * q4 + 3]);
-                }
-            }
-            l_run += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
-            // P is read by the tensor core through the async proxy
-            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-            tc_fence_before();
-            mbar_arrive(&p_full[b]);
+            };
+            if (all_visible)
+                probabilities(std::integral_constant<int, EMULATED<HD>>());
+            else
+                probabilities(std::integral_constant<int, 0>());
+            float s0, s1, s2, s3;
+            split(sum2[0], s0, s1);
+            split(sum2[1], s2, s3);
+            l_run += (s0 + s1) + (s2 + s3);
         }
-        if (ok) {
-            ok = mbar_spin(&o_done[(n_blk - 1) & 1], ((n_blk - 1) >> 1) & 1);
-            ok = __all_sync(0xffffffffu, ok);
-        }
-        if (ok) {
-            // the row's sum: both parts, added in the same order by both threads
-            xch[(4 + half) * 128 + row] = l_run;
-            ok = pair_sync();
-        }
+        if (ok) ok = warp_spin(o_done, (n_blk - 1) & 1);
         if (!ok) {
             if (lane == 0 && !s_failed) { atomicCAS(&g_attn_error, 0, (4 << 16) | (int)(blockIdx.x & 0xffff)); s_failed = 1; }
         } else {
             tc_fence_after();
-            float l_all = xch[4 * 128 + row] + xch[5 * 128 + row];
-            if (FLEX && sinks != nullptr && m_cur != -INFINITY) l_all += ex2(__ldg(sinks + head) * LOG2E - m_cur);   // the sink: no key, no value
-            float inv = l_all > 0.f ? out_scale / l_all : 0.f;
-            if (FLEX && gate != nullptr) inv *= 1.0f / (1.0f + expf(-gate[(size_t)(row_begin + tok0 + ti) * ld_gate + head]));
-            __nv_bfloat16* orow = out + ((size_t)(row_begin + tok0 + ti) * heads + head) * HD + half * (HD / 2);
+            unsigned ov[HD / 32][32];
 #pragma unroll
-            for (int c = 0; c < HD / 64; ++c) {
-                unsigned ov[32];
-                tmem_ld32_async(o_addr + c * 32, ov);
-                tmem_wait_ld();
-                if (live) {
+            for (int c = 0; c < HD / 32; ++c) tmem_ld32_async(o_addr + c * 32, ov[c]);
+            tmem_wait_ld();
+            if (live) {
+                if (FLEX && sinks != nullptr && m_cur != -INFINITY) l_run += ex2(__ldg(sinks + head) * LOG2E - m_cur);   // the sink: no key, no value
+                float inv = l_run > 0.f ? out_scale / l_run : 0.f;
+                if (FLEX && gate != nullptr) inv *= 1.0f / (1.0f + expf(-gate[(size_t)(row_begin + tok0 + ti) * ld_gate + head]));
+                __nv_bfloat16* orow = out + ((size_t)(row_begin + tok0 + ti) * heads + head) * HD;
+#pragma unroll
+                for (int c = 0; c < HD / 32; ++c)
 #pragma unroll
                     for (int d = 0; d < 32; d += 8) {
                         uint4 w;
-                        w.x = pack2(__uint_as_float(ov[d]) * inv, __uint_as_float(ov[d + 1]) * inv);
-                        w.y = pack2(__uint_as_float(ov[d + 2]) * inv, __uint_as_float(ov[d + 3]) * inv);
-                        w.z = pack2(__uint_as_float(ov[d + 4]) * inv, __uint_as_float(ov[d + 5]) * inv);
-                        w.w = pack2(__uint_as_float(ov[d + 6]) * inv, __uint_as_float(ov[d + 7]) * inv);
+                        w.x = pack2(__uint_as_float(ov[c][d]) * inv, __uint_as_float(ov[c][d + 1]) * inv);
+                        w.y = pack2(__uint_as_float(ov[c][d + 2]) * inv, __uint_as_float(ov[c][d + 3]) * inv);
+                        w.z = pack2(__uint_as_float(ov[c][d + 4]) * inv, __uint_as_float(ov[c][d + 5]) * inv);
+                        w.w = pack2(__uint_as_float(ov[c][d + 6]) * inv, __uint_as_float(ov[c][d + 7]) * inv);
                         *reinterpret_cast<uint4*>(orow + c * 32 + d) = w;
                     }
-                }
             }
         }
     }
@@ -489,9 +535,10 @@ int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, 
         configured = true;
     }
     const int tpt = ROWS / (heads / kv_heads);
-    dim3 grid(ceil_div(max_q_len, tpt), n_req, kv_heads);
-    NIB_CUDA(launch_pdl(attention_prefill_tc_kernel<HD, FLEX>, grid, dim3(THREADS), (size_t)Cfg<HD>::SMEM, stream, mq, mk, mv,
-                        (__nv_bfloat16*)out, q_start, ctx_lens, block_table, bt_stride, page_size, num_pages, heads,
+    const long long blocks = (long long)ceil_div(max_q_len, tpt) * n_req * kv_heads;
+    NIB_REQUIRE(blocks <= 0x7fffffffLL, "attention (tcgen05): too many tiles for one launch");
+    NIB_CUDA(launch_pdl(attention_prefill_tc_kernel<HD, FLEX>, dim3((unsigned)blocks), dim3(THREADS), (size_t)Cfg<HD>::SMEM, stream, mq, mk, mv,
+                        (__nv_bfloat16*)out, q_start, ctx_lens, block_table, bt_stride, page_size, num_pages, n_req, heads,
                         kv_heads, scale, window, nib_trace_buffer(), nib_trace_capacity(), softcap, chunk, sinks, out_scale, keep_first, gate, ld_gate));
     return 0;
 }
@@ -503,8 +550,7 @@ int launch(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, 
 NIB_API int nib_attention_prefill_tc_supported(int heads, int kv_heads, int head_dim, int page_size, int q_stride) {
     if (kv_heads <= 0 || heads % kv_heads || heads / kv_heads > ROWS) return 0;
     if (head_dim != 64 && head_dim != 128) return 0;
-    const int keys = head_dim == 64 ? keys_of<64>() : keys_of<128>();
-    if (page_size < 8 || page_size > keys || keys % page_size) return 0;
+    if (page_size < 8 || page_size > KEYS || KEYS % page_size) return 0;
     if (q_stride % 8) return 0;
     return nib_tensor_map_encoder() != nullptr;
 }
@@ -531,7 +577,6 @@ NIB_API int nib_attention_prefill_tc(const void* qkv, int q_stride, void* out, c
     NIB_REQUIRE(n_req >= 0 && max_q_len > 0 && num_pages > 0 && window >= 0 && m_tokens > 0 && chunk >= 0 && softcap >= 0.f && scale > 0.f && keep_first >= 0,
                 "attention (tcgen05): bad sizes");
     NIB_REQUIRE((((uintptr_t)qkv | (uintptr_t)k_pages | (uintptr_t)v_pages | (uintptr_t)out) & 15) == 0, "attention (tcgen05): bases must be 16-byte aligned");
-    NIB_REQUIRE(n_req <= 65535 && kv_heads <= 65535, "attention (tcgen05): too many requests or kv heads for one launch");
     if (n_req == 0) return 0;
     const int n_rep = heads / kv_heads, tpt = ROWS / n_rep;
     CUtensorMap mq, mk, mv;

@@ -846,6 +846,44 @@ def test_general_attention_segments(K, dtype, heads, kv_heads, hd, page, window)
         assert torch.equal(one[0], out[i])
 
 
+@pytest.mark.parametrize("window", [0, 200])
+@pytest.mark.parametrize("heads,kv_heads,hd,page", [(14, 2, 64, 16), (12, 2, 128, 16), (2, 2, 64, 128), (2, 1, 128, 128), (28, 4, 128, 8), (128, 1, 64, 32)])
+def test_prefill_tile_and_block_edges(K, heads, kv_heads, hd, page, window):
+    """The tcgen05 prefill kernel where its tiles (128 rows: 128 // group tokens) and key blocks (128) end: portions one token
+    short of a tile, a whole one, one more; contexts one key short of a block, a whole one, one more; pages as long as a block;
+    many requests of unlike lengths in one launch."""
+    tokens = 128 // (heads // kv_heads)
+    q_lens = [2, max(2, tokens - 1), max(2, tokens), tokens + 1, 127, 128, 129, 2, 40]
+    before = [125, 0, 256 - tokens, 1, 1, 0, 255, 900, 1013]
+    ctx, bt = make_paged_batch(q_lens, before, page, sum(-(-(a + b) // page) for a, b in zip(q_lens, before)) + 3, "cuda", seed=6)
+    kp, vp = _fill_cache(ctx, bt, page, int(bt.max()) + 1, kv_heads, hd, torch.bfloat16, 90)
+    m = sum(q_lens)
+    qkv = rnd((m, (heads + 2 * kv_heads) * hd), torch.bfloat16, 92)
+    out, ref = (torch.empty(m, heads * hd, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    scale = 1.0 / math.sqrt(hd)
+    K.attention(qkv, out, heads, kv_heads, hd, scale, window, ctx, bt, page, kp, vp)
+    REF.attention(qkv, ref, heads, kv_heads, hd, scale, window, ctx, bt, page, kp, vp)
+    assert_close(out, ref, torch.bfloat16, "prefill")
+    assert K.attention_tc_error() == 0
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+def test_prefill_scores_that_grow_from_block_to_block(K, hd):
+    """Every block of keys holds larger scores than the one before, by more than what the running maximum lets pass (2^8), so
+    the output row is rescaled at every block, in some rows and not in others; the first blocks' shares vanish."""
+    heads, kv_heads, page, n = 4, 2, 16, 700
+    ctx, bt = make_paged_batch([n], [0], page, 60, "cuda", seed=7)
+    kp, vp = _fill_cache(ctx, bt, page, 60, kv_heads, hd, torch.bfloat16, 93)
+    qkv = rnd((n, (heads + 2 * kv_heads) * hd), torch.bfloat16, 94)
+    for p in range(-(-n // page)):
+        kp[bt[0, p].item()] *= 0.02 * (1 + 3 * (p * page // 128))
+    qkv[::3, :heads * hd] *= 12.0       # some rows' scores are large, others' are not
+    out, ref = (torch.empty(n, heads * hd, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    K.attention(qkv, out, heads, kv_heads, hd, 1.0, 0, ctx, bt, page, kp, vp)
+    REF.attention(qkv, ref, heads, kv_heads, hd, 1.0, 0, ctx, bt, page, kp, vp)
+    assert_close(out, ref, torch.bfloat16, "prefill")
+
+
 @pytest.mark.parametrize("vocab", [3, 2048, 2049, 32000, 151936, 151937, 389120, 389121, 700000])
 def test_sampling_slices(K, vocab):
     """Slices of a row that are kept in shared memory and those that do not fit (more than 389,120 logits), rows that do not start
