@@ -2,7 +2,7 @@
 // K, no reduced-precision matrix mode.
 //
 // ONE ORDER OF SUMMATION for every M, so that a row's result does not depend on how many rows the call has (the reference
-// guarantees the same: cpp/src/cuda/cuda_gemm.cu:37-45): k is cut into chunks of 128 at absolute multiples of 128; a chunk
+// guarantees the same: cpp/src/cuda/cuda_gemm.cu:37-45): k is cut into chunks of 256 at absolute multiples of 256; a chunk
 // is one chain of fused multiply-adds in ascending k that starts at 0; the chunks' sums are added up in ascending order.
 // Against one chain over all of K that is also the smaller error, and it is what lets threads, warps and CTAs share K. Two
 // kernels give these same sums bit for bit:
@@ -15,7 +15,10 @@
 // * gemm_f32_tile_kernel, more tokens: bound by the multiply-adds. Tiles of 64 x 64, 4 x 4 outputs a thread, the next 16 k
 //   fetched into registers under this block's arithmetic. Few tiles: the chunks are shared by the CTAs of a cluster.
 //
-// Measured on B200 at the 0.5B widths, a step of one token / a prompt of 128: see the figures beside the launch rules below.
+// Measured on B200 at the 0.5B widths (us; before: a thread per output and one chain over all of K): one token, gate/up 189 -> 10.0
+// (35 MB: 5.2 at the copy bandwidth), down 445 -> 4.4 (with the output projection), the head's 545 MB 111 (82); 128 tokens,
+// gate/up 91, the sums into the residual stream 42. With chunks of 128 the one-token kernels are faster (8.2 and 92: half the chain
+// a thread walks), but a product of K <= 256 keeps the bits of one ascending chain with 256.
 //
 // Epilogues: STORE and F32 (out = sum + bias), ADD (out += sum + bias: the residual sum), and the gated ones on W rows n and
 // n + N: SWIGLU silu(gate) * up with silu(g) = g / (1 + exp(-g)) (cpp/src/ops.cpp:86-93), GLU (with limits and constants),
@@ -26,7 +29,7 @@ using namespace nibp;
 
 namespace {
 
-constexpr int CHUNK = 128;
+constexpr int CHUNK = 256;
 
 __device__ __forceinline__ void copy16(unsigned dst, const float* src, int bytes) {      // bytes < 16: the rest is zeros
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
@@ -349,7 +352,7 @@ int launch_cluster(Kernel kernel, dim3 grid, int threads, size_t smem, int ranks
 }
 
 constexpr int ROWS_MAX_TOKENS = 16;
-constexpr int ROWS_CHUNKS = 10;           // of a CTA while that needs no more than eight CTAs for K
+constexpr int ROWS_CHUNKS = 5;            // of a CTA while that needs no more than eight CTAs for K
 constexpr size_t ROWS_SMEM = 200 * 1024, TILE_SMEM = 160 * 1024;
 
 template <int EPI, int RB>
@@ -382,7 +385,7 @@ int launch_f32(const Args& a) {
     }
     const int tiles = ceil_div(a.N, BN) * ceil_div(a.M, BM);
     // CTAs that share the chunks of a tile: as many as keep all CTAs on the GPU at once, two an SM; with more tiles than SMs none,
-    // unless their last turn would leave most SMs idle (152 tiles of 7 chunks on 148 SMs: 105 us with a CTA a tile, 94 with seven)
+    // unless their last turn would leave most SMs idle (152 tiles on 148 SMs, K = 896: 105 us with a CTA a tile, 91 with a CTA a chunk)
     int ranks = 2 * 148 / tiles;
     if (tiles > 148 && ceil_div(tiles, 148) * 148 > tiles + tiles / 2) ranks = 8;
     ranks = max(1, min(min(8, chunks), ranks));
