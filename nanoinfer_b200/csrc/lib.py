@@ -1371,12 +1371,15 @@ class Kernels:
             longest, splits, part_o, part_ml = max(ctx.host.q_lens), 1, None, None
             if longest * (heads // kv_heads) <= 64:
                 # a step of few tokens per request (decoding): a CTA that walks a long context alone waits for memory
-                # tile after tile; two tiles per CTA are both in flight at once
+                # tile after tile; two tiles per CTA are both in flight at once, and one is the shorter way while that
+                # gives no SM a second CTA
                 keys = max(ctx.host.ctx_lens)
                 for bound in (window, chunk):
                     keys = min(keys, bound + keep_first) if bound > 0 else keys
                 most = max(1, (4 * max(1, self.sm_count)) // max(1, ctx.host.num_requests * kv_heads))
-                splits = self.options.fixed_decode_splits or max(1, min(-(-(keys // 64 + 1) // 2), most, 32))
+                tiles, units = keys // 64 + 1, max(1, ctx.host.num_requests * kv_heads)
+                per_cta = 1 if units * min(tiles, 32) <= self.sm_count else 2
+                splits = self.options.fixed_decode_splits or max(1, min(-(-tiles // per_cta), most, 32))
                 if splits > 1:
                     part_o = torch.empty(m * heads * splits * vdim, dtype=torch.float32, device=q.device)
                     part_ml = torch.empty(m * heads * splits * 2, dtype=torch.float32, device=q.device)
