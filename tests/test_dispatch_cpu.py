@@ -86,3 +86,15 @@ def test_decode_attention_splits(rules):
     assert rules.decode_splits(8, 2, 4096, 0, False, 64) == 5
     rules.options = dataclasses.replace(rules.options, fixed_decode_splits=21)
     assert rules.decode_splits(8, 2, 4096, 0, True, 64) == 16
+
+
+def test_decode_attention_splits_while_sms_are_idle(rules):
+    # up to a cluster of eight CTAs for a context of a few tiles, as long as every CTA has an SM
+    assert rules.decode_splits(1, 2, 777, 0, True, 64) == 8
+    assert rules.decode_splits(1, 2, 200, 0, True, 64) == 2              # two tiles of 128 keys
+    assert rules.decode_splits(24, 2, 1500, 0, True, 64) == 2
+    assert rules.decode_splits(74, 2, 777, 0, True, 64) == 1             # 148 CTAs as it is
+    assert rules.decode_splits(1, 2, 777, 512, True, 64) == 1            # a window: few tiles at any context
+    # more than one cluster a token and kv head only where eight CTAs leave SMs idle
+    assert rules.decode_splits(8, 2, 4096, 0, True, 128) == 8
+    assert rules.decode_splits(1, 2, 4096, 0, True, 128) == 16

@@ -759,3 +759,20 @@ def test_command_line_tools_generate_and_serve(folders):
         argv += ["--prompt", " ".join(map(str, p))]
     got = tool("serve", argv)
     assert got == [greedy(p, 6) for p in prompts]
+
+
+@pytest.mark.parametrize("heads,kv,dim,vdim", [(4, 2, 64, 40), (16, 1, 128, 128)])
+@pytest.mark.parametrize("splits", [1, 2, 8, 9, 31, 32, 33, 70])
+def test_decoded_tokens_over_shares_of_the_keys(ops, heads, kv, dim, vdim, splits):
+    """The merge around its eight outputs at a time and its 32 shares a warp, shares that saw no key among them (contexts of one key
+    and of fewer tiles than shares), pages looked up a tile ahead, against the plain statement."""
+    ctx, bt, num_pages = batch([1, 1, 1, 1], [0, 63, 600, 1299], page_size=16)
+    kp, vp = filled_pages(torch.bfloat16, ctx.host.ctx_lens, bt.cpu(), num_pages, kv, dim, vdim, 16, 6)
+    q = rnd(4, heads * dim, seed=7).to(torch.bfloat16)
+    sinks, gate = rnd(heads, seed=8), rnd(4, heads, seed=9)
+    out, ref = torch.empty(4, heads * vdim, dtype=torch.float32, device=DEV), torch.empty(4, heads * vdim, dtype=torch.float64)
+    ops.with_options(fixed_decode_splits=splits).attention_flex(q, out, heads, kv, dim, vdim, dim ** -0.5, 0.0, None, 0, 0, 1.0, ctx, bt, 16,
+                                                                kp, vp, sinks32=sinks, gate32=gate)
+    TorchOps().attention_flex(q.cpu(), ref, heads, kv, dim, vdim, dim ** -0.5, 0.0, None, 0, 0, 1.0, to_cpu(ctx), bt.cpu(), 16,
+                              kp.cpu(), vp.cpu(), sinks32=sinks.cpu(), gate32=gate.cpu())
+    assert_close(out, ref, torch.bfloat16, "attention over shares")
