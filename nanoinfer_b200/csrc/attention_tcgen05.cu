@@ -94,13 +94,16 @@ __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
-// 2^x of two numbers in the multiply-add unit, for -126 <= x < 127: x = n + f with n the nearest whole number (the low bits of
+// 2^x of two numbers in the multiply-add unit, for x < 127: x = n + f with n the nearest whole number (the low bits of
 // x + 1.5 * 2^23), 2^f on [-1/2, 1/2] by a polynomial of degree 5 (Remez exchange for the relative error: 7.5e-8, 2.1e-7 as
-// evaluated here; ex2.approx allows itself 2.4e-7), n added to the exponent.
+// evaluated here; ex2.approx allows itself 2.4e-7), n added to the exponent. What the polynomial does not cover is what
+// ex2.approx.ftz gives: 0 below -126 (-inf, too) and NaN for NaN (a score that overflowed has to show in its row).
+__device__ __forceinline__ float or_limit(float x, float p) {
+    float limit;
+    asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(limit) : "f"(x));
+    return x >= -126.f ? p : limit;
+}
 __device__ __forceinline__ void exp2_fma(f32x2 x, float& p0, float& p1) {
-    float x0, x1;
-    split(x, x0, x1);
-    x = two(fmaxf(x0, -126.f), fmaxf(x1, -126.f));
     const f32x2 magic = two(12582912.f, 12582912.f);
     const f32x2 n = add2(x, magic);
     const f32x2 f = fma2(add2(n, two(-12582912.f, -12582912.f)), two(-1.f, -1.f), x);
@@ -109,11 +112,12 @@ __device__ __forceinline__ void exp2_fma(f32x2 x, float& p0, float& p1) {
     p = fma2(p, f, two(0.24022120237350464f, 0.24022120237350464f));
     p = fma2(p, f, two(0.6931469440460205f, 0.6931469440460205f));
     p = fma2(p, f, two(1.0000001192092896f, 1.0000001192092896f));
-    float n0, n1;
+    float x0, x1, n0, n1;
+    split(x, x0, x1);
     split(n, n0, n1);
     split(p, p0, p1);
-    p0 = __int_as_float(__float_as_int(p0) + (__float_as_int(n0) << 23));
-    p1 = __int_as_float(__float_as_int(p1) + (__float_as_int(n1) << 23));
+    p0 = or_limit(x0, __int_as_float(__float_as_int(p0) + (__float_as_int(n0) << 23)));
+    p1 = or_limit(x1, __int_as_float(__float_as_int(p1) + (__float_as_int(n1) << 23)));
 }
 template <int HD> struct Cfg {
     static constexpr int SUB = HD / 64;                       // sub-tiles of 64 elements (128 bytes) along the head dim

@@ -884,6 +884,42 @@ def test_prefill_scores_that_grow_from_block_to_block(K, hd):
     assert_close(out, ref, torch.bfloat16, "prefill")
 
 
+@pytest.mark.parametrize("hd", [64, 128])
+def test_prefill_scores_that_are_no_numbers(K, hd):
+    """A key whose scores are +inf, -inf or NaN (by the sign of the query's first element), at every place of a block's 32 and in
+    every block: rows that see an infinite or undefined score come out NaN, as the 32-bit statement has them, a score of -inf is a
+    weight of zero, and a row that sees nothing else is zero."""
+    heads, kv_heads, page, n, before = 4, 2, 16, 40, 260
+    ctx, bt = make_paged_batch([n], [before], page, 24, "cuda", seed=8)
+    clean, vp = _fill_cache(ctx, bt, page, 24, kv_heads, hd, torch.bfloat16, 97)
+    qkv = rnd((n, (heads + 2 * kv_heads) * hd), torch.bfloat16, 98)
+    sign = torch.tensor([-1.0, 1.0, -1.0, 0.0], device="cuda")[torch.arange(n, device="cuda") % 4]
+    qkv.view(n, -1, hd)[:, :heads, 0] = sign[:, None].to(torch.bfloat16)
+    out, ref = (torch.empty(n, heads * hd, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+
+    def place(kp, j):
+        kp[bt[0, j // page].item(), :, j % page, 0] = math.inf
+
+    def run(kp):
+        out.fill_(7.0)
+        K.attention(qkv, out, heads, kv_heads, hd, 1.0 / math.sqrt(hd), 0, ctx, bt, page, kp, vp)
+
+    for j in list(range(32)) + [69, 127, 133, 138, 143, 255, 256, 261, 270, 299]:
+        kp = clean.clone()
+        place(kp, j)
+        run(kp)
+        REF.attention(qkv, ref, heads, kv_heads, hd, 1.0 / math.sqrt(hd), 0, ctx, bt, page, kp, vp)
+        bad = (ctx.positions >= j) & (sign >= 0)
+        assert ref[bad].isnan().all() and not ref[~bad].isnan().any()
+        assert out[bad].isnan().all(), j
+        assert_close(out[~bad], ref[~bad], torch.bfloat16, f"key {j}")
+    kp = clean.clone()
+    for j in range(before + n):
+        place(kp, j)
+    run(kp)
+    assert (out[sign < 0] == 0).all() and out[sign >= 0].isnan().all()
+
+
 @pytest.mark.parametrize("vocab", [3, 2048, 2049, 32000, 151936, 151937, 389120, 389121, 700000])
 def test_sampling_slices(K, vocab):
     """Slices of a row that are kept in shared memory and those that do not fit (more than 389,120 logits), rows that do not start
