@@ -186,7 +186,7 @@ attention_generic_kernel(const T* __restrict__ qkv, int q_stride, T* __restrict_
                 const float* other = base + (size_t)w * gen_warp_floats(R, head_dim);
                 const float* other_ml = other + 2 * GEN_BLOCK * pitch + GEN_BLOCK * R;
                 const float mw = other_ml[2 * r], lw = other_ml[2 * r + 1];
-                if (mw == -INFINITY) continue;          // no key of the block is seen
+                if (mw == -INFINITY && lw == 0.f) continue;          // no key of the block is seen (or only scores of -inf); a sum of NaN goes on
                 const float m_new = fmaxf(m, mw);
                 const float a = m == -INFINITY ? 0.f : expf(m - m_new), b = expf(mw - m_new);
                 o = o * a + other[e] * b;
@@ -205,7 +205,7 @@ attention_generic_kernel(const T* __restrict__ qkv, int q_stride, T* __restrict_
     for (int e = threadIdx.x; e < n_heads * head_dim; e += blockDim.x) {
         const int r = e / head_dim, d = e % head_dim;
         const float l = ml[(round & 1) * 2 * R + 2 * r + 1];
-        Elem<T>::store(o + e, l > 0.f ? tot[r * pitch + d] * (1.0f / l) : 0.f);
+        Elem<T>::store(o + e, tot[r * pitch + d] * (l > 0.f ? 1.0f / l : 0.f));       // a row with an undefined score stays NaN
     }
 }
 

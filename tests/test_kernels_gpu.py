@@ -920,6 +920,46 @@ def test_prefill_scores_that_are_no_numbers(K, hd):
     assert (out[sign < 0] == 0).all() and out[sign >= 0].isnan().all()
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("hd", [5, 40, 64])
+def test_general_attention_scores_that_are_no_numbers(K, dtype, hd):
+    """The general kernel: a row that sees an infinite or undefined score is NaN, whichever block it lies in and whatever that block's
+    maximum is; a score of -inf weighs nothing, and a row that sees nothing else is zero."""
+    K = K.with_options(force_general_attention=True)
+    heads, kv_heads, page, n, before = 4, 2, 8, 10, 75
+    ctx, bt = make_paged_batch([n, 3], [before, 0], page, 24, "cuda", seed=9)
+    clean, vp = _fill_cache(ctx, bt, page, 24, kv_heads, hd, dtype, 99)
+    qkv = rnd((n + 3, (heads + 2 * kv_heads) * hd), dtype, 100)
+    sign = torch.tensor([-1.0, 1.0, -1.0, 0.0], device="cuda")[torch.arange(n + 3, device="cuda") % 4]
+    qkv.view(n + 3, -1, hd)[:, :heads, 0] = sign[:, None].to(dtype)
+    qkv[n + 1] = math.nan               # a request's second token: every score of its only block is undefined
+    first = ctx.req_index == 0
+    out, ref = (torch.empty(n + 3, heads * hd, dtype=dtype, device="cuda") for _ in range(2))
+
+    def place(kp, j):
+        kp[bt[0, j // page].item(), :, j % page, 0] = math.inf
+
+    def run(kp):
+        out.fill_(7.0)
+        K.attention(qkv, out, heads, kv_heads, hd, 1.0 / math.sqrt(hd), 0, ctx, bt, page, kp, vp)
+
+    for j in (0, 31, 32, 40, 64, 76, 84):
+        kp = clean.clone()
+        place(kp, j)
+        run(kp)
+        REF.attention(qkv, ref, heads, kv_heads, hd, 1.0 / math.sqrt(hd), 0, ctx, bt, page, kp, vp)
+        bad = first & (ctx.positions >= j) & (sign >= 0)
+        bad[n + 1] = True
+        assert ref[bad].isnan().all() and not ref[~bad].isnan().any()
+        assert out[bad].isnan().all(), j
+        assert_close(out[~bad], ref[~bad], dtype, f"key {j}")
+    kp = clean.clone()
+    for j in range(before + n):
+        place(kp, j)
+    run(kp)
+    assert (out[first & (sign < 0)] == 0).all() and out[first & (sign >= 0)].isnan().all()
+
+
 @pytest.mark.parametrize("vocab", [3, 2048, 2049, 32000, 151936, 151937, 389120, 389121, 700000])
 def test_sampling_slices(K, vocab):
     """Slices of a row that are kept in shared memory and those that do not fit (more than 389,120 logits), rows that do not start
