@@ -51,21 +51,21 @@ __device__ __forceinline__ void gen_load(float (&v)[R], const float* p) {
 // (below 0: zeros). 32-bit rows that start on 16 bytes go as asynchronous copies, as many rows at a time as the warp's lanes
 // cover: nothing waits for them here. (What lies behind a row is read, but what comes of it is not.)
 template <typename T>
-__device__ __forceinline__ void gen_send_rows(float* dst, const T* pages, int row, int d, int pitch, bool wide, int lane) {
+__device__ __forceinline__ void gen_send_rows(float* dst, const T* pages, long long row, int d, int pitch, bool wide, int lane) {
     if (sizeof(T) == 4 && wide) {
         const int units = d >> 2, per_row = units <= 8 ? 8 : units <= 16 ? 16 : 32, u0 = lane & (per_row - 1);
 #pragma unroll 4
         for (int r = lane / per_row; r < GEN_BLOCK; r += 32 / per_row) {
-            const int rj = __shfl_sync(0xffffffffu, row, r);
-            const T* src = pages + (long long)max(rj, 0) * d;
+            const long long rj = __shfl_sync(0xffffffffu, row, r);
+            const T* src = pages + max(rj, 0ll) * d;
             const unsigned to = (unsigned)__cvta_generic_to_shared(dst + r * pitch);
             for (int u = u0; u < units; u += per_row)
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(to + 16 * u), "l"(src + 4 * u), "r"(rj >= 0 ? 16 : 0) : "memory");
         }
     } else {
         for (int r = 0; r < GEN_BLOCK; ++r) {
-            const int rj = __shfl_sync(0xffffffffu, row, r);
-            const T* src = pages + (long long)max(rj, 0) * d;
+            const long long rj = __shfl_sync(0xffffffffu, row, r);
+            const T* src = pages + max(rj, 0ll) * d;
             for (int i = lane; i < pitch; i += 32) dst[r * pitch + i] = rj >= 0 && i < d ? Elem<T>::load(src + i) : 0.f;
         }
     }
@@ -115,10 +115,10 @@ attention_generic_kernel(const T* __restrict__ qkv, int q_stride, T* __restrict_
     for (int b0 = lo / GEN_BLOCK; b0 <= b_last; b0 += warps, ++round) {
         if (b0 + warp <= b_last) {
             const int j = (b0 + warp) * GEN_BLOCK + lane;
-            int row = -1;       // this lane's key: its row in the pages
+            long long row = -1;       // this lane's key: its row in the pages
             if (j >= lo && j <= pos) {
                 const int page = bt[j / page_size];
-                if (page >= 0 && page < num_pages) row = (page * kv_heads + kvh) * page_size + j % page_size;
+                if (page >= 0 && page < num_pages) row = ((long long)page * kv_heads + kvh) * page_size + j % page_size;
             }
             gen_send_rows(k_s, k_pages, row, head_dim, pitch, wide, lane);
             asm volatile("cp.async.commit_group;\n" ::: "memory");
@@ -249,7 +249,6 @@ NIB_API int nib_attention_generic(const void* qkv, int q_stride, void* out, cons
     NIB_REQUIRE(m_tokens >= 0 && heads > 0 && kv_heads > 0 && heads % kv_heads == 0, "attention: bad head counts %d / %d", heads, kv_heads);
     NIB_REQUIRE(head_dim > 0 && head_dim <= GEN_MAX_D, "attention: head_dim %d is outside 1..%d", head_dim, GEN_MAX_D);
     NIB_REQUIRE(page_size > 0 && num_pages > 0 && window >= 0, "attention: bad page_size/num_pages/window");
-    NIB_REQUIRE((long long)num_pages * kv_heads * page_size <= 0x7fffffffLL, "attention: more rows of keys than a 32-bit index counts");
     NIB_REQUIRE(dtype == NIB_F32 || dtype == NIB_BF16, "attention: unknown dtype %d", dtype);
     if (m_tokens == 0) return 0;
     // As many heads a CTA as still leaves a CTA for every SM: few tokens take fewer (a warp's arithmetic on a block of keys is

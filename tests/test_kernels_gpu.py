@@ -960,6 +960,22 @@ def test_general_attention_scores_that_are_no_numbers(K, dtype, hd):
     assert (out[first & (sign < 0)] == 0).all() and out[first & (sign >= 0)].isnan().all()
 
 
+def test_general_attention_over_more_rows_than_32_bits_count(K):
+    """A pool of narrow heads with more than 2^31 rows (4.3 GB), the request's pages at its two ends."""
+    page, hd = 1024, 1
+    pages = (1 << 21) + 5
+    pool = torch.empty(pages, 1, page, hd, dtype=torch.bfloat16, device="cuda")
+    ctx, _ = make_paged_batch([2], [1500], page, 4, "cuda")
+    bt = torch.tensor([[pages - 1, 3]], dtype=torch.int32, device="cuda")
+    for p in bt[0].tolist():
+        pool[p] = rnd((1, page, hd), torch.bfloat16, 101)
+    qkv = rnd((2, 3 * hd), torch.bfloat16, 102)
+    out, ref = (torch.empty(2, hd, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    K.with_options(force_general_attention=True).attention(qkv, out, 1, 1, hd, 3.0, 0, ctx, bt, page, pool, pool)
+    REF.attention(qkv, ref, 1, 1, hd, 3.0, 0, ctx, bt, page, pool, pool)
+    assert_close(out, ref, torch.bfloat16, "far rows")
+
+
 @pytest.mark.parametrize("vocab", [3, 2048, 2049, 32000, 151936, 151937, 389120, 389121, 700000])
 def test_sampling_slices(K, vocab):
     """Slices of a row that are kept in shared memory and those that do not fit (more than 389,120 logits), rows that do not start
