@@ -224,7 +224,8 @@ static int launch_generic(const void* qkv, int q_stride, void* out, const int* p
     while (warps > 1 && cta + warps * per_warp > GEN_SMEM) --warps;
     const size_t smem = cta + warps * per_warp;
     const int wide = head_dim % 4 == 0 && ((uintptr_t)k_pages | (uintptr_t)v_pages) % 16 == 0;
-    if (smem > 48 * 1024) NIB_CUDA(cudaFuncSetAttribute(attention_generic_kernel<T, R, DI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // the most that any call takes: the attribute is the kernel's, and a call's own size would lower it under another thread's launch
+    if (smem > 48 * 1024) NIB_CUDA(cudaFuncSetAttribute(attention_generic_kernel<T, R, DI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEN_SMEM));
     NIB_CUDA(launch_pdl(attention_generic_kernel<T, R, DI>, dim3((unsigned)blocks), dim3(32 * warps), smem, stream, (const T*)qkv, q_stride,
                         (T*)out, positions, req_index, block_table, bt_stride, page_size, (const T*)k_pages, (const T*)v_pages, num_pages,
                         heads, kv_heads, head_dim, scale, window, wide));

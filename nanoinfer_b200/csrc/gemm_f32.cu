@@ -330,9 +330,11 @@ struct Args {
     cudaStream_t stream;
 };
 
+// `most`: what the kernel's largest launch takes. The attribute belongs to the kernel, not to a launch: set to a call's own size it
+// would be lowered under a larger launch that another thread has just allowed.
 template <typename Kernel>
-int launch_cluster(Kernel kernel, dim3 grid, int threads, size_t smem, int ranks, const Args& a, int chunks_per_cta) {
-    if (smem > 16 * 1024) NIB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));   // (beside up to 26 KB of static)
+int launch_cluster(Kernel kernel, dim3 grid, int threads, size_t smem, size_t most, int ranks, const Args& a, int chunks_per_cta) {
+    if (smem > 16 * 1024) NIB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));   // (beside up to 26 KB of static)
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
@@ -362,10 +364,10 @@ template <int EPI, int RB>
 int launch_rows(const Args& a, int cpc, int ranks) {
     constexpr int FEATURES = epi_dual(EPI) ? 8 : 8 * RB;
     const dim3 grid(ceil_div(a.N, FEATURES) * ranks);
-    if (a.M == 1) return launch_cluster(gemm_f32_rows_kernel<EPI, RB, 1>, grid, ROWS_THREADS, rows_smem<EPI, RB>(1, cpc), ranks, a, cpc);
-    if (a.M == 2) return launch_cluster(gemm_f32_rows_kernel<EPI, RB, 2>, grid, ROWS_THREADS, rows_smem<EPI, RB>(2, cpc), ranks, a, cpc);
-    if (a.M <= 4) return launch_cluster(gemm_f32_rows_kernel<EPI, RB, 4>, grid, ROWS_THREADS, rows_smem<EPI, RB>(4, cpc), ranks, a, cpc);
-    return launch_cluster(gemm_f32_rows_kernel<EPI, RB, 8>, grid, ROWS_THREADS, rows_smem<EPI, RB>(8, cpc), ranks, a, cpc);
+    if (a.M == 1) return launch_cluster(gemm_f32_rows_kernel<EPI, RB, 1>, grid, ROWS_THREADS, rows_smem<EPI, RB>(1, cpc), ROWS_SMEM, ranks, a, cpc);
+    if (a.M == 2) return launch_cluster(gemm_f32_rows_kernel<EPI, RB, 2>, grid, ROWS_THREADS, rows_smem<EPI, RB>(2, cpc), ROWS_SMEM, ranks, a, cpc);
+    if (a.M <= 4) return launch_cluster(gemm_f32_rows_kernel<EPI, RB, 4>, grid, ROWS_THREADS, rows_smem<EPI, RB>(4, cpc), ROWS_SMEM, ranks, a, cpc);
+    return launch_cluster(gemm_f32_rows_kernel<EPI, RB, 8>, grid, ROWS_THREADS, rows_smem<EPI, RB>(8, cpc), ROWS_SMEM, ranks, a, cpc);
 }
 
 template <int EPI>
@@ -393,8 +395,8 @@ int launch_f32(const Args& a) {
     ranks = ceil_div(chunks, cpc);
     const size_t smem = sizeof(float) * (size_t)cpc * (DUAL ? 2 : 1) * BM * BN;
     const dim3 grid(ceil_div(a.N, BN) * (smem <= TILE_SMEM ? ranks : 1), ceil_div(a.M, BM));
-    if (ranks > 1 && smem <= TILE_SMEM) return launch_cluster(gemm_f32_tile_kernel<EPI, true>, grid, TILE_THREADS, smem, ranks, a, cpc);
-    return launch_cluster(gemm_f32_tile_kernel<EPI, false>, grid, TILE_THREADS, (size_t)0, 1, a, chunks);
+    if (ranks > 1 && smem <= TILE_SMEM) return launch_cluster(gemm_f32_tile_kernel<EPI, true>, grid, TILE_THREADS, smem, TILE_SMEM, ranks, a, cpc);
+    return launch_cluster(gemm_f32_tile_kernel<EPI, false>, grid, TILE_THREADS, (size_t)0, (size_t)0, 1, a, chunks);
 }
 
 }  // namespace

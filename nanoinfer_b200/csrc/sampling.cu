@@ -192,6 +192,7 @@ __device__ __forceinline__ void mass_add(unsigned (*m)[COPIES * BINS], unsigned 
 constexpr int ST = 256;      // chunks of a CTA's slice: what is summed in order is summed by so many threads
 constexpr int NT = 512;      // threads of a CTA
 constexpr int CS = 8;        // CTAs of the cluster that shares a row
+constexpr size_t SAMPLE_SMEM = 200 * 1024;      // dynamic shared memory of a CTA at most
 
 __device__ __forceinline__ unsigned ld_peer_u32(unsigned addr) {
     unsigned v;
@@ -663,9 +664,10 @@ NIB_API int nib_sample(const float* logits, int rows, int vocab, const float* te
     NIB_REQUIRE((long long)vocab <= (1LL << 17) * 8, "sample: a row of %d logits is more than the fixed-point histograms hold", vocab);
     const int per = (ceil_div(vocab, CS * ST) + 3) & ~3;
     const size_t hist = sizeof(unsigned) * 4 * COPIES * BINS, slice = sizeof(float) * (size_t)ST * per;
-    const bool kept = hist + slice <= 200 * 1024;
+    const bool kept = hist + slice <= SAMPLE_SMEM;
     const size_t smem = hist + (kept ? slice : 0);
-    if (kept) NIB_CUDA(cudaFuncSetAttribute(sample_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // the most that any call takes: the attribute is the kernel's, and a call's own size would lower it under another thread's launch
+    if (kept) NIB_CUDA(cudaFuncSetAttribute(sample_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SAMPLE_SMEM));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(rows * CS);
     cfg.blockDim = dim3(NT);

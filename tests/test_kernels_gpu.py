@@ -976,6 +976,54 @@ def test_general_attention_over_more_rows_than_32_bits_count(K):
     assert_close(out, ref, torch.bfloat16, "far rows")
 
 
+@pytest.mark.parametrize("which", ["product of few tokens", "product of many tokens", "attention", "sampling"])
+def test_launches_of_unlike_sizes_from_several_threads(K, which):
+    """Kernels whose shared memory depends on the call, launched by four threads at once, one with large calls and three with small
+    ones: none takes the other's room away."""
+    def jobs(large):
+        if which == "attention":
+            ctx, bt = make_paged_batch([1], [1500 if large else 70], 16, 120, "cuda", seed=3)
+            kp, vp = _fill_cache(ctx, bt, 16, 120, 2, 64, torch.float32, 103)
+            qkv, out = rnd((1, 18 * 64), torch.float32, 104), torch.empty(1, 14 * 64, device="cuda")
+            return out, lambda k: k.attention(qkv, out, 14, 2, 64, 0.125, 0, ctx, bt, 16, kp, vp)
+        if which == "sampling":
+            one = lambda v, dtype=torch.float32: torch.tensor([v], dtype=dtype, device="cuda")
+            logits, out = rnd((1, 151936 if large else 20000), torch.float32, 105), torch.empty(1, dtype=torch.int32, device="cuda")
+            args = (one(0.7), one(0, torch.int32), one(0.9), one(0.4))
+            return out, lambda k: k.sample(logits, *args, out)
+        m, n, k_ = (3, 40, 4864 if large else 1024) if which == "product of few tokens" else (64, 64, 2048 if large else 512)
+        a, w, out = rnd((m, k_), torch.float32, 106), rnd((n, k_), torch.float32, 107), torch.empty(m, n, device="cuda")
+        return out, lambda k: k.linear(a, w, None, out, "f32")
+
+    import threading
+    failed, start = [], threading.Barrier(4)
+
+    def work(out, call):
+        k = K.with_options()
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                start.wait(60)
+                call(k)
+                torch.cuda.current_stream().synchronize()
+                want = out.clone()
+                for _ in range(10000):
+                    call(k)
+                torch.cuda.current_stream().synchronize()
+                assert torch.equal(out, want)
+        except Exception as e:
+            failed.append(e)
+            start.abort()
+
+    calls = [jobs(large) for large in (True, False, False, False)]
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=j) for j in calls]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
+
+
 @pytest.mark.parametrize("vocab", [3, 2048, 2049, 32000, 151936, 151937, 389120, 389121, 700000])
 def test_sampling_slices(K, vocab):
     """Slices of a row that are kept in shared memory and those that do not fit (more than 389,120 logits), rows that do not start
