@@ -174,13 +174,14 @@ constexpr float FIX_ONE = 1099511627776.0f;  // 2^40
 // the first radix pass (the key's top 8 bits: sign and exponent of the scaled logit) puts almost every element of a
 // row into a handful of bins: a thousand threads queueing there with such loops made a pure top-p row cost two
 // milliseconds. A row's masses sum to 2^40, so every chunk's sum over up to 2^17 elements stays below 2^32. Lanes that add
-// to one bin queue too, so there are COPIES of every histogram, a lane uses its own and each lies a bank further on.
-constexpr int COPIES = 8, BINS = 257;       // (bins of a copy, with the bank in between)
-__device__ __forceinline__ void mass_add(unsigned (*m)[COPIES * BINS], unsigned at, unsigned long long q) {
+// to one bin queue too, so there are copies of every histogram, a lane uses its own and each lies a bank further on. `at`: the
+// bin's place in the first of the three histograms, which lie `apart` places from one another.
+constexpr int BINS = 257;       // bins of a copy, with the bank in between
+__device__ __forceinline__ void mass_add(unsigned* at, int apart, unsigned long long q) {
     const unsigned a = (unsigned)(q & 0x3fffull), b = (unsigned)((q >> 14) & 0x3fffull), c = (unsigned)(q >> 28);
-    if (a) atomicAdd(&m[1][at], a);
-    if (b) atomicAdd(&m[2][at], b);
-    if (c) atomicAdd(&m[3][at], c);
+    if (a) atomicAdd(at, a);
+    if (b) atomicAdd(at + apart, b);
+    if (c) atomicAdd(at + 2 * apart, c);
 }
 
 // ---- the sampling kernel: a cluster of CS CTAs per row. One SM working through a row of 152K logits a dozen times was
@@ -190,9 +191,11 @@ __device__ __forceinline__ void mass_add(unsigned (*m)[COPIES * BINS], unsigned 
 // and of fixed-point masses: any order gives the same) or a float sum in a fixed order (threads, warps, lanes and CTAs
 // in ascending order), so a row's token depends on the row alone.
 constexpr int ST = 256;      // chunks of a CTA's slice: what is summed in order is summed by so many threads
-constexpr int NT = 512;      // threads of a CTA
 constexpr int CS = 8;        // CTAs of the cluster that shares a row
 constexpr size_t SAMPLE_SMEM = 200 * 1024;      // dynamic shared memory of a CTA at most
+// Threads of a CTA (NT) and copies of its histograms: 512 and 4 while all rows are at work at once, which is a matter of latency;
+// 256 and 1 for more rows, where what counts is the work of all of them together and how many an SM holds (see the launch).
+template <int NT> constexpr int COPIES = NT == 512 ? 4 : 1;
 
 __device__ __forceinline__ unsigned ld_peer_u32(unsigned addr) {
     unsigned v;
@@ -209,7 +212,7 @@ __device__ __forceinline__ unsigned long long ld_peer_u64(unsigned addr) {
 // the first pass has left them (a dozen passes over global memory, two loads in flight a thread, took half of the kernel's
 // time), or, for a vocabulary whose slice does not fit, from global memory each time. Element i of the slice; ``vec``: the
 // row starts on 16 bytes.
-template <bool KEPT>
+template <bool KEPT, int NT>
 struct Slice {
     const float* p;         // KEPT: shared memory, scaled; else the slice's first logit
     int n;
@@ -221,42 +224,57 @@ struct Slice {
         if (!KEPT) { v.x *= inv_t; v.y *= inv_t; v.z *= inv_t; v.w *= inv_t; }
         return v;
     }
+    // f(x) for the groups of four tid, tid + T, tid + 2 T, ... in ascending order; from global memory two of them are in flight (a
+    // thread with one load in flight waits out the whole latency of the memory system for every group)
+    template <int T, typename F>
+    __device__ __forceinline__ int fours(F&& f) const {
+        const int n4 = n >> 2;
+        int i = threadIdx.x;
+        for (; i + T < n4; i += 2 * T) {
+            const float4 a = at4(i), b = at4(i + T);
+            f(a.x); f(a.y); f(a.z); f(a.w);
+            f(b.x); f(b.y); f(b.z); f(b.w);
+        }
+        if (i < n4) {
+            const float4 a = at4(i);
+            f(a.x); f(a.y); f(a.z); f(a.w);
+        }
+        return 4 * n4;
+    }
     // f(x) for every element, in no particular order, by all threads of the CTA
     template <typename F>
     __device__ __forceinline__ void each(F&& f) const {
-        int done = 0;
-        if (KEPT || vec) {
-            const int n4 = n >> 2;
-#pragma unroll 2
-            for (int i = threadIdx.x; i < n4; i += blockDim.x) {
-                const float4 v = at4(i);
-                f(v.x); f(v.y); f(v.z); f(v.w);
-            }
-            done = 4 * n4;
-        }
-        for (int i = done + threadIdx.x; i < n; i += blockDim.x) f(at(i));
+        const int done = KEPT || vec ? fours<NT>(f) : 0;
+        for (int i = done + threadIdx.x; i < n; i += NT) f(at(i));
     }
     // the same by threads 0..ST-1, each its elements in ascending order: groups of four ST groups apart where the row starts
     // on 16 bytes, elements ST apart otherwise
     template <typename F>
     __device__ __forceinline__ void each_in_order(F&& f) const {
         if (threadIdx.x >= ST) return;
-        int done = 0;
-        if (vec) {
-            const int n4 = n >> 2;
-            for (int i = threadIdx.x; i < n4; i += ST) {
-                const float4 v = at4(i);
-                f(v.x); f(v.y); f(v.z); f(v.w);
-            }
-            done = 4 * n4;
-        }
+        const int done = vec ? fours<ST>(f) : 0;
         for (int i = done + threadIdx.x; i < n; i += ST) f(at(i));
     }
-    // f(i, x) for i = begin .. end - 1 in ascending order (a thread's chunk; begin is a multiple of 4), until f returns false
+    // f(i, x) for i = begin .. end - 1 in ascending order (a thread's chunk; begin is a multiple of 4), until f returns false; from
+    // global memory all of a group of 16 elements are sent for before the first is used
     template <typename F>
     __device__ __forceinline__ void chunk(int begin, int end, F&& f) const {
         int i = begin;
-        if (KEPT || vec) {
+        if (!KEPT && vec) {
+            for (; i + 16 <= end; i += 16) {
+                float4 v[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v[j] = at4((i >> 2) + j);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (!f(i + 4 * j, v[j].x)) return;
+                    if (!f(i + 4 * j + 1, v[j].y)) return;
+                    if (!f(i + 4 * j + 2, v[j].z)) return;
+                    if (!f(i + 4 * j + 3, v[j].w)) return;
+                }
+            }
+        }
+        if (KEPT) {
             for (; i + 4 <= end; i += 4) {
                 const float4 v = at4(i >> 2);
                 if (!f(i, v.x)) return;
@@ -276,20 +294,21 @@ __device__ __forceinline__ float weight(float d) { return __expf(d); }
 
 // temperature > 0 for every row given to this kernel. grid: CS CTAs (one cluster) per row. Dynamic shared memory: the
 // histograms' copies and, KEPT, the slice.
-template <bool KEPT>
-__global__ void __launch_bounds__(NT)
+template <bool KEPT, int NT>
+__global__ void __launch_bounds__(NT, NT == 512 ? 2 : 5)
 sample_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p, const float* __restrict__ uniform,
               int* __restrict__ out) {
     using namespace nibp;
     extern __shared__ __align__(16) float dyn[];
-    unsigned (*copies)[COPIES * BINS] = reinterpret_cast<unsigned (*)[COPIES * BINS]>(dyn);      // counts, then masses as three histograms
-    float* kept = dyn + 4 * COPIES * BINS;          // of 14-bit chunks: mass = m1 + m2 * 2^14 + m3 * 2^28
+    constexpr int HIST = COPIES<NT> * BINS;
+    unsigned* copies = reinterpret_cast<unsigned*>(dyn);      // [4][HIST]: counts, then masses as three histograms
+    float* kept = dyn + 4 * HIST;                   // of 14-bit chunks: mass = m1 + m2 * 2^14 + m3 * 2^28
     __shared__ float scratch[NT / 32];
     __shared__ unsigned pub[2][4][256];             // this CTA's histograms of a radix pass, for the cluster; the passes take turns
     __shared__ unsigned tot_hist[256];              // the cluster's sums
     __shared__ unsigned long long tot_mass[256];
-    __shared__ unsigned dec_prefix, dec_remaining;  // what a radix pass decided (every CTA decides for itself, alike)
+    __shared__ unsigned dec_prefix, dec_remaining;  // what a radix pass decided (512 threads: every CTA for itself, alike; 256: CTA 0)
     __shared__ unsigned long long dec_above;
     __shared__ float x_max, x_z, x_total;           // what this CTA tells the others
     __shared__ int x_ties;
@@ -310,7 +329,7 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
     const int s_begin = min(vocab, (int)rank * ST * per), s_n = min(vocab, s_begin + ST * per) - s_begin;
     const int begin = tid < ST ? min(s_n, tid * per) : 0, end = tid < ST ? min(s_n, begin + per) : 0;
     const bool vec = (reinterpret_cast<uintptr_t>(l) & 15) == 0;
-    const Slice<KEPT> slice{KEPT ? kept : l + s_begin, s_n, inv_t, vec};
+    const Slice<KEPT, NT> slice{KEPT ? kept : l + s_begin, s_n, inv_t, vec};
 
     auto cta_reduce = [&](float v, bool is_max, int warps) -> float {      // over the CTA's first warps, in a fixed order
         v = is_max ? warp_max(v) : warp_sum(v);
@@ -352,15 +371,16 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
     cluster_sync();
     for (unsigned r = 0; r < CS; ++r) mx = fmaxf(mx, ld_peer_f32(peer_smem(&x_max, r)));
 
-    // One radix pass over the slice: histogram (and masses), told to the cluster; every CTA sums them up and chooses the
-    // digit (``choose``, warp 0). A pass tells its results in the buffer of the pass before the last one: whoever is past the
-    // last pass's barrier has read that.
+    // One radix pass over the slice: histogram (and masses), told to the cluster, which sums them up and chooses the digit
+    // (``choose``, warp 0). With 512 threads every CTA does so for itself: one barrier of the cluster a pass instead of two. With 256
+    // CTA 0 does it for all, an eighth of the reads of peers' memory. A pass tells its results in the buffer of the pass before
+    // the last one: whoever is past the last pass's barrier has read that.
     int pass = 0;
-    const unsigned copy = (lane & (COPIES - 1)) * BINS;
+    const unsigned copy = (lane & (COPIES<NT> - 1)) * BINS;
     auto radix_pass = [&](bool with_mass, auto&& add, auto&& choose) {
         unsigned (*mine)[256] = pub[pass++ & 1];
         const int used = with_mass ? 4 : 1;
-        for (int i = tid; i < used * COPIES * BINS; i += NT) copies[0][i] = 0u;
+        for (int i = tid; i < used * HIST; i += NT) copies[i] = 0u;
         __syncthreads();
         slice.each(add);
         __syncthreads();
@@ -368,34 +388,41 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
             const int h = i >> 8, b = i & 255;
             unsigned sum = 0u;
 #pragma unroll
-            for (int c = 0; c < COPIES; ++c) sum += copies[h][c * BINS + b];
+            for (int c = 0; c < COPIES<NT>; ++c) sum += copies[h * HIST + c * BINS + b];
             mine[h][b] = sum;
         }
         cluster_sync();
-        if (tid < 256) {
-            unsigned v[CS], n = 0u;
+        if (NT == 512 || rank == 0) {
+            const int b = tid & 255;
+            if (NT == 256 || tid < 256) {
+                unsigned v[CS], n = 0u;
 #pragma unroll
-            for (unsigned r = 0; r < CS; ++r) v[r] = ld_peer_u32(peer_smem(&mine[0][tid], r));
+                for (unsigned r = 0; r < CS; ++r) v[r] = ld_peer_u32(peer_smem(&mine[0][b], r));
 #pragma unroll
-            for (unsigned r = 0; r < CS; ++r) n += v[r];
-            tot_hist[tid] = n;
-        } else if (with_mass) {
-            const int b = tid - 256;
-            unsigned v[3][CS];
-            unsigned long long m = 0ull;
+                for (unsigned r = 0; r < CS; ++r) n += v[r];
+                tot_hist[b] = n;
+            }
+            if (with_mass && (NT == 256 || tid >= 256)) {
+                unsigned v[3][CS];
+                unsigned long long m = 0ull;
 #pragma unroll
-            for (unsigned r = 0; r < CS; ++r)
+                for (unsigned r = 0; r < CS; ++r)
 #pragma unroll
-                for (int h = 0; h < 3; ++h) v[h][r] = ld_peer_u32(peer_smem(&mine[1 + h][b], r));
+                    for (int h = 0; h < 3; ++h) v[h][r] = ld_peer_u32(peer_smem(&mine[1 + h][b], r));
 #pragma unroll
-            for (unsigned r = 0; r < CS; ++r) m += (unsigned long long)v[0][r] + ((unsigned long long)v[1][r] << 14) + ((unsigned long long)v[2][r] << 28);
-            tot_mass[b] = m;
+                for (unsigned r = 0; r < CS; ++r) m += (unsigned long long)v[0][r] + ((unsigned long long)v[1][r] << 14) + ((unsigned long long)v[2][r] << 28);
+                tot_mass[b] = m;
+            }
+            __syncthreads();
+            if (tid < 32) choose();          // warp 0: lane j looks at the bins 8j..8j+7
         }
-        __syncthreads();
-        if (tid < 32) choose();          // warp 0: lane j looks at the bins 8j..8j+7
-        __syncthreads();
+        if (NT == 512)
+            __syncthreads();
+        else
+            cluster_sync();
     };
-    static_assert(NT == 512, "the first 256 threads sum the counts, the others the masses");
+    static_assert(NT == 512 || NT == 256, "the first 256 threads sum the counts, the last 256 the masses");
+    const unsigned decider = NT == 512 ? rank : 0u;
 
     // ---- top-k: key of the k-th largest scaled logit (0 keeps everything)
     unsigned kth_key = 0u;
@@ -407,7 +434,7 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
             radix_pass(false,
                        [&](float x) {
                            const unsigned key = key_of(x);
-                           if ((key & mask) == prefix) atomicAdd(&copies[0][copy + ((key >> shift) & 255u)], 1u);
+                           if ((key & mask) == prefix) atomicAdd(&copies[copy + ((key >> shift) & 255u)], 1u);
                        },
                        [&]() {
                            // the highest bin b >= 1 with (elements in bins >= b) >= remaining, else bin 0; what is still to
@@ -438,8 +465,8 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
                                dec_remaining = has ? r : remaining - (all - tot_hist[0]);
                            }
                        });
-            prefix = dec_prefix;
-            remaining = dec_remaining;
+            prefix = ld_peer_u32(peer_smem(&dec_prefix, decider));
+            remaining = ld_peer_u32(peer_smem(&dec_remaining, decider));
         }
         kth_key = prefix;
     }
@@ -470,9 +497,9 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
                        [&](float x) {
                            const unsigned key = key_of(x);
                            if (key >= kth_key && (key & mask) == prefix) {
-                               const unsigned at = copy + ((key >> shift) & 255u);
-                               mass_add(copies, at, (unsigned long long)(weight(x - mx) * fix_over_z));
-                               atomicAdd(&copies[0][at], 1u);
+                               unsigned* at = copies + copy + ((key >> shift) & 255u);
+                               mass_add(at + HIST, HIST, (unsigned long long)(weight(x - mx) * fix_over_z));
+                               atomicAdd(at, 1u);
                            }
                        },
                        [&]() {
@@ -515,8 +542,8 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
                                dec_above = chosen_above;
                            }
                        });
-            prefix = dec_prefix;
-            above0 = dec_above;
+            prefix = ld_peer_u32(peer_smem(&dec_prefix, decider));
+            above0 = ld_peer_u64(peer_smem(&dec_above, decider));
         }
         p_key = prefix;
         if (p_key < kth_key) p_key = kth_key;
@@ -663,14 +690,23 @@ NIB_API int nib_sample(const float* logits, int rows, int vocab, const float* te
     if (rows == 0) return 0;
     NIB_REQUIRE((long long)vocab <= (1LL << 17) * 8, "sample: a row of %d logits is more than the fixed-point histograms hold", vocab);
     const int per = (ceil_div(vocab, CS * ST) + 3) & ~3;
-    const size_t hist = sizeof(unsigned) * 4 * COPIES * BINS, slice = sizeof(float) * (size_t)ST * per;
-    const bool kept = hist + slice <= SAMPLE_SMEM;
-    const size_t smem = hist + (kept ? slice : 0);
+    // Up to 32 rows all CTAs are at work at once, two an SM, and a row's time is what counts: 512 threads, and the slice kept in
+    // shared memory if two of them fit an SM's (else for the 12 rows that one an SM holds). More rows: as many CTAs an SM as there can
+    // be (five), and the slice kept only where it is small. Measured at a vocabulary of 151,936, top-p 0.9, us: 1 row 47 (68 with 256
+    // threads and nothing kept), 12 rows 49 (70), 16 rows 64 (82; 93 with one CTA an SM), 32 rows 69 (85; 143), 34 rows 97 (with 512
+    // threads, which are two turns then, 99), 64 rows 122 (131); 32,000: 34 rows 35 (51 with 512 threads), 64 rows 41 (64; 53 with
+    // nothing kept).
+    const size_t slice = sizeof(float) * (size_t)ST * per;
+    const auto room = [&](int copies) { return sizeof(unsigned) * 4 * copies * BINS + slice; };
+    const bool wide = rows <= 32;
+    const bool kept = wide ? room(COPIES<512>) <= (rows <= 12 ? SAMPLE_SMEM : 98 * 1024) : room(COPIES<256>) <= 30 * 1024;
+    const size_t smem = room(wide ? COPIES<512> : COPIES<256>) - (kept ? 0 : slice);
+    auto* kernel = wide ? (kept ? sample_kernel<true, 512> : sample_kernel<false, 512>) : (kept ? sample_kernel<true, 256> : sample_kernel<false, 256>);
     // the most that any call takes: the attribute is the kernel's, and a call's own size would lower it under another thread's launch
-    if (kept) NIB_CUDA(cudaFuncSetAttribute(sample_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SAMPLE_SMEM));
+    if (kept && wide) NIB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SAMPLE_SMEM));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(rows * CS);
-    cfg.blockDim = dim3(NT);
+    cfg.blockDim = dim3(wide ? 512 : 256);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -680,7 +716,7 @@ NIB_API int nib_sample(const float* logits, int rows, int vocab, const float* te
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    NIB_CUDA(cudaLaunchKernelEx(&cfg, kept ? sample_kernel<true> : sample_kernel<false>, logits, vocab, temperature, top_k, top_p, uniform, out));
+    NIB_CUDA(cudaLaunchKernelEx(&cfg, kernel, logits, vocab, temperature, top_k, top_p, uniform, out));
     NIB_LAUNCH_CHECK();
     return 0;
 }

@@ -1024,9 +1024,9 @@ def test_launches_of_unlike_sizes_from_several_threads(K, which):
     assert not failed, failed
 
 
-@pytest.mark.parametrize("vocab", [3, 2048, 2049, 32000, 151936, 151937, 389120, 389121, 700000])
+@pytest.mark.parametrize("vocab", [3, 2048, 2049, 32000, 151936, 151937, 368640, 368641, 389121, 700000])
 def test_sampling_slices(K, vocab):
-    """Slices of a row that are kept in shared memory and those that do not fit (more than 389,120 logits), rows that do not start
+    """Slices of a row that are kept in shared memory and those that do not fit (of five rows: more than 368,640 logits), rows that do not start
     on 16 bytes, slices that are empty: the drawn token is the plain pipeline's wherever the number drawn is not within rounding
     (1e-4 of the mass) of the border between two tokens, and a row's token does not depend on the rows beside it."""
     rows = 5
@@ -1049,3 +1049,22 @@ def test_sampling_slices(K, vocab):
         K.sample(logits[r:r + 1].clone(), temperature[r:r + 1], top_k[r:r + 1], top_p[r:r + 1], uniform[r:r + 1], alone)
         # (a row that starts on 16 bytes adds up its normaliser in another order than one that does not)
         assert int(alone[0]) == t or vocab % 4, (r, t)
+
+
+@pytest.mark.parametrize("vocab", [5, 2052, 49152, 49156, 151936, 163840, 163844, 368640, 368644])
+def test_sampling_of_many_rows(K, vocab):
+    """Up to 12 rows, up to 32 and more take other numbers of threads and keep slices of other lengths: every row's token is the one it
+    gets alone."""
+    for rows in (12, 13, 32, 33, 70):
+        logits = 2.0 * rnd((rows, vocab), torch.float32, 108)
+        logits[:, :: max(1, vocab // 37)] += 5.0
+        i = torch.arange(rows, device="cuda")
+        temperature, top_p = 0.6 + 0.05 * (i % 9), torch.tensor([1.0, 0.9, 1.0, 0.8, 0.95], device="cuda")[i % 5]
+        top_k = torch.tensor([0, 0, 40, 7, 0, 50, 1], dtype=torch.int32, device="cuda")[i % 7]
+        uniform = torch.rand(rows, generator=torch.Generator().manual_seed(109)).cuda()
+        out, alone = (torch.empty(n, dtype=torch.int32, device="cuda") for n in (rows, 1))
+        K.sample(logits, temperature, top_k, top_p, uniform, out)
+        for r in range(rows):
+            if (r * vocab) % 4 == 0:        # (a row that does not start on 16 bytes adds up in another order)
+                K.sample(logits[r:r + 1], temperature[r:r + 1], top_k[r:r + 1], top_p[r:r + 1], uniform[r:r + 1], alone)
+                assert int(alone[0]) == int(out[r]), (rows, r)
