@@ -628,9 +628,12 @@ class Kernels:
         """Into how many CTAs the keys of a decoding token are split. The kernel with TMA page loads keeps
         several tiles in flight per CTA: about 256 CTAs in all (measured best from 1 to 64 requests), at
         least four of its tiles (128 keys for heads of 64, else 64) each. While that leaves SMs without work, up to eight CTAs
-        that merge in one cluster and a tile each will do, as long as every CTA has an SM (one token of 777 keys, heads of 64:
-        3.7 us with eight, 6.7 with one; 4 tokens of 1,500: 4.8 and 6.9 with two; 24 tokens of up to 1,500: 7.0 with two, 7.4
-        with four, 11.6 with one), but not with a window, whose few tiles come at any context. More than one cluster of eight
+        that merge in one cluster and a tile each will do: eight while tokens and kv heads leave 16 SMs for each (heads of 64) or
+        8 (heads of 128), four while they leave 4 (heads of 64, four tiles or less: 8). Heads of 64, us, with the norm of a few rows before
+        it: one token of 600 keys, 5.3 with eight, 6.4 with two; 4 tokens of 1,300, 6.3 and 6.7 with four; 8 of 800, 6.5 with
+        four, 6.9 with eight, 7.4 with two; 8 of 450, 6.0 with four, 6.8 with one, 12 of 350, 6.3 and 6.1. Not for contexts of 256
+        keys or less, which replayed steps do not tell apart: one token of 40 keys takes 4.4 with one CTA and 5.2 with two, with heads
+        of 128 5.0 and 5.9 with four (255 keys: 6.7 and 6.0). Not with a window, whose few tiles come at any context. More than one cluster of eight
         a token and kv head, and with it a second kernel, only where eight leave SMs idle
         (heads of 128, 8 tokens of 4,096: 11.4 us with 8, 13.0 with 16; 1 token: 9.3 and 8.9). The cp.async kernel: two key tiles
         per CTA (both are in flight at once, so a
@@ -646,8 +649,13 @@ class Kernels:
             tile_keys = 128 if head_dim == 64 else 64           # the kernel's tile
             tiles = -(-keys // tile_keys)
             n = max(1, min(want, tiles // 4, 64))
-            if window <= 0 and units <= self.sm_count:
-                n = max(n, min(8, 1 << (self.sm_count // units).bit_length() - 1, 1 << (tiles - 1).bit_length()))
+            if window <= 0 and max_ctx > 256:
+                share = self.sm_count // units          # SMs for each token and kv head
+                if head_dim == 64:
+                    most = 8 if share >= 16 else 4 if share >= (4 if tiles > 4 else 8) else 1
+                else:
+                    most = 8 if share >= 8 else 4 if share >= 4 else 1
+                n = max(n, min(most, 1 << (tiles - 1).bit_length()))
             if n > 8 and 8 * units >= 128:
                 n = 8
             return _cluster_splits(n)

@@ -91,10 +91,22 @@ def test_decode_attention_splits(rules):
 def test_decode_attention_splits_while_sms_are_idle(rules):
     # up to a cluster of eight CTAs for a context of a few tiles, as long as every CTA has an SM
     assert rules.decode_splits(1, 2, 777, 0, True, 64) == 8
-    assert rules.decode_splits(1, 2, 200, 0, True, 64) == 2              # two tiles of 128 keys
+    assert rules.decode_splits(1, 2, 400, 0, True, 64) == 4              # four tiles of 128 keys
     assert rules.decode_splits(24, 2, 1500, 0, True, 64) == 2
     assert rules.decode_splits(74, 2, 777, 0, True, 64) == 1             # 148 CTAs as it is
     assert rules.decode_splits(1, 2, 777, 512, True, 64) == 1            # a window: few tiles at any context
     # more than one cluster a token and kv head only where eight CTAs leave SMs idle
     assert rules.decode_splits(8, 2, 4096, 0, True, 128) == 8
     assert rules.decode_splits(1, 2, 4096, 0, True, 128) == 16
+
+
+def test_decode_attention_splits_of_short_contexts(rules):
+    # a replayed step plans for 256 keys at least: whatever it holds up to there is one CTA's work
+    for heads_dim in (64, 128):
+        for n_tokens in (1, 4, 8, 16, 37, 64):
+            for keys in (17, 128, 200, 256):
+                assert rules.decode_splits(n_tokens, 2, keys, 0, True, heads_dim) == 1
+    # heads of 64: eight CTAs while 16 SMs are left for each token and kv head, four while 4 are (a context of four tiles: 8)
+    assert [rules.decode_splits(n, 2, 512, 0, True, 64) for n in (1, 4, 8, 9, 10, 16, 32)] == [4, 4, 4, 4, 1, 1, 1]
+    assert [rules.decode_splits(n, 2, 1024, 0, True, 64) for n in (1, 4, 5, 8, 16, 18, 19, 32)] == [8, 8, 4, 4, 4, 4, 2, 2]
+    assert [rules.decode_splits(n, 2, 512, 0, True, 128) for n in (1, 9, 10, 18, 19, 32)] == [8, 8, 4, 4, 2, 2]
