@@ -10,9 +10,16 @@
 // blocks.
 //
 // A CTA takes one token and up to eight query heads that read the same keys: a key is fetched once for all of them. Its
-// warps take blocks in turn; a warp sends for all keys and values of its block at once (a block costs one trip to memory:
-// that latency is what bounds a token with a short context), then a lane owns a key for the scores and channels lane,
-// lane + 32, ... of the output for the values.
+// warps take blocks in turn; a warp sends for all keys and values of its block at once, as they are stored (a block costs one
+// trip to memory: that latency is what bounds a token with a short context, and how many blocks an SM has under way a prompt),
+// then a lane owns a key for the scores and channels of the output for the values. (Sending for the next block's keys under
+// the sums of this one's values was slower: one token of 777 keys, 14 heads of 64, 32-bit, 27.5 us instead of 23.7.)
+//
+// us, with a warp per (token, head) that reads keys from global memory / with rows of 32-bit numbers that bfloat16 was copied into
+// element by element / this: bfloat16, 8 heads of 72, a prompt of 1,024 tokens, 757 / 3,896 / 300; 64 tokens of 500 keys,
+// 218 / 299 / 25; 16 tokens, 8 and 2 heads of 100, 14.6 / 44.8 / 8.1; 32-bit, 8 heads of 72, 1,024 tokens, 873 / 1,039 / 620; one token of
+// 777 keys, 14 and 2 heads of 64, 323 / 22.3 / 19.9. Rows of an odd number of elements go as 32-bit words: 8 heads of 33 and 16 tokens,
+// 9.1 / 26 / 8.2, but 8 heads of 129 and 1,024 tokens, bfloat16, 1,134 / - / 1,802 (one token of 777 keys, 474 / - / 68).
 //
 // Formula: cpp/src/ops.cpp:206-270 (score = dot * scale, scale after the dot; max-subtracted exp;
 // sum of p_j v_j / sum p_j); kv head = head / (heads / kv_heads): cpp/src/paged.cpp:171. Warp-level
@@ -24,13 +31,18 @@ constexpr int GEN_MAX_WARPS = 8;
 constexpr int GEN_BLOCK = 32;            // keys of a block: a lane each
 constexpr size_t GEN_SMEM = 200 * 1024;
 
-// Floats of a CTA's shared memory: queries [R][pitch], running output [R][pitch], running (max, sum) twice; per warp keys
-// and values [32][pitch], weights [32][R], the block's (max, sum). Rows are padded with zeros to a multiple of four and lie
-// an odd number of 16-byte units apart: eight lanes that read a row each meet no bank conflict. A block's output takes
-// the place of its keys.
-__host__ __device__ constexpr int gen_pitch(int d) { return ((d + 3) / 4 | 1) * 4; }
-__host__ __device__ constexpr int gen_warp_floats(int R, int d) { return 2 * GEN_BLOCK * gen_pitch(d) + GEN_BLOCK * R + (2 * R + 3) / 4 * 4; }
-__host__ __device__ constexpr int gen_cta_floats(int R, int d) { return 2 * R * gen_pitch(d) + 4 * R; }
+// A CTA's shared memory: queries [R][pitch] floats, running output [R][pitch], running (max, sum) twice; per warp keys and values
+// [32][row] in the storage type, weights [32][R], the block's (max, sum). Rows are padded with zeros to whole 16-byte units of the
+// storage type and lie an odd number of them apart: eight lanes that read a row each meet no bank conflict. A block's output,
+// [R][pitch] floats, takes the place of its keys (R <= 8, and a row has at least as many bytes as a pitch has floats).
+// (`unit`, see gen_send_rows(): 0 takes room for one element more.)
+template <typename T> __host__ __device__ constexpr int gen_row(int d, int unit) { return (int)(((d + (unit == 0)) * sizeof(T) + 15) / 16 | 1) * 16; }      // bytes
+template <typename T> __host__ __device__ constexpr int gen_filled(int d) { return (int)((d * sizeof(T) + 15) / 16 * (16 / sizeof(T))); }  // elements
+template <typename T> __host__ __device__ constexpr int gen_pitch(int d) { return (gen_filled<T>(d) / 4 | 1) * 4; }              // floats
+template <typename T> __host__ __device__ constexpr int gen_warp_bytes(int R, int d, int unit) {
+    return 2 * GEN_BLOCK * gen_row<T>(d, unit) + 4 * (GEN_BLOCK * R + (2 * R + 3) / 4 * 4);
+}
+template <typename T> __host__ __device__ constexpr int gen_cta_bytes(int R, int d) { return 4 * (2 * R * gen_pitch<T>(d) + 4 * R); }
 
 // R floats from shared memory (16-byte aligned where R is a multiple of four).
 template <int R>
@@ -47,50 +59,146 @@ __device__ __forceinline__ void gen_load(float (&v)[R], const float* p) {
     }
 }
 
-// The block's rows of keys or values into shared memory as floats, by one warp: row jj is row `row` of lane jj in the pages
-// (below 0: zeros). 32-bit rows that start on 16 bytes go as asynchronous copies, as many rows at a time as the warp's lanes
-// cover: nothing waits for them here. (What lies behind a row is read, but what comes of it is not.)
-template <typename T>
-__device__ __forceinline__ void gen_send_rows(float* dst, const T* pages, long long row, int d, int pitch, bool wide, int lane) {
-    if (sizeof(T) == 4 && wide) {
-        const int units = d >> 2, per_row = units <= 8 ? 8 : units <= 16 ? 16 : 32, u0 = lane & (per_row - 1);
+// The block's rows of keys or values into shared memory, by one warp: row jj is row `row` of lane jj in the pages (below 0:
+// zeros). Asynchronous copies of U bytes, 32 consecutive ones of the block at a time: nothing waits for them here.
+template <typename T, int U>
+__device__ __forceinline__ void gen_send_units(unsigned char* dst, int pitch, const T* pages, long long row, int d, int lane) {
+    const int units = gen_filled<T>(d) * (int)sizeof(T) / U, have = U == 16 ? units : d * (int)sizeof(T) / U;
+    const unsigned to = (unsigned)__cvta_generic_to_shared(dst);
+    const int step_r = 32 / units, step_u = 32 - step_r * units;
+    int r = lane / units, u = lane - r * units;
 #pragma unroll 4
-        for (int r = lane / per_row; r < GEN_BLOCK; r += 32 / per_row) {
-            const long long rj = __shfl_sync(0xffffffffu, row, r);
-            const T* src = pages + max(rj, 0ll) * d;
-            const unsigned to = (unsigned)__cvta_generic_to_shared(dst + r * pitch);
-            for (int u = u0; u < units; u += per_row)
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(to + 16 * u), "l"(src + 4 * u), "r"(rj >= 0 ? 16 : 0) : "memory");
+    for (int k = 0; k < units; ++k) {
+        const long long rj = __shfl_sync(0xffffffffu, row, r);
+        const char* src = reinterpret_cast<const char*>(pages + max(rj, 0ll) * d);
+        const bool there = rj >= 0 && u < have;
+        if (U == 16)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(to + r * pitch + U * u), "l"(src + U * u), "r"(there ? U : 0) : "memory");
+        else
+            asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n"
+                         ::"r"(to + r * pitch + U * u), "l"(there ? src + U * u : src), "n"(U), "r"(there ? U : 0) : "memory");
+        r += step_r;
+        u += step_u;
+        if (u >= units) {
+            u -= units;
+            ++r;
         }
+    }
+}
+// Rows of bfloat16 that begin at any element (an odd width, say): the 32-bit words that a row lies in, its first element in the upper
+// half of the first one if the row begins in the middle of a word (the lower half is the row's before it; no word is read that holds
+// nothing of the row). gen_align_rows() moves such a row down by an element.
+__device__ __forceinline__ void gen_send_words(unsigned char* dst, int pitch, const __nv_bfloat16* pages, long long row, int d, int lane) {
+    const int words = max(gen_filled<__nv_bfloat16>(d), d + 2) / 2, step_r = 32 / words, step_u = 32 - step_r * words;
+    const unsigned to = (unsigned)__cvta_generic_to_shared(dst);
+    int r = lane / words, u = lane - r * words;
+#pragma unroll 4
+    for (int k = 0; k < words; ++k) {
+        const long long rj = __shfl_sync(0xffffffffu, row, r);
+        const uintptr_t begin = reinterpret_cast<uintptr_t>(pages + max(rj, 0ll) * d), first = begin & ~(uintptr_t)3;
+        const int bytes = rj >= 0 ? max(0, min(4, (int)(begin - first) + 2 * d - 4 * u)) : 0;       // 2: the word's upper half is not the row's
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n"
+                     ::"r"(to + r * pitch + 4 * u), "l"(first + (bytes > 0 ? 4 * u : 0)), "r"(bytes) : "memory");
+        r += step_r;
+        u += step_u;
+        if (u >= words) {
+            u -= words;
+            ++r;
+        }
+    }
+}
+__device__ __forceinline__ void gen_align_rows(unsigned char* dst, int pitch, const __nv_bfloat16* pages, long long row, int d, int lane) {
+    const int words = max(gen_filled<__nv_bfloat16>(d), d + 2) / 2;
+    unsigned odd = __ballot_sync(0xffffffffu, row >= 0 && (reinterpret_cast<uintptr_t>(pages + max(row, 0ll) * d) & 2) != 0);
+    for (; odd != 0; odd &= odd - 1) {
+        unsigned* w = reinterpret_cast<unsigned*>(dst + (__ffs(odd) - 1) * pitch);
+        for (int u0 = 0; u0 < words; u0 += 32) {
+            const int u = u0 + lane;
+            const unsigned low = u < words ? w[u] >> 16 : 0u, high = u + 1 < words ? w[u + 1] << 16 : 0u;
+            __syncwarp();
+            if (u < words) w[u] = low | high;
+            __syncwarp();
+        }
+    }
+}
+// `unit`: the largest of 16, 8 and 4 bytes that the rows are made of; 0 where there is none.
+template <typename T>
+__device__ __forceinline__ void gen_send_rows(unsigned char* dst, int pitch, const T* pages, long long row, int d, int unit, int lane) {
+    if (unit == 16) {
+        gen_send_units<T, 16>(dst, pitch, pages, row, d, lane);
+    } else if (unit == 8) {
+        gen_send_units<T, 8>(dst, pitch, pages, row, d, lane);
+    } else if (sizeof(T) == 4 || unit == 4) {
+        gen_send_units<T, 4>(dst, pitch, pages, row, d, lane);
     } else {
-        for (int r = 0; r < GEN_BLOCK; ++r) {
-            const long long rj = __shfl_sync(0xffffffffu, row, r);
-            const T* src = pages + max(rj, 0ll) * d;
-            for (int i = lane; i < pitch; i += 32) dst[r * pitch + i] = rj >= 0 && i < d ? Elem<T>::load(src + i) : 0.f;
+        if constexpr (sizeof(T) == 2) gen_send_words(dst, pitch, pages, row, d, lane);
+    }
+}
+
+// Two bfloat16 of a 32-bit word.
+__device__ __forceinline__ float gen_low(unsigned w) { return __uint_as_float(w << 16); }
+__device__ __forceinline__ float gen_high(unsigned w) { return __uint_as_float(w & 0xffff0000u); }
+
+// s[r] += q[r] . k over the 16 bytes of a key at `k`, in ascending order of the elements; queries `pitch` floats apart.
+template <typename T, int R>
+__device__ __forceinline__ void gen_dot(float (&s)[R], const float* q, int pitch, const unsigned char* k) {
+    float kd[16 / sizeof(T)];
+    if constexpr (sizeof(T) == 4) {
+        *reinterpret_cast<float4*>(kd) = *reinterpret_cast<const float4*>(k);
+    } else {
+        const uint4 w = *reinterpret_cast<const uint4*>(k);
+        kd[0] = gen_low(w.x); kd[1] = gen_high(w.x); kd[2] = gen_low(w.y); kd[3] = gen_high(w.y);
+        kd[4] = gen_low(w.z); kd[5] = gen_high(w.z); kd[6] = gen_low(w.w); kd[7] = gen_high(w.w);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int i = 0; i < (int)(16 / sizeof(T)); i += 4) {
+            const float4 qd = *reinterpret_cast<const float4*>(q + r * pitch + i);
+            s[r] = fmaf(qd.w, kd[i + 3], fmaf(qd.z, kd[i + 2], fmaf(qd.y, kd[i + 1], fmaf(qd.x, kd[i], s[r]))));
+        }
+}
+// The output channel that a lane's i-th sum is of: 32 apart, or pairs 64 apart where a word holds two values.
+template <typename T> __device__ __forceinline__ int gen_channel(int i, int lane) {
+    return sizeof(T) == 4 ? lane + 32 * i : 2 * lane + 64 * (i >> 1) + (i & 1);
+}
+template <typename T, int DI>
+__device__ __forceinline__ void gen_values(float (&v)[DI], const unsigned char* row, int filled, int lane) {
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll
+        for (int i = 0; i < DI; ++i) v[i] = lane + 32 * i < filled ? reinterpret_cast<const float*>(row)[lane + 32 * i] : 0.f;
+    } else {
+#pragma unroll
+        for (int i = 0; i < DI; i += 2) {
+            const unsigned w = 2 * lane + 32 * i < filled ? reinterpret_cast<const unsigned*>(row)[lane + 16 * i] : 0u;
+            v[i] = gen_low(w);
+            v[i + 1] = gen_high(w);
         }
     }
 }
 
 template <typename T, int R, int DI>
-__global__ void __launch_bounds__(GEN_MAX_WARPS * 32)
+__global__ void __launch_bounds__(GEN_MAX_WARPS * 32, R <= 2 ? 4 : 2)
 attention_generic_kernel(const T* __restrict__ qkv, int q_stride, T* __restrict__ out,
                          const int* __restrict__ positions, const int* __restrict__ req_index,
                          const int* __restrict__ block_table, int bt_stride, int page_size,
                          const T* __restrict__ k_pages, const T* __restrict__ v_pages, int num_pages,
-                         int heads, int kv_heads, int head_dim, float scale, int window, int wide) {
+                         int heads, int kv_heads, int head_dim, float scale, int window, int unit) {
     extern __shared__ __align__(16) float smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     const int group = heads / kv_heads, sets = (group + R - 1) / R;
     const int set = blockIdx.x % sets, kvh = (blockIdx.x / sets) % kv_heads, token = blockIdx.x / (sets * kv_heads);
     const int h0 = kvh * group + set * R, n_heads = min(R, group - set * R);
-    const int pitch = gen_pitch(head_dim);
+    const int pitch = gen_pitch<T>(head_dim), key_row = gen_row<T>(head_dim, unit), filled = gen_filled<T>(head_dim);
+    const int warp_floats = gen_warp_bytes<T>(R, head_dim, unit) / 4;
     float* q_s = smem;                                  // [R][pitch]
     float* tot = q_s + R * pitch;                       // [R][pitch]
     float* ml = tot + R * pitch;                        // two copies of [R][2]
-    float* base = ml + 4 * R;
-    float* k_s = base + (size_t)warp * gen_warp_floats(R, head_dim);      // [32][pitch]; then the block's output [R][pitch]
-    float* v_s = k_s + GEN_BLOCK * pitch;               // [32][pitch]
-    float* p_s = v_s + GEN_BLOCK * pitch;               // [32][R]
+    float* base = ml + 4 * R;                           // per warp: keys (then the block's output), values, weights, (max, sum)
+    float* o_s = base + (size_t)warp * warp_floats;     // [R][pitch]
+    unsigned char* k_s = reinterpret_cast<unsigned char*>(o_s);      // [32][key_row]
+    unsigned char* v_s = k_s + GEN_BLOCK * key_row;
+    float* p_s = reinterpret_cast<float*>(v_s + GEN_BLOCK * key_row);      // [32][R]
     float* b_ml = p_s + GEN_BLOCK * R;                  // [R][2]
     pdl_launch_dependents();
     pdl_wait();
@@ -120,24 +228,19 @@ attention_generic_kernel(const T* __restrict__ qkv, int q_stride, T* __restrict_
                 const int page = bt[j / page_size];
                 if (page >= 0 && page < num_pages) row = ((long long)page * kv_heads + kvh) * page_size + j % page_size;
             }
-            gen_send_rows(k_s, k_pages, row, head_dim, pitch, wide, lane);
+            gen_send_rows(k_s, key_row, k_pages, row, head_dim, unit, lane);
             asm volatile("cp.async.commit_group;\n" ::: "memory");
-            gen_send_rows(v_s, v_pages, row, head_dim, pitch, wide, lane);
+            gen_send_rows(v_s, key_row, v_pages, row, head_dim, unit, lane);
             asm volatile("cp.async.commit_group;\n" ::: "memory");
             asm volatile("cp.async.wait_group 1;\n" ::: "memory");
             __syncwarp();
+            if constexpr (sizeof(T) == 2)
+                if (unit == 0) gen_align_rows(k_s, key_row, k_pages, row, head_dim, lane);
             float s[R];
 #pragma unroll
             for (int r = 0; r < R; ++r) s[r] = 0.f;
 #pragma unroll 4
-            for (int d = 0; d < head_dim; d += 4) {
-                const float4 kd = *reinterpret_cast<const float4*>(k_s + lane * pitch + d);
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const float4 qd = *reinterpret_cast<const float4*>(q_s + r * pitch + d);
-                    s[r] = fmaf(qd.w, kd.w, fmaf(qd.z, kd.z, fmaf(qd.y, kd.y, fmaf(qd.x, kd.x, s[r]))));
-                }
-            }
+            for (int d = 0; d < filled; d += 16 / sizeof(T)) gen_dot<T, R>(s, q_s + d, pitch, k_s + lane * key_row + d * sizeof(T));
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 s[r] = row >= 0 ? s[r] * scale : -INFINITY;
@@ -152,6 +255,8 @@ attention_generic_kernel(const T* __restrict__ qkv, int q_stride, T* __restrict_
             }
             asm volatile("cp.async.wait_group 0;\n" ::: "memory");
             __syncwarp();
+            if constexpr (sizeof(T) == 2)
+                if (unit == 0) gen_align_rows(v_s, key_row, v_pages, row, head_dim, lane);
             float acc[R][DI];
 #pragma unroll
             for (int r = 0; r < R; ++r)
@@ -161,8 +266,7 @@ attention_generic_kernel(const T* __restrict__ qkv, int q_stride, T* __restrict_
             for (int jj = 0; jj < GEN_BLOCK; ++jj) {
                 float p[R], v[DI];
                 gen_load<R>(p, p_s + jj * R);
-#pragma unroll
-                for (int i = 0; i < DI; ++i) v[i] = lane + 32 * i < pitch ? v_s[jj * pitch + lane + 32 * i] : 0.f;
+                gen_values<T, DI>(v, v_s + jj * key_row, filled, lane);
 #pragma unroll
                 for (int r = 0; r < R; ++r)
 #pragma unroll
@@ -172,7 +276,7 @@ attention_generic_kernel(const T* __restrict__ qkv, int q_stride, T* __restrict_
             for (int r = 0; r < R; ++r)
 #pragma unroll
                 for (int i = 0; i < DI; ++i)
-                    if (lane + 32 * i < pitch) k_s[r * pitch + lane + 32 * i] = acc[r][i];
+                    if (gen_channel<T>(i, lane) < pitch) o_s[r * pitch + gen_channel<T>(i, lane)] = acc[r][i];
         }
         __syncthreads();
         // this round's blocks, merged in ascending order
@@ -183,8 +287,8 @@ attention_generic_kernel(const T* __restrict__ qkv, int q_stride, T* __restrict_
             const int r = e / pitch;
             float m = ml_in[2 * r], l = ml_in[2 * r + 1], o = tot[e];
             for (int w = 0; w < live; ++w) {
-                const float* other = base + (size_t)w * gen_warp_floats(R, head_dim);
-                const float* other_ml = other + 2 * GEN_BLOCK * pitch + GEN_BLOCK * R;
+                const float* other = base + (size_t)w * warp_floats;
+                const float* other_ml = other + GEN_BLOCK * key_row / 2 + GEN_BLOCK * R;
                 const float mw = other_ml[2 * r], lw = other_ml[2 * r + 1];
                 if (mw == -INFINITY && lw == 0.f) continue;          // no key of the block is seen (or only scores of -inf); a sum of NaN goes on
                 const float m_new = fmaxf(m, mw);
@@ -220,15 +324,16 @@ static int launch_generic(const void* qkv, int q_stride, void* out, const int* p
     NIB_REQUIRE(blocks <= 0x7fffffffLL, "attention: too many tokens for one launch");
     // a warp per block of keys, as many as eight; of a prompt's many tokens each gets fewer: their CTAs fill the GPU anyway
     int warps = max(1, min(blocks >= 8 * 148 ? 4 : GEN_MAX_WARPS, ceil_div(max_keys, GEN_BLOCK)));
-    const size_t cta = sizeof(float) * gen_cta_floats(R, head_dim), per_warp = sizeof(float) * gen_warp_floats(R, head_dim);
+    const uintptr_t bytes = (uintptr_t)k_pages | (uintptr_t)v_pages | (uintptr_t)(head_dim * sizeof(T));      // what rows begin at and are long
+    const int unit = bytes % 16 == 0 ? 16 : bytes % 8 == 0 ? 8 : bytes % 4 == 0 ? 4 : 0;
+    const size_t cta = gen_cta_bytes<T>(R, head_dim), per_warp = gen_warp_bytes<T>(R, head_dim, unit);
     while (warps > 1 && cta + warps * per_warp > GEN_SMEM) --warps;
     const size_t smem = cta + warps * per_warp;
-    const int wide = head_dim % 4 == 0 && ((uintptr_t)k_pages | (uintptr_t)v_pages) % 16 == 0;
     // the most that any call takes: the attribute is the kernel's, and a call's own size would lower it under another thread's launch
     if (smem > 48 * 1024) NIB_CUDA(cudaFuncSetAttribute(attention_generic_kernel<T, R, DI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEN_SMEM));
     NIB_CUDA(launch_pdl(attention_generic_kernel<T, R, DI>, dim3((unsigned)blocks), dim3(32 * warps), smem, stream, (const T*)qkv, q_stride,
                         (T*)out, positions, req_index, block_table, bt_stride, page_size, (const T*)k_pages, (const T*)v_pages, num_pages,
-                        heads, kv_heads, head_dim, scale, window, wide));
+                        heads, kv_heads, head_dim, scale, window, unit));
     NIB_LAUNCH_CHECK();
     return 0;
 }

@@ -824,9 +824,9 @@ def test_f32_gated_product_edges(K, m, inter, k):
 @pytest.mark.parametrize("heads,kv_heads,hd,page,window", [
     (14, 2, 64, 16, 0), (9, 1, 40, 8, 0), (3, 3, 5, 4, 0), (4, 2, 256, 16, 0), (14, 2, 64, 16, 129), (8, 2, 100, 16, 33), (16, 1, 64, 8, 700)])
 def test_general_attention_segments(K, dtype, heads, kv_heads, hd, page, window):
-    """The general kernel at the edges of its blocks (32 keys), segments (128) and rounds (up to eight segments), of groups
-    larger than a CTA's eight heads, and with windows that begin inside a segment; a token alone gets the same bits as in a
-    batch of others (where another number of warps shares its keys)."""
+    """The general kernel at the edges of its blocks (32 keys) and rounds (up to eight blocks, a warp each), of groups larger than a
+    CTA's eight heads, and with windows that begin inside a block; a token alone gets the same bits as in a batch of others (where
+    another number of warps shares its keys)."""
     K = K.with_options(force_general_attention=True)
     before = [0, 31, 126, 127, 128, 255, 1023, 1100, 2047, 0]
     q_lens = [1] * 9 + [40]
@@ -1022,6 +1022,31 @@ def test_launches_of_unlike_sizes_from_several_threads(K, which):
     for t in threads:
         t.join()
     assert not failed, failed
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("heads,kv_heads,hd", [(4, 4, 1), (6, 2, 6), (8, 8, 33), (4, 1, 34), (3, 3, 36), (8, 8, 72), (2, 2, 130), (2, 1, 255)])
+def test_general_attention_rows_of_any_width_and_place(K, dtype, heads, kv_heads, hd):
+    """Rows made of 16, 8, 4 and 2 bytes, pages that begin at any element, what lies around them being NaN."""
+    K = K.with_options(force_general_attention=True)
+    page, before, q_lens = 8, [0, 31, 70, 500], [3, 1, 2, 1]
+    ctx, bt = make_paged_batch(q_lens, before, page, 90, "cuda", seed=11)
+    kp, vp = _fill_cache(ctx, bt, page, 90, kv_heads, hd, dtype, 110)
+    m = sum(q_lens)
+    qkv = rnd((m, (heads + 2 * kv_heads) * hd), dtype, 111)
+    out, ref, first = (torch.empty(m, heads * hd, dtype=dtype, device="cuda") for _ in range(3))
+    REF.attention(qkv, ref, heads, kv_heads, hd, 1.0 / math.sqrt(hd), 40, ctx, bt, page, kp, vp)
+    for off in (0, 1, 2, 4, 8):
+        moved = []
+        for t in (kp, vp):
+            room = torch.full((t.numel() + 16,), math.nan, dtype=dtype, device="cuda")
+            moved.append(room[off:off + t.numel()].view(t.shape))
+            moved[-1].copy_(t)
+        K.attention(qkv, out, heads, kv_heads, hd, 1.0 / math.sqrt(hd), 40, ctx, bt, page, *moved)
+        assert_close(out, ref, dtype, f"offset {off}")
+        if off == 0:
+            first.copy_(out)
+        assert torch.equal(out, first)
 
 
 @pytest.mark.parametrize("vocab", [3, 2048, 2049, 32000, 151936, 151937, 368640, 368641, 389121, 700000])
