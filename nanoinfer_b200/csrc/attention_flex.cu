@@ -85,25 +85,32 @@ __device__ __forceinline__ void prepare_unit(const float* __restrict__ qkv, int 
     for (int c = lane; c < d; c += 32) x_s[c] = gain != nullptr ? src[c] * norm * gain[c] : src[c];
     __syncwarp();
     // Pairs in place, a lane a pair: the first element is turned with minus, the second with plus; pairs are (i, i + rot/2) or
-    // (2i, 2i + 1). One loop that is not unrolled, with one sine and one cosine in the program: eight elements a lane, unrolled,
-    // were 32 of them, and a step of few tokens spent its time fetching instructions (3 tokens of 16 heads: 7.0 us, 3.5 now).
+    // (2i, 2i + 1). One loop that is not unrolled, with one sine and cosine in the program: eight elements a lane, unrolled,
+    // were 32 of them, and a step of few tokens spent its time fetching instructions (3 tokens of 16 heads: 7.0 us, 3.5 now). The
+    // squares for a norm after the rotation are summed on the way (3 tokens of 16 + 16 heads of 64: 2.95 us; 3.15 in a loop of its own).
     const int half = rot >> 1;
     const bool interleaved = (flags & FXP_INTERLEAVED) != 0;
+    float ss = 0.f;
 #pragma unroll 1
     for (int i = lane; i < half; i += 32) {
         const int c0 = interleaved ? 2 * i : i, c1 = interleaved ? c0 + 1 : i + half;
         const float a = (float)pos * freq[i];
-        const float cs = cosf(a), sn = sinf(a), x0 = x_s[c0], x1 = x_s[c1];
-        x_s[c0] = x0 * cs - x1 * sn;
-        x_s[c1] = x1 * cs + x0 * sn;
+        float cs, sn;
+        sincosf(a, &sn, &cs);
+        const float x0 = x_s[c0], x1 = x_s[c1];
+        const float y0 = x0 * cs - x1 * sn, y1 = x1 * cs + x0 * sn;
+        x_s[c0] = y0;
+        x_s[c1] = y1;
+        ss = fmaf(y0, y0, fmaf(y1, y1, ss));
     }
     __syncwarp();
     float after = 1.0f;
     if (flags & FXP_UNIT_NORM_AFTER) {
-        float ss = 0.f;
-        for (int c = lane; c < d; c += 32) ss = fmaf(x_s[c], x_s[c], ss);
+#pragma unroll 1
+        for (int c = rot + lane; c < d; c += 32) ss = fmaf(x_s[c], x_s[c], ss);
         after = 1.0f / sqrtf(warp_sum(ss) / (float)d + eps);
     }
+#pragma unroll 1
     for (int c = lane; c < d; c += 32) Elem<T>::store(dst + c, x_s[c] * after);
     __syncwarp();       // x_s is the warp's own and may be filled again for its next unit
 }
