@@ -131,6 +131,7 @@ template <int HD> struct Cfg {
     static constexpr int COL_S = 0, COL_P = P_OWN ? KEYS : 0, COL_O = P_OWN ? KEYS + KEYS / 2 : KEYS;
     static constexpr int TMEM_COLS = 256;
     static_assert(COL_O + HD <= TMEM_COLS, "two CTAs share an SM's tensor memory");
+    static_assert(prompt_fits_tmem(SMEM, TMEM_COLS), "CTAs that share an SM must not wait for one another's tensor memory");
 };
 
 // The running maximum of a row is replaced by a larger one only when it grew by more than this (in log2 units):
@@ -162,7 +163,11 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     unsigned long long* k_empty = bars + 3;
     unsigned long long* v_full = bars + 5;
     unsigned long long* v_empty = bars + 7;
-    // phase j of each of these belongs to block j; no phase can complete before the one before it was seen
+    // Phase j of each of these belongs to block j. A wait for a phase is one for its parity, so it must not come while the phase two
+    // before it is still open. Every phase is seen by its waiter before the next can complete, except those of o_done where the
+    // probabilities lie on the scores: it is waited for only when a row is rescaled and at the end. There the scores of block j are
+    // multiplied and told behind P.V of block j - 1 by the same thread, and a softmax warp that waits for o_done has seen s_full(j):
+    // P.V of block j - 1 is done then, and o_done at most about to be told of it, never a phase behind that.
     unsigned long long* s_full = bars + 9;        // the scores are in tensor memory
     unsigned long long* s_empty = bars + 10;      // P_OWN: ... and in registers (an arrival per softmax warp)
     unsigned long long* p_full = bars + 11;       // [2] the probabilities of a half of the keys are in tensor memory (an arrival per softmax warp)

@@ -61,6 +61,7 @@ template <int TOK, bool DUAL, int HD = 0> struct Cfg {
     static constexpr int ACC_COLS = (DUAL ? 2 : 1) * TOK;                 // columns of one accumulator buffer
     static constexpr int TMEM_COLS = tmem_cols(2 * ACC_COLS);             // two buffers
     static_assert(2 * ACC_COLS <= 512, "two accumulator buffers must fit the 512 TMEM columns");
+    static_assert(product_fits_tmem(SMEM, TMEM_COLS), "CTAs that share an SM must not wait for one another's tensor memory");
 };
 
 __device__ __forceinline__ void red_add_v4(float* p, float a, float b, float c, float d) {
@@ -568,6 +569,7 @@ template <int NT> struct PairCfg {
     static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 256;
     static constexpr int TMEM_COLS = tmem_cols(2 * NT);                   // two accumulator buffers
     static_assert(2 * NT <= 512, "two accumulator buffers must fit the 512 TMEM columns");
+    static_assert(product_fits_tmem(SMEM, TMEM_COLS), "CTAs that share an SM must not wait for one another's tensor memory");
 };
 
 // map_m: activations [tokens, K], box 64 x 128 rows; map_n: weights [rows, K], box 64 x NT/2 rows.

@@ -49,6 +49,7 @@ template <int TOK, bool DUAL> struct Cfg {
     static constexpr int ACC_COLS = (DUAL ? 2 : 1) * TOK;                 // columns of one accumulator buffer
     static constexpr int TMEM_COLS = tmem_cols(2 * ACC_COLS);             // two buffers
     static_assert(2 * ACC_COLS <= 512, "two accumulator buffers must fit the 512 TMEM columns");
+    static_assert(product_fits_tmem(SMEM, TMEM_COLS), "CTAs that share an SM must not wait for one another's tensor memory");
 };
 
 __device__ __forceinline__ void red_add_v4(float* p, float a, float b, float c, float d) {

@@ -22,6 +22,18 @@ __device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, 
 // a wait of the whole warp, with one answer
 __device__ __forceinline__ bool warp_wait(unsigned long long* bar, unsigned parity) { return __all_sync(0xffffffffu, nibp::mbar_wait(bar, parity)); }
 
+// ---- who may share an SM. With dependent launches a CTA of the next kernel can be resident beside CTAs of this one, and an allocation
+// of tensor memory waits until columns are free: a CTA that held columns which a CTA of an earlier kernel still has to allocate
+// would wait for that kernel's end for good. So CTAs that fit an SM's shared memory together fit its 512 columns together: two of the
+// prompt attention's, or one of any product's and as many of the prompt attention's as fit beside it, and no two products'.
+constexpr int SM_SHARED = 228 * 1024, CTA_RESERVED = 1024, SM_TMEM_COLS = 512;       // bytes, bytes, columns
+constexpr int PROMPT_SMEM = 5 * 16384 + 1280, PROMPT_COLS = 256;                      // the prompt attention's smallest CTA
+constexpr bool product_fits_tmem(int smem, int cols) {
+    return 2 * (smem + CTA_RESERVED) > SM_SHARED &&
+           cols + (SM_SHARED - smem - CTA_RESERVED) / (PROMPT_SMEM + CTA_RESERVED) * PROMPT_COLS <= SM_TMEM_COLS;
+}
+constexpr bool prompt_fits_tmem(int smem, int cols) { return smem >= PROMPT_SMEM && cols == PROMPT_COLS && 3 * (PROMPT_SMEM + CTA_RESERVED) > SM_SHARED; }
+
 // ---- tensor memory: allocated and freed by one whole warp; the address arrives in shared memory
 __device__ __forceinline__ void tmem_alloc(unsigned* dst_smem, unsigned cols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(dst_smem)), "r"(cols) : "memory");
