@@ -5,15 +5,15 @@
 // result does not depend on how many other rows the call has (the reference guarantees the same:
 // cpp/src/cuda/cuda_gemm.cu:37-45). Tiling after cpp/src/cuda/cuda_gemm.cu:80-150 in spirit only.
 //
-// Epilogues: STORE (T out = acc + bias), ADD (float out += acc + bias: the residual sum),
+// Epilogues: STORE (bfloat16 out = acc + bias), ADD (float out += acc + bias: the residual sum),
 // F32 (float out = acc + bias: logits), SWIGLU (two accumulators, W rows n and n + N:
-// T out = silu(gate) * up, silu(g) = g / (1 + exp(-g)), cpp/src/ops.cpp:86-93), GLU (the same with limits and constants),
+// bfloat16 out = silu(gate) * up, silu(g) = g / (1 + exp(-g)), cpp/src/ops.cpp:86-93), GLU (the same with limits and constants),
 // GEGLU (gelu(gate) * up).
 #include "common.cuh"
 
-template <typename T, int EPI>
+template <int EPI>
 __global__ void __launch_bounds__(256)
-gemm_simt_kernel(const T* __restrict__ A, const T* __restrict__ W, const float* __restrict__ bias,
+gemm_simt_kernel(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ W, const float* __restrict__ bias,
                  void* __restrict__ out, int M, int N, int K, int lda, int ldo, const NibGlu glu) {
     constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
     constexpr bool DUAL = epi_dual(EPI);
@@ -47,10 +47,10 @@ gemm_simt_kernel(const T* __restrict__ A, const T* __restrict__ W, const float* 
             const int gk = k0 + kk;
             float a = 0.f, w = 0.f, u = 0.f;
             if (gk < K) {
-                if (m0 + r < M) a = Elem<T>::load(A + (size_t)(m0 + r) * lda + gk);
+                if (m0 + r < M) a = Elem<__nv_bfloat16>::load(A + (size_t)(m0 + r) * lda + gk);
                 if (n0 + r < N) {
-                    w = Elem<T>::load(W + (size_t)(n0 + r) * K + gk);
-                    if (DUAL) u = Elem<T>::load(W + (size_t)(N + n0 + r) * K + gk);
+                    w = Elem<__nv_bfloat16>::load(W + (size_t)(n0 + r) * K + gk);
+                    if (DUAL) u = Elem<__nv_bfloat16>::load(W + (size_t)(N + n0 + r) * K + gk);
                 }
             }
             As[kk][r] = a;
@@ -93,31 +93,30 @@ gemm_simt_kernel(const T* __restrict__ A, const T* __restrict__ W, const float* 
             float v = acc[i][j] + (bias ? bias[n] : 0.f);
             const size_t o = (size_t)m * ldo + n;
             if (EPI == EPI_STORE) {
-                Elem<T>::store((T*)out + o, v);
+                Elem<__nv_bfloat16>::store((__nv_bfloat16*)out + o, v);
             } else if (EPI == EPI_ADD) {
                 ((float*)out)[o] += v;
             } else if (EPI == EPI_F32) {
                 ((float*)out)[o] = v;
             } else {
                 const float g = v, u = acc2[DUAL ? i : 0][DUAL ? j : 0];
-                Elem<T>::store((T*)out + o, EPI == EPI_GLU ? nib_glu_exact(glu, g, u) : EPI == EPI_GEGLU ? nib_geglu_exact(g, u) : g / (1.0f + expf(-g)) * u);
+                Elem<__nv_bfloat16>::store((__nv_bfloat16*)out + o, EPI == EPI_GLU ? nib_glu_exact(glu, g, u) : EPI == EPI_GEGLU ? nib_geglu_exact(g, u) : g / (1.0f + expf(-g)) * u);
             }
         }
     }
 }
 
-template <typename T>
 static int launch_simt(const void* A, const void* W, const float* bias, void* out, int M, int N, int K,
                        int lda, int ldo, int epi, const NibGlu& glu, cudaStream_t stream) {
     dim3 grid(ceil_div(N, 64), ceil_div(M, 64));
     dim3 block(256);
     switch (epi) {
-        case EPI_STORE: gemm_simt_kernel<T, EPI_STORE><<<grid, block, 0, stream>>>((const T*)A, (const T*)W, bias, out, M, N, K, lda, ldo, glu); break;
-        case EPI_ADD: gemm_simt_kernel<T, EPI_ADD><<<grid, block, 0, stream>>>((const T*)A, (const T*)W, bias, out, M, N, K, lda, ldo, glu); break;
-        case EPI_F32: gemm_simt_kernel<T, EPI_F32><<<grid, block, 0, stream>>>((const T*)A, (const T*)W, bias, out, M, N, K, lda, ldo, glu); break;
-        case EPI_SWIGLU: gemm_simt_kernel<T, EPI_SWIGLU><<<grid, block, 0, stream>>>((const T*)A, (const T*)W, bias, out, M, N, K, lda, ldo, glu); break;
-        case EPI_GLU: gemm_simt_kernel<T, EPI_GLU><<<grid, block, 0, stream>>>((const T*)A, (const T*)W, bias, out, M, N, K, lda, ldo, glu); break;
-        case EPI_GEGLU: gemm_simt_kernel<T, EPI_GEGLU><<<grid, block, 0, stream>>>((const T*)A, (const T*)W, bias, out, M, N, K, lda, ldo, glu); break;
+        case EPI_STORE: gemm_simt_kernel<EPI_STORE><<<grid, block, 0, stream>>>((const __nv_bfloat16*)A, (const __nv_bfloat16*)W, bias, out, M, N, K, lda, ldo, glu); break;
+        case EPI_ADD: gemm_simt_kernel<EPI_ADD><<<grid, block, 0, stream>>>((const __nv_bfloat16*)A, (const __nv_bfloat16*)W, bias, out, M, N, K, lda, ldo, glu); break;
+        case EPI_F32: gemm_simt_kernel<EPI_F32><<<grid, block, 0, stream>>>((const __nv_bfloat16*)A, (const __nv_bfloat16*)W, bias, out, M, N, K, lda, ldo, glu); break;
+        case EPI_SWIGLU: gemm_simt_kernel<EPI_SWIGLU><<<grid, block, 0, stream>>>((const __nv_bfloat16*)A, (const __nv_bfloat16*)W, bias, out, M, N, K, lda, ldo, glu); break;
+        case EPI_GLU: gemm_simt_kernel<EPI_GLU><<<grid, block, 0, stream>>>((const __nv_bfloat16*)A, (const __nv_bfloat16*)W, bias, out, M, N, K, lda, ldo, glu); break;
+        case EPI_GEGLU: gemm_simt_kernel<EPI_GEGLU><<<grid, block, 0, stream>>>((const __nv_bfloat16*)A, (const __nv_bfloat16*)W, bias, out, M, N, K, lda, ldo, glu); break;
         default: nib_set_error("gemm: unknown epilogue %d", epi); return 1;
     }
     NIB_LAUNCH_CHECK();
@@ -134,7 +133,7 @@ NIB_API int nib_gemm_simt(const void* A, const void* W, const float* bias, void*
     const NibGlu constants = glu != nullptr ? *glu : NibGlu{};
     if (M == 0) return 0;
     NIB_REQUIRE(ceil_div(M, 64) <= 65535, "gemm: M=%d is too large for one launch", M);
-    return launch_simt<__nv_bfloat16>(A, W, bias, out, M, N, K, lda, ldo, epi, constants, stream);
+    return launch_simt(A, W, bias, out, M, N, K, lda, ldo, epi, constants, stream);
 }
 
 // ---------------------------------------------------------------------------------- block-diagonal product, few tokens
