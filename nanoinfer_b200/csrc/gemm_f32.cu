@@ -374,7 +374,11 @@ template <int EPI>
 int launch_f32(const Args& a) {
     constexpr bool DUAL = epi_dual(EPI);
     const int chunks = ceil_div(a.K, CHUNK);
-    if (a.M <= ROWS_MAX_TOKENS) {
+    // Not where a chunk is mostly the zeros that fill it up, which a thread of the rows kernel walks like the rest and the tile kernel
+    // leaves out: 20,000 rows of 64 k, 16 tokens, 25 us by rows and 10.9 by tiles (a thread per output: 13.9), 4 tokens 12.6 and 10.6; 24
+    // rows of 16 k, one token, 3.7 and 2.5. Of 128 k: 896 rows, 16 tokens, 9.1 and 6.9, 8 tokens 5.6 and 6.6.
+    const int short_k = a.M > 8 ? 128 : a.M > 2 ? 64 : 32;
+    if (a.M <= ROWS_MAX_TOKENS && a.K > short_k) {
         int ranks = min(8, ceil_div(chunks, ROWS_CHUNKS));
         const int cpc = ceil_div(chunks, ranks);
         ranks = ceil_div(chunks, cpc);          // every CTA of a cluster has a chunk
