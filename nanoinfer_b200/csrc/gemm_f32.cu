@@ -391,9 +391,12 @@ int launch_f32(const Args& a) {
     }
     const int tiles = ceil_div(a.N, BN) * ceil_div(a.M, BM);
     // CTAs that share the chunks of a tile: as many as keep all CTAs on the GPU at once, two an SM; with more tiles than SMs none,
-    // unless their last turn would leave most SMs idle (152 tiles on 148 SMs, K = 896: 105 us with a CTA a tile, 91 with a CTA a chunk)
+    // unless their last turn would leave most SMs idle and there are four chunks to share. us by a CTA a tile and by four, 64 tokens:
+    // 152 tiles of 896 k, 65 and 57, gated 104 and 86; of 4,864, 340 and 245, gated 545 and 450; 184 tiles of 2,048, 144 and 119; but 152 of
+    // 300 k 25 and (by two) 39, of 520 (by three) 40 and 43, 190 tiles of 1,536 108 and 106, gated 176 and 173, 196 gated 176 and 184. (By
+    // eight: 152 gated tiles of 4,864 609, 184 721.)
     int ranks = 2 * 148 / tiles;
-    if (tiles > 148 && ceil_div(tiles, 148) * 148 > tiles + tiles / 2) ranks = 8;
+    if (tiles > 148 && 8 * tiles < 5 * 2 * 148 && chunks >= 4) ranks = 4;
     ranks = max(1, min(min(8, chunks), ranks));
     const int cpc = ceil_div(chunks, ranks);
     ranks = ceil_div(chunks, cpc);

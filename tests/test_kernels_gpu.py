@@ -784,7 +784,7 @@ def test_qkv_projection_with_rotation_and_cache_write(K, heads, kv_heads, hd, ro
 
 
 @pytest.mark.parametrize("m", [1, 2, 3, 5, 8, 9, 16, 17, 64, 65, 300])
-@pytest.mark.parametrize("n,k", [(8, 4), (9, 255), (64, 256), (65, 257), (100, 1280), (40, 1284), (33, 2600), (4736, 256), (24, 4864), (16, 18944), (70, 32), (20, 33), (100, 64), (9, 65), (200, 128), (33, 129)])
+@pytest.mark.parametrize("n,k", [(8, 4), (9, 255), (64, 256), (65, 257), (100, 1280), (40, 1284), (33, 2600), (4736, 256), (24, 4864), (16, 18944), (70, 32), (20, 33), (100, 64), (9, 65), (200, 128), (33, 129), (9700, 770), (11776, 1000), (11840, 770)])
 def test_f32_product_edges(K, m, n, k):
     """The 32-bit products at the edges of their chunks (256 of k), tiles (8, 16 and 64 rows), clusters and shared memory, also
     with operands that are not 16-byte aligned: values, what lies behind them, and rows that are the same bits whatever the
