@@ -207,8 +207,9 @@ class PortionGraphs:
 
     A long prompt is cut into portions of the scheduler's token budget, so the same shape (the entries' token
     counts, the number of wanted rows, the block tables' widths rounded up to a power of two) comes again and
-    again. Such a step is some two hundred launches whose host side costs about as much as a tenth of the
-    device's work; captured once, the third time its shape is seen, it is one launch. Everything a kernel
+    again. Such a step is some two hundred launches, whose host side is hidden behind the device's work for
+    thousands of tokens and several times as long as it for a few dozen; captured once, the third time its shape
+    is seen, it is one launch. Everything a kernel
     reads of the step (ids, positions, lengths, wanted rows, block tables) lies in a device buffer of fixed
     address that one copy refreshes; the launch geometry depends on the shape alone (for the decoded tokens of
     a mixed step: on the power of two that bounds their contexts, as in DecodeGraphs). A shape seen once is
