@@ -1049,7 +1049,7 @@ def test_general_attention_rows_of_any_width_and_place(K, dtype, heads, kv_heads
         assert torch.equal(out, first)
 
 
-@pytest.mark.parametrize("vocab", [3, 2048, 2049, 32000, 151936, 151937, 368640, 368641, 389121, 700000])
+@pytest.mark.parametrize("vocab", [3, 2048, 2049, 32000, 151936, 151937, 368640, 368641, 389120, 389121, 700000])
 def test_sampling_slices(K, vocab):
     """Slices of a row that are kept in shared memory and those that do not fit (of five rows: more than 368,640 logits), rows that do not start
     on 16 bytes, slices that are empty: the drawn token is the plain pipeline's wherever the number drawn is not within rounding
