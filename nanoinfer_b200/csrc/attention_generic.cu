@@ -19,7 +19,9 @@
 // element by element / this: bfloat16, 8 heads of 72, a prompt of 1,024 tokens, 757 / 3,896 / 300; 64 tokens of 500 keys,
 // 218 / 299 / 25; 16 tokens, 8 and 2 heads of 100, 14.6 / 44.8 / 8.1; 32-bit, 8 heads of 72, 1,024 tokens, 873 / 1,039 / 620; one token of
 // 777 keys, 14 and 2 heads of 64, 323 / 22.3 / 19.9. Rows of an odd number of elements go as 32-bit words: 8 heads of 33 and 16 tokens,
-// 9.1 / 26 / 8.2, but 8 heads of 129 and 1,024 tokens, bfloat16, 1,134 / - / 1,802 (one token of 777 keys, 474 / - / 68).
+// 9.1 / 26 / 8.2. With an odd width and one query head a kv head the copies' instructions are what a long prompt waits for (a
+// fourth of the bytes each): 8 heads of 129 and 1,024 tokens, bfloat16, 1,134 / - / 1,725 (one token of 777 keys, 458 / - / 65; 64 of 500
+// keys, 348 / - / 184; eight heads on two kv heads, 1,142 / - / 614), 32-bit 1,052 / - / 3,587 (458 / - / 85; 345 / - / 212).
 //
 // Formula: cpp/src/ops.cpp:206-270 (score = dot * scale, scale after the dot; max-subtracted exp;
 // sum of p_j v_j / sum p_j); kv head = head / (heads / kv_heads): cpp/src/paged.cpp:171. Warp-level
@@ -87,7 +89,8 @@ __device__ __forceinline__ void gen_send_units(unsigned char* dst, int pitch, co
 }
 // Rows of bfloat16 that begin at any element (an odd width, say): the 32-bit words that a row lies in, its first element in the upper
 // half of the first one if the row begins in the middle of a word (the lower half is the row's before it; no word is read that holds
-// nothing of the row). gen_align_rows() moves such a row down by an element.
+// nothing of the row). gen_align_rows() moves such a row down by an element. A lane reads and writes its own words only and gets the upper half
+// of a word from the lane above.
 __device__ __forceinline__ void gen_send_words(unsigned char* dst, int pitch, const __nv_bfloat16* pages, long long row, int d, int lane) {
     const int words = max(gen_filled<__nv_bfloat16>(d), d + 2) / 2, step_r = 32 / words, step_u = 32 - step_r * words;
     const unsigned to = (unsigned)__cvta_generic_to_shared(dst);
@@ -110,16 +113,20 @@ __device__ __forceinline__ void gen_send_words(unsigned char* dst, int pitch, co
 __device__ __forceinline__ void gen_align_rows(unsigned char* dst, int pitch, const __nv_bfloat16* pages, long long row, int d, int lane) {
     const int words = max(gen_filled<__nv_bfloat16>(d), d + 2) / 2;
     unsigned odd = __ballot_sync(0xffffffffu, row >= 0 && (reinterpret_cast<uintptr_t>(pages + max(row, 0ll) * d) & 2) != 0);
+    constexpr int TURNS = (GEN_MAX_D + 2 + 63) / 64;        // of 32 words
     for (; odd != 0; odd &= odd - 1) {
         unsigned* w = reinterpret_cast<unsigned*>(dst + (__ffs(odd) - 1) * pitch);
-        for (int u0 = 0; u0 < words; u0 += 32) {
-            const int u = u0 + lane;
-            const unsigned low = u < words ? w[u] >> 16 : 0u, high = u + 1 < words ? w[u + 1] << 16 : 0u;
-            __syncwarp();
-            if (u < words) w[u] = low | high;
-            __syncwarp();
+        unsigned v[TURNS + 1];
+#pragma unroll
+        for (int i = 0; i <= TURNS; ++i) v[i] = lane + 32 * i < words ? w[lane + 32 * i] : 0u;
+#pragma unroll
+        for (int i = 0; i < TURNS; ++i) {
+            if (32 * i >= words) break;
+            const unsigned next = __shfl_sync(0xffffffffu, lane == 0 ? v[i + 1] : v[i], lane + 1);      // (lane 31's: lane 0's next word)
+            if (lane + 32 * i < words) w[lane + 32 * i] = v[i] >> 16 | next << 16;
         }
     }
+    __syncwarp();
 }
 // `unit`: the largest of 16, 8 and 4 bytes that the rows are made of; 0 where there is none.
 template <typename T>
