@@ -9,7 +9,7 @@ from __future__ import annotations
 from dataclasses import dataclass
 from typing import Optional
 
-_ROUTES = (None, "smallm", "smallm_fused", "tc", "tc_pair")
+_ROUTES = (None, "smallm", "smallm_fused", "tc", "tc_pair", "stream")
 
 
 @dataclass(frozen=True)
@@ -20,7 +20,7 @@ class KernelOptions:
     separate_combine: bool = True           # cp.async decode kernel: merge its splits in a second kernel (False: the CTA that finishes last merges)
     fixed_decode_splits: int = 0            # a fixed split count of the keys for the decode kernels (0 = chosen)
     force_simt_gemm: bool = False           # the CUDA-core product for bfloat16 too
-    gemm_route: Optional[str] = None        # "smallm" | "smallm_fused" | "tc" | "tc_pair" instead of the measured choice
+    gemm_route: Optional[str] = None        # "smallm" | "smallm_fused" | "tc" | "tc_pair" | "stream" instead of the measured choice
     tc_token_tile: int = 0                  # token tile of the tcgen05 product (0 = chosen; 16, 32, 64, 128, 256)
     tc_splits: int = 0                      # work items along K per tile of the tcgen05 products (0 = chosen, 1 = none)
     pair_n_tile: int = 0                    # feature tile of the two-SM product (0 = chosen; 128, 256)

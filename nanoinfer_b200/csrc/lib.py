@@ -133,7 +133,8 @@ class Kernels:
                      "nib_attention_prepare", "nib_attention_flex", "nib_attention_flex_mma", "nib_attention_flex_mma_supported",
                      "nib_rmsnorm_add", "nib_moe_route", "nib_moe_max_tiles", "nib_moe_group", "nib_moe_gemm_simt", "nib_moe_combine",
                      "nib_moe_tc_supported", "nib_moe_tc_error", "nib_moe_gather_rows", "nib_moe_gemm_tc", "nib_moe_step", "nib_moe_step_supported", "nib_moe_identity", "nib_stream_mix", "nib_grouped_state_scan", "nib_grouped_state_error", "nib_pdl_skip_next", "nib_memory_gates", "nib_layernorm",
-                     "nib_decay_state_scan", "nib_decay_state_chunks_supported"):
+                     "nib_decay_state_scan", "nib_decay_state_chunks_supported",
+                     "nib_gemm_stream", "nib_gemm_stream_supported", "nib_gemm_stream_error"):
             getattr(self._lib, name).restype = c_int
         self._lib.nib_grouped_state_scratch.restype = self._lib.nib_decay_state_scratch.restype = c_longlong
 
@@ -343,6 +344,40 @@ class Kernels:
         tiles = -(-rows // 256) * -(-m // 256)
         return tiles >= 48
 
+    def _use_stream(self, m: int, n: int, k: int, epi: int, has_norm: bool) -> int:
+        """Into how many CTAs' stretches of K the streamed product (weights copied into shared memory ahead of everything) cuts
+        this product of at most 16 tokens; 0: another kernel takes it. Measured as whole decode steps at the widths of the
+        0.5B, 1.5B and 7B models: gate/up behind its norm wins for every number of tokens up to 16 (us a step without / with: one token 565 /
+        498, 1,060 / 1,005, 585 / 560; 8 tokens 640 / 571, 1,176 / 1,106; 16 tokens of the 0.5B 814 / 699); up to 8 tokens of an input
+        that is normed already the small-M product is as good (5,632 x 2,048: 11.2 us and 11.6). The down projection wins for one
+        token while a CTA of eight that share K holds its weights whole (498 / 474; two tokens 507 / 503, 8 at 4,096 640 / 661; 1.5B, one
+        token 1,005 / 1,094)."""
+        o = self.options
+        if o.gemm_route not in (None, "stream") or o.tc_token_tile or o.tc_splits or o.smallm_ksplit or o.smallm_cross or m > 16 or k % 64:
+            return 0
+        if epi in _DUAL:
+            return 1 if has_norm or m > 8 or o.gemm_route == "stream" else 0
+        if epi != _EPI["add"]:
+            return 0
+        if o.gemm_route == "stream":
+            return 8 if k > 2048 else 1
+        return 8 if m == 1 and 2048 < k <= 8192 and 2 * n * k <= 9 << 20 else 0
+
+    def _streamed(self, splits, a, lazy, w, bias32, out, m, n, k, epi, glu) -> bool:
+        """The streamed product if it takes these operands. From 9 tokens on every CTA's reading the 32-bit stream for the norm costs more
+        than the norm's kernel (16 tokens at the 0.5B widths: 800 us a step instead of 699)."""
+        norm = lazy if m <= 8 and lazy is not None and lazy.fold.gain32.data_ptr() % 16 == 0 else None
+        if lazy is not None and norm is None:
+            a = self._resolve(lazy, False)
+        src = a if norm is None else norm.fold.x32
+        if self._lib.nib_gemm_stream_supported(_ptr(src), _ptr(w), c_int(m), c_int(k), c_int(src.stride(0)), c_int(2 if norm is None else 4), c_int(splits)) != 1:
+            return False
+        self._check(self._lib.nib_gemm_stream(
+            _ptr(src), _ptr(w), _ptr(bias32), _ptr(out), c_int(m), c_int(n), c_int(k), c_int(src.stride(0)), c_int(out.stride(0)), c_int(epi),
+            c_int(splits), _ptr(None if norm is None else norm.fold.gain32), c_float(0.0 if norm is None else norm.fold.eps), glu, self._stream()),
+            "linear (streamed)")
+        return True
+
     def _resolve(self, lazy, before_small_m: bool):
         """The norm's values for a product that cannot apply the norm itself. The norm kernel is told what follows it: a
         small-M product of up to 16 tokens has next to no set-up of its own and is let in late (see nib_rmsnorm); measured at batch 8:
@@ -367,6 +402,11 @@ class Kernels:
         if lazy is not None and not self._foldable(lazy):
             a, lazy = lazy.resolve(), None
         bf16 = a.dtype == torch.bfloat16 and not self.options.force_simt_gemm
+        splits = self._use_stream(m, n, k, epi, lazy is not None) if bf16 and (lazy is None or epi in _DUAL) else 0
+        if splits and self._streamed(splits, a, lazy, w, bias32, out, m, n, k, epi, glu):
+            return
+        if lazy is not None and lazy.resolved is not None:
+            a, lazy = lazy.resolved, None
         if bf16 and self.options.tc_token_tile == 0:
             kernel, fuse = self._route(m, w.shape[0], k, epi, lazy is not None)
             if lazy is not None and not fuse:
@@ -618,6 +658,7 @@ class Kernels:
         raise_device_errors([
             ("tensor-core GEMM (gemm_tcgen05.cu)", self.gemm_tc_error(), _GEMM_TC_ROLES),
             ("tcgen05 prefill attention (attention_tcgen05.cu)", self.attention_tc_error(), _ATTN_TC_ROLES),
+            ("streamed GEMM (gemm_stream.cu)", self._lib.nib_gemm_stream_error(), _GEMM_STREAM_ROLES),
             ("TMA decode attention (attention_decode_tma.cu)", self.attention_decode_tma_error(), _DECODE_TMA_ROLES),
             ("routed experts on the tensor cores (moe_tcgen05.cu)", self._lib.nib_moe_tc_error(), _GEMM_TC_ROLES),
             ("walk over matrix states (grouped_state.cu)", self._lib.nib_grouped_state_error(), {1: "walking warp: a group never arrived", 2: "sending warp: a buffer was never freed"}),
@@ -1644,6 +1685,7 @@ _GEMM_TC_ROLES = {1: "copy warp: a stage was never freed", 2: "MMA warp: a stage
                   3: "epilogue: the accumulator never arrived", 4: "MMA warp: the accumulator buffer was never drained",
                   5: "pair kernel, copy warp: a stage was never freed", 6: "pair kernel, MMA warp: the accumulator buffer was never drained",
                   7: "pair kernel, MMA warp: a stage was never filled", 8: "pair kernel, epilogue: the accumulator never arrived"}
+_GEMM_STREAM_ROLES = {1: "consumer warps: a stage never arrived", 2: "copy warp: a stage was never freed"}
 _ATTN_TC_ROLES = {1: "copy warp: a key/value stage was never freed", 2: "MMA warp: the queries never arrived",
                   3: "MMA warp: keys, values or probabilities never arrived", 4: "softmax warps: scores or outputs never arrived"}
 _DECODE_TMA_ROLES = {1: "consumer warps: a page tile never arrived", 2: "copy warp: a stage was never freed"}
