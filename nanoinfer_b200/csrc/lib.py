@@ -5,6 +5,7 @@ library cannot be built or loaded, or the device is not a CUDA device, they rais
 from __future__ import annotations
 
 import ctypes
+import struct
 from contextlib import nullcontext
 from ctypes import c_float, c_int, c_longlong, c_void_p
 from types import SimpleNamespace
@@ -134,7 +135,7 @@ class Kernels:
                      "nib_rmsnorm_add", "nib_moe_route", "nib_moe_max_tiles", "nib_moe_group", "nib_moe_gemm_simt", "nib_moe_combine",
                      "nib_moe_tc_supported", "nib_moe_tc_error", "nib_moe_gather_rows", "nib_moe_gemm_tc", "nib_moe_step", "nib_moe_step_supported", "nib_moe_identity", "nib_stream_mix", "nib_grouped_state_scan", "nib_grouped_state_error", "nib_pdl_skip_next", "nib_memory_gates", "nib_layernorm",
                      "nib_decay_state_scan", "nib_decay_state_chunks_supported",
-                     "nib_gemm_stream", "nib_gemm_stream_supported", "nib_gemm_stream_error"):
+                     "nib_gemm_stream", "nib_gemm_stream_supported", "nib_gemm_stream_error", "nib_sample_rows"):
             getattr(self._lib, name).restype = c_int
         self._lib.nib_grouped_state_scratch.restype = self._lib.nib_decay_state_scratch.restype = c_longlong
 
@@ -1654,6 +1655,24 @@ class Kernels:
         rows, vocab = logits.shape
         self._check(self._lib.nib_sample(_ptr(logits), c_int(rows), c_int(vocab), _ptr(temperature), _ptr(top_k),
                                          _ptr(top_p), _ptr(uniform), _ptr(out), self._stream()), "sample")
+
+    sample_rows_most = 64       # rows whose parameters a launch takes by value
+
+    def sample_rows(self, logits, rows, out):
+        """The same for up to ``sample_rows_most`` rows of (temperature, top_k, top_p, first, seed, counter), numbers of the host
+        that the launch takes with it; a row's uniform number is made from its seed and counter, or is 0 (``first``). ``out`` (int32)
+        may be a page-locked tensor of the host's."""
+        _need(logits, torch.float32, "sample logits")
+        n, vocab = logits.shape
+        if out.dtype != torch.int32 or not out.is_contiguous() or out.numel() < n or not (out.is_cuda or out.is_pinned()):
+            raise KernelError("sample out: contiguous int32, on the device or page-locked")
+        if len(rows) != n or n > self.sample_rows_most:
+            raise KernelError(f"sample_rows: {len(rows)} rows of parameters for {n} rows of logits, at most {self.sample_rows_most}")
+        flat = []
+        for row in rows:
+            flat += row
+        self._check(self._lib.nib_sample_rows(_ptr(logits), c_int(n), c_int(vocab), struct.pack("=" + "fifiQQ" * n, *flat),
+                                              c_void_p(out.data_ptr()), self._stream()), "sample")
 
 
 # kernel ids of the timeline (common.cuh: NibTraceKernel)

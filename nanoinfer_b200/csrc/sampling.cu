@@ -292,13 +292,29 @@ struct Slice {
 // fast exponential (2 ulp) is plenty for a draw.
 __device__ __forceinline__ float weight(float d) { return __expf(d); }
 
+// What a row is sampled with, as the host passes it by value: up to this many rows need no copy to the device ahead of the launch. The
+// uniform number is made here: 24 bits of the splitmix64 finaliser of (seed, counter).
+struct NibSampleRow { float temperature; int top_k; float top_p; int first; unsigned long long seed, counter; };      // first: draw at 0
+constexpr int ROWS_BY_VALUE = 64;
+struct SampleRows { NibSampleRow row[ROWS_BY_VALUE]; };
+
+__device__ __forceinline__ float uniform_of(unsigned long long seed, unsigned long long counter) {
+    unsigned long long x = seed * 0x9E3779B97F4A7C15ull + (counter + 1ull) * 0xD1B54A32D192ED03ull;
+    x ^= x >> 30;
+    x *= 0xBF58476D1CE4E5B9ull;
+    x ^= x >> 27;
+    x *= 0x94D049BB133111EBull;
+    x ^= x >> 31;
+    return (float)(unsigned)(x >> 40) * (1.0f / 16777216.0f);
+}
+
 // temperature > 0 for every row given to this kernel. grid: CS CTAs (one cluster) per row. Dynamic shared memory: the
 // histograms' copies and, KEPT, the slice.
 template <bool KEPT, int NT>
 __global__ void __launch_bounds__(NT, NT == 512 ? 2 : 5)
 sample_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p, const float* __restrict__ uniform,
-              int* __restrict__ out) {
+              int* __restrict__ out, const __grid_constant__ SampleRows by_value) {
     using namespace nibp;
     extern __shared__ __align__(16) float dyn[];
     constexpr int HIST = COPIES<NT> * BINS;
@@ -316,11 +332,14 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
     __shared__ int tie_count[ST];
     __shared__ float lane_total[32];
     __shared__ int s_pick;
+    __shared__ unsigned s_count, x_count;           // elements that this CTA has gathered
+    __shared__ unsigned s_low, s_high;              // keys chosen among the gathered ones
 
     const int row = blockIdx.x / CS;
     const unsigned rank = cluster_rank();
     const float* l = logits + (size_t)row * vocab;
-    const float inv_t = 1.0f / temperature[row];
+    const bool given = temperature == nullptr;      // the rows' parameters come by value
+    const float inv_t = 1.0f / (given ? by_value.row[row].temperature : temperature[row]);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
     // a thread's chunk of the row (vocabulary order: rank, then thread), a multiple of 4 long so that chunks start on 16 bytes;
@@ -421,12 +440,48 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
         else
             cluster_sync();
     };
+    // The elements that `wanted` says yes to, of the whole row, as keys into every CTA's shared memory (in the histograms' place, in no
+    // order): few enough are left after the first pass of a select, and each then finds its own rank among them, without a pass and a
+    // barrier of the cluster for every further digit. A pass in the buffers' turn. Returns how many there are. (8 rows of 151,936, us
+    // without / with lists and the first pass by distance: top-p 0.9 at temperature 0.7 48.5 / 39.8, top-k 50 with top-p 0.95 48.9 / 34.0,
+    // top-k 40 27.2 / 23.5; with bins of an eighth instead of a sixteenth the first of them overflows the list: 57.4.)
+    constexpr int LIST = NT == 512 ? 1024 : 0;
+    static_assert(LIST <= 4 * 256 && 3 * LIST <= 4 * HIST, "a CTA's list lies in a buffer of pub, the cluster's and its masses where the histograms are");
+    unsigned* keys = copies;                                                                // [LIST], filled up with zeros to whole fours
+    unsigned long long* masses = reinterpret_cast<unsigned long long*>(copies + LIST);      // [LIST]
+    auto gather = [&](auto&& wanted) {
+        unsigned* mine = &pub[pass++ & 1][0][0];
+        if (tid == 0) s_count = 0u;
+        __syncthreads();
+        slice.each([&](float x) {
+            if (wanted(x, key_of(x))) {
+                const unsigned at = atomicAdd(&s_count, 1u);
+                if ((int)at < LIST) mine[at] = key_of(x);
+            }
+        });
+        __syncthreads();
+        if (tid == 0) x_count = s_count;
+        cluster_sync();
+        unsigned n[CS], before = 0u;
+#pragma unroll
+        for (unsigned r = 0; r < CS; ++r) n[r] = ld_peer_u32(peer_smem(&x_count, r));
+#pragma unroll
+        for (unsigned r = 0; r < CS; ++r) {
+            for (unsigned i = tid; i < n[r] && (int)(before + i) < LIST; i += NT) keys[before + i] = ld_peer_u32(peer_smem(mine + i, r));
+            before += n[r];
+        }
+        const int listed = min((int)before, LIST);
+        if (tid < ((4 - listed) & 3)) keys[listed + tid] = 0u;
+        __syncthreads();
+        return listed;
+    };
     static_assert(NT == 512 || NT == 256, "the first 256 threads sum the counts, the last 256 the masses");
     const unsigned decider = NT == 512 ? rank : 0u;
 
     // ---- top-k: key of the k-th largest scaled logit (0 keeps everything)
     unsigned kth_key = 0u;
-    const int k = top_k[row];
+    const int k = given ? by_value.row[row].top_k : top_k[row];
+    int survivors = vocab;      // elements whose key is at least kth_key
     if (k > 0 && k < vocab) {
         unsigned prefix = 0u, remaining = (unsigned)k;
         for (int shift = 24; shift >= 0; shift -= 8) {
@@ -467,6 +522,33 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
                        });
             prefix = ld_peer_u32(peer_smem(&dec_prefix, decider));
             remaining = ld_peer_u32(peer_smem(&dec_remaining, decider));
+            if constexpr (NT == 512) {
+                const unsigned inside = tot_hist[(prefix >> shift) & 255u];
+                if (shift == 0) {
+                    survivors = (int)((unsigned)k - remaining + inside);
+                } else if (inside <= LIST) {
+                    const int listed = gather([&](float, unsigned key) { return (key & (0xffffffffu << shift)) == prefix; });
+                    for (int i = tid; i < listed; i += NT) {
+                        const unsigned key = keys[i];
+                        unsigned above = 0u, same = 0u;
+#pragma unroll 4
+                        for (int j = 0; j < listed; j += 4) {
+                            const uint4 o = *reinterpret_cast<const uint4*>(keys + j);      // (the zeros behind the last one: neither, unless the key is 0, an element's last of all)
+                            above += (o.x > key) + (o.y > key) + (o.z > key) + (o.w > key);
+                            same += (o.x == key) + (o.y == key) + (o.z == key) + (o.w == key);
+                        }
+                        if (above < remaining && remaining <= above + same) {       // the key of that rank; equal ones all say so
+                            dec_prefix = key;
+                            dec_remaining = (unsigned)k - remaining + above + same;
+                        }
+                    }
+                    __syncthreads();
+                    prefix = dec_prefix;
+                    survivors = (int)dec_remaining;
+                    __syncthreads();
+                    break;
+                }
+            }
         }
         kth_key = prefix;
     }
@@ -486,64 +568,130 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
     // ---- top-p: smallest key whose "probability of strictly larger keys" is <= p
     unsigned p_key = kth_key;
     long long ties_kept = -1;  // -1: every element equal to p_key stays
-    const float tp = top_p[row];
+    const float tp = given ? by_value.row[row].top_p : top_p[row];
     if (tp < 1.0f) {
         const unsigned long long limit = (unsigned long long)((double)tp * (double)FIX_ONE);
         unsigned prefix = 0u;
         unsigned long long above0 = 0ull;
-        for (int shift = 24; shift >= 0; shift -= 8) {
-            const unsigned mask = shift == 24 ? 0u : (0xffffffffu << (shift + 8));
-            radix_pass(true,
-                       [&](float x) {
-                           const unsigned key = key_of(x);
-                           if (key >= kth_key && (key & mask) == prefix) {
-                               unsigned* at = copies + copy + ((key >> shift) & 255u);
-                               mass_add(at + HIST, HIST, (unsigned long long)(weight(x - mx) * fix_over_z));
-                               atomicAdd(at, 1u);
-                           }
-                       },
-                       [&]() {
-                           // the lowest non-empty bin whose "mass above" (the bins above it, and what earlier passes left
-                           // above) is still within the limit; the very first (largest) element always stays, so if even
-                           // the highest non-empty bin is past the limit, that one
-                           unsigned long long mine = 0ull;
-                           for (int i = 0; i < 8; ++i) mine += tot_mass[lane * 8 + i];
-                           unsigned long long above = mine;
+        const auto mass_of = [&](float x) { return (unsigned long long)(weight(x - mx) * fix_over_z); };
+        const auto choose = [&]() {
+            // the lowest non-empty bin whose "mass above" (the bins above it, and what earlier passes left
+            // above) is still within the limit; the very first (largest) element always stays, so if even
+            // the highest non-empty bin is past the limit, that one
+            unsigned long long mine = 0ull;
+            for (int i = 0; i < 8; ++i) mine += tot_mass[lane * 8 + i];
+            unsigned long long above = mine;
 #pragma unroll
-                           for (int o = 1; o < 32; o <<= 1) {
-                               const unsigned long long v = __shfl_down_sync(0xffffffffu, above, o);
-                               if (lane + o < 32) above += v;
-                           }
-                           above = above - mine + above0;               // mass above this lane's bins
-                           int low = -1, high = -1;
-                           unsigned long long low_above = 0ull, high_above = 0ull, run = above;
-                           for (int i = 7; i >= 0; --i) {
-                               const int b = lane * 8 + i;
-                               if (tot_hist[b] != 0u) {
-                                   if (high < 0) { high = b; high_above = run; }
-                                   if (run <= limit) { low = b; low_above = run; }
-                               }
-                               run += tot_mass[b];
-                           }
-                           const unsigned within = __ballot_sync(0xffffffffu, low >= 0), any = __ballot_sync(0xffffffffu, high >= 0);
-                           int chosen = 0;
-                           unsigned long long chosen_above = above0;
-                           if (within) {                                // the lowest lane with one holds the lowest such bin
-                               const int src = __ffs(within) - 1;
-                               chosen = __shfl_sync(0xffffffffu, low, src);
-                               chosen_above = __shfl_sync(0xffffffffu, low_above, src);
-                           } else if (any) {
-                               const int src = 31 - __clz(any);
-                               chosen = __shfl_sync(0xffffffffu, high, src);
-                               chosen_above = __shfl_sync(0xffffffffu, high_above, src);
-                           }
-                           if (lane == 0) {
-                               dec_prefix = prefix | ((unsigned)chosen << shift);
-                               dec_above = chosen_above;
-                           }
-                       });
-            prefix = ld_peer_u32(peer_smem(&dec_prefix, decider));
-            above0 = ld_peer_u64(peer_smem(&dec_above, decider));
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned long long v = __shfl_down_sync(0xffffffffu, above, o);
+                if (lane + o < 32) above += v;
+            }
+            above = above - mine + above0;               // mass above this lane's bins
+            int low = -1, high = -1;
+            unsigned long long low_above = 0ull, high_above = 0ull, run = above;
+            for (int i = 7; i >= 0; --i) {
+                const int b = lane * 8 + i;
+                if (tot_hist[b] != 0u) {
+                    if (high < 0) { high = b; high_above = run; }
+                    if (run <= limit) { low = b; low_above = run; }
+                }
+                run += tot_mass[b];
+            }
+            const unsigned within = __ballot_sync(0xffffffffu, low >= 0), any = __ballot_sync(0xffffffffu, high >= 0);
+            int chosen = 0;
+            unsigned long long chosen_above = above0;
+            if (within) {                                // the lowest lane with one holds the lowest such bin
+                const int src = __ffs(within) - 1;
+                chosen = __shfl_sync(0xffffffffu, low, src);
+                chosen_above = __shfl_sync(0xffffffffu, low_above, src);
+            } else if (any) {
+                const int src = 31 - __clz(any);
+                chosen = __shfl_sync(0xffffffffu, high, src);
+                chosen_above = __shfl_sync(0xffffffffu, high_above, src);
+            }
+            if (lane == 0) {
+                dec_prefix = (unsigned)chosen;
+                dec_above = chosen_above;
+            }
+        };
+        const auto count_mass = [&](float x, unsigned bin) {
+            unsigned* at = copies + copy + bin;
+            mass_add(at + HIST, HIST, mass_of(x));
+            atomicAdd(at, 1u);
+        };
+        // Among the keys of a list: the lowest whose mass above is within the limit (else the highest, as a pass would have it).
+        const auto choose_listed = [&](int listed) {
+            for (int i = tid; i < ((listed + 3) & ~3); i += NT) masses[i] = i < listed ? mass_of(float_of_key(keys[i])) : 0ull;
+            if (tid == 0) {
+                s_low = 0xffffffffu;
+                s_high = 0u;
+            }
+            __syncthreads();
+            unsigned long long above[LIST > 0 ? (LIST + NT - 1) / NT : 1];
+#pragma unroll
+            for (int t = 0; t < (LIST + NT - 1) / NT; ++t) {
+                const int i = tid + t * NT;
+                above[t] = above0;
+                if (i >= listed) continue;
+                const unsigned key = keys[i];
+#pragma unroll 2
+                for (int j = 0; j < listed; j += 4) {
+                    const uint4 o = *reinterpret_cast<const uint4*>(keys + j);
+                    const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(masses + j), b = *reinterpret_cast<const ulonglong2*>(masses + j + 2);
+                    above[t] += (o.x > key ? a.x : 0ull) + (o.y > key ? a.y : 0ull) + (o.z > key ? b.x : 0ull) + (o.w > key ? b.y : 0ull);
+                }
+                if (above[t] <= limit) atomicMin(&s_low, key);
+                atomicMax(&s_high, key);
+            }
+            __syncthreads();
+            // (0xffffffff is the key of a NaN only, and then every key's mass is nothing and the lowest is taken)
+            const unsigned key = s_low != 0xffffffffu ? s_low : s_high;
+#pragma unroll
+            for (int t = 0; t < (LIST + NT - 1) / NT; ++t)
+                if (tid + t * NT < listed && keys[tid + t * NT] == key) dec_above = above[t];
+            __syncthreads();
+            prefix = key;
+            above0 = dec_above;
+            __syncthreads();
+        };
+        if (NT == 512 && survivors <= LIST) {
+            choose_listed(gather([&](float, unsigned key) { return key >= kth_key; }));
+        } else {
+            // The first pass goes by the distance from the maximum, in sixteenths, which spreads a row over the bins (by the key's first eight
+            // bits, sign and exponent, almost all of it falls into a handful, where the adds queue: 20 of a nucleus row's 48 us); what
+            // it chooses is a stretch of keys like any other digit's.
+            const auto bin_of = [&](float x) { return 255u - (unsigned)min(255, (int)((mx - x) * 16.0f)); };
+            // (With 256 threads, whose rows have no lists, it would be one more pass: 64 rows 184 us instead of 178.)
+            unsigned bin = 0u;
+            bool found = false;
+            if constexpr (NT == 512) {
+                radix_pass(true, [&](float x) { if (key_of(x) >= kth_key) count_mass(x, bin_of(x)); }, choose);
+                bin = dec_prefix;
+                above0 = dec_above;
+                if (tot_hist[bin] <= LIST) {
+                    choose_listed(gather([&](float x, unsigned key) { return key >= kth_key && bin_of(x) == bin; }));
+                    found = true;
+                }
+            }
+            for (int shift = 24; shift >= 0 && !found; shift -= 8) {
+                const unsigned mask = shift == 24 ? 0u : (0xffffffffu << (shift + 8));
+                radix_pass(true,
+                           [&](float x) {
+                               const unsigned key = key_of(x);
+                               if (key >= kth_key && (key & mask) == prefix && (NT != 512 || bin_of(x) == bin)) count_mass(x, (key >> shift) & 255u);
+                           },
+                           choose);
+                const unsigned digit = ld_peer_u32(peer_smem(&dec_prefix, decider));
+                prefix |= digit << shift;
+                above0 = ld_peer_u64(peer_smem(&dec_above, decider));
+                if constexpr (NT == 512) {
+                    if (shift > 0 && tot_hist[digit] <= LIST) {
+                        const unsigned low = 0xffffffffu << shift, want = prefix;
+                        choose_listed(gather([&](float x, unsigned key) { return key >= kth_key && (key & low) == want && bin_of(x) == bin; }));
+                        found = true;
+                    }
+                }
+            }
         }
         p_key = prefix;
         if (p_key < kth_key) p_key = kth_key;
@@ -614,7 +762,7 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
     cluster_sync();
     float cta_total[CS], total = 0.f;
     for (unsigned r = 0; r < CS; ++r) { cta_total[r] = ld_peer_f32(peer_smem(&x_total, r)); total += cta_total[r]; }
-    const float target = uniform[row] * total;
+    const float target = (!given ? uniform[row] : by_value.row[row].first ? 0.f : uniform_of(by_value.row[row].seed, by_value.row[row].counter)) * total;
     // which CTA: the first whose totals reach past the target; if rounding runs past the end, the last with mass
     int cta_pick = -1, last_cta = CS - 1;
     float cta_before = 0.f;
@@ -684,15 +832,15 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
     cluster_sync();         // nobody leaves while a peer may still read its shared memory
 }
 
-NIB_API int nib_sample(const float* logits, int rows, int vocab, const float* temperature, const int* top_k,
-                       const float* top_p, const float* uniform, int* out, cudaStream_t stream) {
+static int launch_sample(const float* logits, int rows, int vocab, const float* temperature, const int* top_k, const float* top_p,
+                         const float* uniform, int* out, const SampleRows& by_value, cudaStream_t stream) {
     NIB_REQUIRE(rows >= 0 && vocab > 0, "sample: bad sizes");
     if (rows == 0) return 0;
     NIB_REQUIRE((long long)vocab <= (1LL << 17) * 8, "sample: a row of %d logits is more than the fixed-point histograms hold", vocab);
     const int per = (ceil_div(vocab, CS * ST) + 3) & ~3;
     // Up to 32 rows all CTAs are at work at once, two an SM, and a row's time is what counts: 512 threads, and the slice kept in
     // shared memory if two of them fit an SM's (else for the 12 rows that one an SM holds). More rows: as many CTAs an SM as there can
-    // be (five), and the slice kept only where it is small. Measured at a vocabulary of 151,936, top-p 0.9, us: 1 row 47 (68 with 256
+    // be (five), and the slice kept only where it is small. Measured with another top-p select, at a vocabulary of 151,936, top-p 0.9, us: 1 row 47 (68 with 256
     // threads and nothing kept), 12 rows 49 (70), 16 rows 64 (82; 93 with one CTA an SM), 32 rows 69 (85; 143), 34 rows 97 (with 512
     // threads, which are two turns then, 99), 64 rows 122 (131); 32,000: 34 rows 35 (51 with 512 threads), 64 rows 41 (64; 53 with
     // nothing kept).
@@ -716,7 +864,26 @@ NIB_API int nib_sample(const float* logits, int rows, int vocab, const float* te
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    NIB_CUDA(cudaLaunchKernelEx(&cfg, kernel, logits, vocab, temperature, top_k, top_p, uniform, out));
+    NIB_CUDA(cudaLaunchKernelEx(&cfg, kernel, logits, vocab, temperature, top_k, top_p, uniform, out, by_value));
     NIB_LAUNCH_CHECK();
     return 0;
+}
+
+NIB_API int nib_sample(const float* logits, int rows, int vocab, const float* temperature, const int* top_k,
+                       const float* top_p, const float* uniform, int* out, cudaStream_t stream) {
+    NIB_REQUIRE(rows == 0 || (temperature && top_k && top_p && uniform), "sample: parameters are needed");
+    static const SampleRows none{};
+    return launch_sample(logits, rows, vocab, temperature, top_k, top_p, uniform, out, none, stream);
+}
+
+NIB_API int nib_sample_rows_most() { return ROWS_BY_VALUE; }
+
+// The same for up to nib_sample_rows_most() rows whose parameters lie in host memory (read before this returns) and whose uniform
+// numbers are made on the device. ``out`` may be page-locked host memory: each row's token is one store.
+NIB_API int nib_sample_rows(const float* logits, int rows, int vocab, const NibSampleRow* params, int* out, cudaStream_t stream) {
+    NIB_REQUIRE(rows >= 0 && rows <= ROWS_BY_VALUE && (rows == 0 || params != nullptr), "sample: up to %d rows by value", ROWS_BY_VALUE);
+    SampleRows by_value;
+    memset(&by_value, 0, sizeof(by_value));
+    if (rows > 0) memcpy(by_value.row, params, sizeof(NibSampleRow) * (size_t)rows);
+    return launch_sample(logits, rows, vocab, nullptr, nullptr, nullptr, nullptr, out, by_value, stream);
 }

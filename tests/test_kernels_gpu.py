@@ -1093,3 +1093,34 @@ def test_sampling_of_many_rows(K, vocab):
             if (r * vocab) % 4 == 0:        # (a row that does not start on 16 bytes adds up in another order)
                 K.sample(logits[r:r + 1], temperature[r:r + 1], top_k[r:r + 1], top_p[r:r + 1], uniform[r:r + 1], alone)
                 assert int(alone[0]) == int(out[r]), (rows, r)
+
+
+def test_sampling_from_gathered_elements_and_without(K):
+    """Up to 32 rows, a radix select goes on over a list once few enough elements are left; more rows never do. The same tokens for
+    rows whose candidates fit the list after one pass, after several and never, with ties at the edge, and parameters by value."""
+    from nanoinfer_b200.sampling.sampler import uniform_for
+    vocab, g = 20000, torch.Generator(device="cuda").manual_seed(5)
+    base = 2.0 * torch.randn(8, vocab, generator=g, device="cuda")
+    base[1] = (base[1] * 64).round() / 64                       # some ties everywhere
+    base[2] = (base[2] * 2).round() / 2                         # thousands of equal values: no list is ever short enough
+    base[3] = 1.5                                               # one value
+    base[4, :1024] += 40.0                                      # exactly as many above the rest as a list holds
+    base[5, :1025] = 30.0 + base[5, :1025].round()              # one more, and ties
+    base[6] = -base[6].abs() - 3.0                              # nothing above zero
+    base[7, 100:] = float("-inf")
+    kinds = [(1, 1.0), (40, 1.0), (700, 0.9), (1024, 0.999), (1025, 0.5), (5000, 0.95), (0, 0.1), (0, 0.9), (0, 0.9999), (0, 1.0), (vocab, 0.3), (1023, 0.0)]
+    for top_k, top_p in kinds:
+        for temperature in (1.0, 0.3, 25.0):
+            many = base.repeat(5, 1).contiguous()               # 40 rows
+            n = many.shape[0]
+            par = [torch.full((n,), v, dtype=t, device="cuda") for v, t in ((temperature, torch.float32), (top_k, torch.int32), (top_p, torch.float32))]
+            uniform = torch.tensor([uniform_for(i, 3 * i) for i in range(n)], device="cuda")
+            want, few = (torch.empty(n, dtype=torch.int32, device="cuda") for _ in range(2))
+            host = torch.empty(8, dtype=torch.int32).pin_memory()
+            K.sample(many, *par, uniform, want)
+            for r in range(0, n, 8):
+                K.sample(many[r:r + 8], *(p[r:r + 8].clone() for p in par), uniform[r:r + 8].clone(), few[r:r + 8])
+                K.sample_rows(many[r:r + 8], [(temperature, top_k, top_p, 0, i, 3 * i) for i in range(r, r + 8)], host)
+                torch.cuda.synchronize()
+                assert host.tolist() == few[r:r + 8].tolist(), (top_k, top_p, temperature, r)
+            assert torch.equal(want, few), (top_k, top_p, temperature, (want != few).nonzero().flatten().tolist())
