@@ -18,6 +18,7 @@ import torch
 from .params import SamplingParams
 
 _M64 = (1 << 64) - 1
+_INF = float("inf")
 
 
 def uniform_for(seed: int, counter: int) -> float:
@@ -92,6 +93,8 @@ class Sampler:
         self._penalise(logits, rows, pending)
         if all(r.params.greedy for r in rows):
             self.ops.argmax(logits, out)
+        elif on_gpu and self._by_value(n):
+            self.ops.sample_rows(logits, self._row_parameters(rows), out)
         else:
             self.ops.sample(logits, *self._device_parameters(rows, out.device, stage), out)
         if not on_gpu:       # a host backend (tests): nothing is asynchronous
@@ -109,6 +112,14 @@ class Sampler:
         assert logits.shape[0] == n
         dev = logits.device
         self._penalise(logits, rows, None)
+        if dev.type == "cuda" and self._by_value(n) and not all(r.params.greedy for r in rows):
+            # the parameters go with the launch and the tokens are stored to page-locked memory: no copy either way
+            host, _ = self._pinned_pair(n)
+            self.ops.sample_rows(logits, self._row_parameters(rows), host)
+            done = torch.cuda.Event()
+            done.record()
+            done.synchronize()
+            return host[:n].tolist()
         out = torch.empty(n, dtype=torch.int32, device=dev)
         if all(r.params.greedy for r in rows):
             self.ops.argmax(logits, out)
@@ -156,6 +167,23 @@ class Sampler:
             self._pinned_ids = [torch.empty(max(4096, 2 * size), dtype=torch.int32).pin_memory() for _ in range(self._RING)]
         self._seen_turn = (self._seen_turn + 1) % self._RING
         return self._pinned_ids[self._seen_turn]
+
+    def _by_value(self, n: int) -> bool:
+        return n <= getattr(self.ops, "sample_rows_most", 0)
+
+    @staticmethod
+    def _row_parameters(rows: Sequence[SampleRow]):
+        """(temperature, top_k, top_p, first, seed, counter) of each row as ``ops.sample_rows`` takes them; a greedy row as in
+        ``_device_parameters``."""
+        out = []
+        for r in rows:
+            p = r.params
+            t = p.temperature
+            if t == 0.0:
+                out.append((1.0, 1, 1.0, 1, 0, 0))
+            else:
+                out.append((t if t < 3.4e38 else _INF, min(p.k, 0x7FFFFFFF), p.p, 0, int(r.seed) & _M64, int(r.generated) & _M64))
+        return out
 
     def _device_parameters(self, rows: Sequence[SampleRow], dev, stage=None):
         """Temperature, top-k, top-p and the uniform numbers of the rows on the device: one array (top-k as integer
