@@ -86,11 +86,12 @@ gemm_smallm_kernel(const void* __restrict__ A, const __nv_bfloat16* __restrict__
     extern __shared__ float part[];                      // [KSPLIT][ACCS][NT][E][32] when KSPLIT > 1
     __shared__ int s_last;
 
-    // Up to 16 tokens the kernel behind this one may start only when this kernel's own loads are out (below): measured,
-    // dependents that are resident from this kernel's first instruction on take issue slots and bandwidth from it
-    // (batch 8: 3 us a step at the 0.5B widths, 30 us at the 1.5B widths). With more tokens the attention behind the
-    // q/k/v product wants its keys and values on their way as early as can be (batch 64: 1.53 against 1.56 ms).
-    constexpr bool LATE_DEPENDENTS = NT <= 2;
+    // Up to 16 tokens the kernel behind this one may start only when this kernel's own loads are out (below), where that is one that
+    // streams weights through registers: resident from this kernel's first instruction on it would take issue slots and bandwidth from
+    // it. Behind the output projection comes the gate/up product, which sends for its weights without either, and behind q/k/v the
+    // attention, which wants its keys and values on their way as early as can be: both are let in at once (us a step, 0.5B widths,
+    // one token at 777, 482 late and 475 at once, 16 at 1,000 715 and 707; 1.5B, 8 at 4,096 1,244 and 1,203, 4 at 500 1,021 and 994).
+    constexpr bool LATE_DEPENDENTS = NT <= 2 && EPI != EPI_ADD && EPI != EPI_QKV;
     if (!LATE_DEPENDENTS) pdl_launch_dependents();
     bool waited = false;          // pdl_wait() comes after the first batch of weight loads has been issued
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
