@@ -277,6 +277,23 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     __syncthreads();
     tc_fence_after();
     const unsigned tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    // The weights of the first item's stages are sent for before the wait: no kernel writes them, and this CTA is here only since
+    // nobody else's shared memory is in its way.
+    const auto send_w = [&](int s, int kb, int f0) {
+        unsigned char* st = smem + s * C::STAGE_BYTES;
+        mbar_expect_tx(&full_bar[s], C::STAGE_BYTES);
+        tma_load_2d(st, &map_w, &full_bar[s], kb * BLOCK_K, f0);
+        if (DUAL) tma_load_2d(st + C::W_BYTES, &map_w, &full_bar[s], kb * BLOCK_K, n_out + f0);
+    };
+    int ahead = 0;
+    if (warp == 0 && (int)blockIdx.x < items) {
+        const int tile = blockIdx.x / splits, kb = (blockIdx.x - tile * splits) * kb_per_split;
+        ahead = max(0, min(C::STAGES, min(k_blocks, kb + kb_per_split) - kb));
+        for (int i = 0; i < ahead; ++i) {
+            if (elect_one()) send_w(i, kb + i, (tile % f_tiles) * BLOCK_F);
+            __syncwarp();
+        }
+    }
     pdl_wait();         // from here on the kernel reads what earlier kernels wrote (activations, the residual stream)
     if (threadIdx.x == 0) nib_trace_mark(trace, trace_cap, NIB_TK_GEMM_TC, EPI, 1);
 
@@ -292,12 +309,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 const int s = it % C::STAGES;
                 ok = warp_wait(&empty_bar[s], ((it / C::STAGES) & 1) ^ 1);
                 if (!ok) break;
-                unsigned char* st = smem + s * C::STAGE_BYTES;
                 if (elect_one()) {
-                    mbar_expect_tx(&full_bar[s], C::STAGE_BYTES);
-                    tma_load_2d(st, &map_w, &full_bar[s], kb * BLOCK_K, f0);
-                    if (DUAL) tma_load_2d(st + C::W_BYTES, &map_w, &full_bar[s], kb * BLOCK_K, n_out + f0);
-                    tma_load_2d(st + (DUAL ? 2 : 1) * C::W_BYTES, &map_a, &full_bar[s], kb * BLOCK_K, t0);
+                    if (it >= ahead) send_w(s, kb, f0);
+                    tma_load_2d(smem + s * C::STAGE_BYTES + (DUAL ? 2 : 1) * C::W_BYTES, &map_a, &full_bar[s], kb * BLOCK_K, t0);
                 }
                 __syncwarp();
             }
