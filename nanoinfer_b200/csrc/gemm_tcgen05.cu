@@ -633,6 +633,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_m, const __grid_constan
     cluster_sync();            // the peer's barriers exist before anything signals them
     tc_fence_after();
     const unsigned tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+    // as in gemm_tc_kernel: the first item's weights before the wait
+    int ahead = 0;
+    if (warp == 0 && cluster_id < items) {
+        const int tile = cluster_id / splits, kb = (cluster_id - tile * splits) * kb_per_split, f0 = (tile % n_tiles) * FEAT;
+        ahead = max(0, min(C::STAGES, min(k_blocks, kb + kb_per_split) - kb));
+        for (int i = 0; i < ahead; ++i) {
+            const unsigned bar0 = peer_smem(&full_bar[i], 0);
+            if (elect_one()) {
+                if (rank == 0) mbar_expect_tx(&full_bar[i], 2 * C::STAGE_BYTES);
+                tma_load_2d_pair(smem + i * C::STAGE_BYTES + C::M_BYTES, &map_n, bar0, (kb + i) * BLOCK_K, GU ? f0 + (int)rank * n_out : f0 + (int)rank * (NT / 2));
+            }
+            __syncwarp();
+        }
+    }
     pdl_wait();
     if (threadIdx.x == 0) nib_trace_mark(trace, trace_cap, NIB_TK_GEMM_PAIR, EPI, 1);
 
@@ -653,9 +667,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_m, const __grid_constan
                 unsigned char* st = smem + s * C::STAGE_BYTES;
                 const unsigned bar0 = peer_smem(&full_bar[s], 0);
                 if (elect_one()) {
-                    if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * C::STAGE_BYTES);
+                    if (rank == 0 && it >= ahead) mbar_expect_tx(&full_bar[s], 2 * C::STAGE_BYTES);
                     tma_load_2d_pair(st, &map_m, bar0, kb * BLOCK_K, t0);
-                    tma_load_2d_pair(st + C::M_BYTES, &map_n, bar0, kb * BLOCK_K, w0);
+                    if (it >= ahead) tma_load_2d_pair(st + C::M_BYTES, &map_n, bar0, kb * BLOCK_K, w0);
                 }
                 __syncwarp();
             }
