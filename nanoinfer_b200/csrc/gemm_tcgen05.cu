@@ -935,6 +935,11 @@ NIB_API int nib_gemm_tc_splitk(const void* A, const void* W, const float* bias, 
         // The sum into the output can split K over CTAs instead, which reads large weights once (measured better from
         // about 16 MB of weights on: +8 % at the 7B widths, -2 % at the 0.5B widths).
         if (tok_tile == 64 && 2LL * f_tiles <= sm_count() && (epi != EPI_ADD || 2LL * N * K <= (16LL << 20))) tok_tile = 32;
+        // The gated product's feature tiles are twice as many rows: tiles of 16 tokens while they are one turn of the SMs and the
+        // weights are few, so that a tile's weights read once more come from L2 (us alone, by 32 and by 16: 4,864 x 896, 24 tokens 8.1 and
+        // 7.6, 40 8.7 and 7.8; 64 would be two turns, 8.7 and 11.6; 8,960 x 1,536, 24 tokens 13.3 and 14.6).
+        const long long sixteens = (long long)f_tiles * ceil_div(tokens, 16);      // (so many that K is not split besides)
+        if (epi_dual(epi) && tokens > 16 && tokens <= 64 && sixteens <= sm_count() && 2 * sixteens > sm_count() && 4LL * N * K <= (32LL << 20)) tok_tile = 16;
     }
     NIB_REQUIRE(ceil_div(tokens, tok_tile) <= 65535, "gemm (tensor cores): too many token tiles");
     SplitK sk;
