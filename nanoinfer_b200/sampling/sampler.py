@@ -9,7 +9,9 @@ reproducible only within one engine; so are these.
 """
 from __future__ import annotations
 
+from collections import deque
 from dataclasses import dataclass
+from threading import Lock
 from typing import List, Optional, Sequence
 
 import numpy as np
@@ -43,22 +45,29 @@ class SampleRow:
 
 class PendingTokens:
     """Tokens sampled on the device whose copy to the host is under way: ``device`` can feed the next
-    step at once, ``wait()`` returns the ids."""
+    step at once, ``wait()`` returns the ids. The page-locked buffer they arrive in is nobody else's until then."""
 
-    def __init__(self, device: torch.Tensor, host: torch.Tensor, event, n: int):
-        self.device, self._host, self._event, self._n = device, host, event, n
+    def __init__(self, device: torch.Tensor, host: torch.Tensor, event, n: int, give_back=None):
+        self.device, self._host, self._event, self._n, self._give_back = device, host, event, n, give_back
+        self._ids: Optional[List[int]] = None
+        self._lock = Lock()         # the buffer is given back once
 
     def wait(self) -> List[int]:
-        if self._event is not None:
-            self._event.synchronize()
-        return self._host[:self._n].tolist()
+        with self._lock:
+            if self._ids is None:
+                if self._event is not None:
+                    self._event.synchronize()
+                self._ids, host, self._host = self._host[:self._n].tolist(), self._host, None
+                if self._give_back is not None:
+                    self._give_back(host)
+        return list(self._ids)
 
 
 class Sampler:
     def __init__(self, ops, device):
         self.ops, self.device = ops, torch.device(device)
-        self._pinned: List[torch.Tensor] = []       # host buffers of the asynchronous reads, used in turn
-        self._pinned_par: List[torch.Tensor] = []   # and of the sampling parameters on their way to the device
+        self._free_tokens = deque(maxlen=8)         # page-locked buffers for tokens that no call is using
+        self._pinned_par: List[torch.Tensor] = []   # host buffers of the sampling parameters on their way to the device, used in turn
         self._turn = 0
         self._pinned_ids: List[torch.Tensor] = []   # and of the ids that a repetition penalty applies to
         self._seen_turn = 0
@@ -71,14 +80,21 @@ class Sampler:
 
     _RING = 4       # pinned buffers in rotation: one is reused only after three more steps have been launched
 
-    def _pinned_pair(self, n: int):
-        """This call's pinned buffers (tokens out, sampling parameters in), large enough for ``n`` rows."""
-        if not self._pinned or self._pinned[0].numel() < n:
-            size = max(256, 2 * n)
-            self._pinned = [torch.empty(size, dtype=torch.int32).pin_memory() for _ in range(self._RING)]
-            self._pinned_par = [torch.empty(4 * size, dtype=torch.float32).pin_memory() for _ in range(self._RING)]
+    def _pinned_parameters(self, n: int) -> torch.Tensor:
+        """This call's pinned buffer for the parameters of ``n`` rows."""
+        if not self._pinned_par or self._pinned_par[0].numel() < 4 * n:
+            self._pinned_par = [torch.empty(4 * max(256, 2 * n), dtype=torch.float32).pin_memory() for _ in range(self._RING)]
         self._turn = (self._turn + 1) % self._RING
-        return self._pinned[self._turn], self._pinned_par[self._turn]
+        return self._pinned_par[self._turn]
+
+    def _token_buffer(self, n: int) -> torch.Tensor:
+        """A page-locked buffer for ``n`` tokens that belongs to the caller until it gives it back to ``_free_tokens`` (a read that
+        is still out must not be written by the calls behind it, however many there are, nor by another thread's)."""
+        try:
+            host = self._free_tokens.pop()
+        except IndexError:
+            host = None
+        return host if host is not None and host.numel() >= n else torch.empty(max(256, 2 * n), dtype=torch.int32).pin_memory()
 
     def sample_async(self, logits: torch.Tensor, rows: Sequence[SampleRow],
                      pending: Optional[torch.Tensor] = None) -> PendingTokens:
@@ -89,20 +105,20 @@ class Sampler:
         assert logits.shape[0] == n and self.can_sample_async(rows)
         out = torch.empty(n, dtype=torch.int32, device=logits.device)
         on_gpu = out.device.type == "cuda"
-        host, stage = self._pinned_pair(n) if on_gpu else (None, None)
         self._penalise(logits, rows, pending)
         if all(r.params.greedy for r in rows):
             self.ops.argmax(logits, out)
         elif on_gpu and self._by_value(n):
             self.ops.sample_rows(logits, self._row_parameters(rows), out)
         else:
-            self.ops.sample(logits, *self._device_parameters(rows, out.device, stage), out)
+            self.ops.sample(logits, *self._device_parameters(rows, out.device), out)
         if not on_gpu:       # a host backend (tests): nothing is asynchronous
             return PendingTokens(out, out, None, n)
+        host = self._token_buffer(n)
         host[:n].copy_(out, non_blocking=True)
         event = torch.cuda.Event()
         event.record()
-        return PendingTokens(out, host, event, n)
+        return PendingTokens(out, host, event, n, self._free_tokens.append)
 
     def sample(self, logits: torch.Tensor, rows: Sequence[SampleRow]) -> List[int]:
         """One token per row of ``logits [len(rows), vocab]`` (float32, on the device; penalised in place)."""
@@ -114,12 +130,14 @@ class Sampler:
         self._penalise(logits, rows, None)
         if dev.type == "cuda" and self._by_value(n) and not all(r.params.greedy for r in rows):
             # the parameters go with the launch and the tokens are stored to page-locked memory: no copy either way
-            host, _ = self._pinned_pair(n)
+            host = self._token_buffer(n)
             self.ops.sample_rows(logits, self._row_parameters(rows), host)
             done = torch.cuda.Event()
             done.record()
             done.synchronize()
-            return host[:n].tolist()
+            tokens = host[:n].tolist()
+            self._free_tokens.append(host)
+            return tokens
         out = torch.empty(n, dtype=torch.int32, device=dev)
         if all(r.params.greedy for r in rows):
             self.ops.argmax(logits, out)
@@ -162,7 +180,7 @@ class Sampler:
         self.ops.repetition_penalty(logits, d[2 * n + 1:], d[n:2 * n + 1], d[:n].view(torch.float32), pending)
 
     def _pinned_seen(self, size: int) -> torch.Tensor:
-        """Pinned staging for the ids of the penalty, in the same rotation as the other two buffers."""
+        """Pinned staging for the ids of the penalty, in the same rotation as the parameters' buffers."""
         if len(self._pinned_ids) != self._RING or self._pinned_ids[0].numel() < size:
             self._pinned_ids = [torch.empty(max(4096, 2 * size), dtype=torch.int32).pin_memory() for _ in range(self._RING)]
         self._seen_turn = (self._seen_turn + 1) % self._RING
@@ -182,10 +200,10 @@ class Sampler:
             if t == 0.0:
                 out.append((1.0, 1, 1.0, 1, 0, 0))
             else:
-                out.append((t if t < 3.4e38 else _INF, min(p.k, 0x7FFFFFFF), p.p, 0, int(r.seed) & _M64, int(r.generated) & _M64))
+                out.append((_INF if t >= 3.4e38 else t, min(p.k, 0x7FFFFFFF), p.p, 0, int(r.seed) & _M64, int(r.generated) & _M64))
         return out
 
-    def _device_parameters(self, rows: Sequence[SampleRow], dev, stage=None):
+    def _device_parameters(self, rows: Sequence[SampleRow], dev):
         """Temperature, top-k, top-p and the uniform numbers of the rows on the device: one array (top-k as integer
         bits), one copy from pinned memory. A greedy row beside sampled ones is the draw at 0 from the one largest
         logit at temperature 1: of the elements that are kept (the maxima) the first in vocabulary order is taken,
@@ -197,9 +215,7 @@ class Sampler:
             if not p.greedy:
                 temperature[i], top_k[i], top_p[i], uniform[i] = p.temperature, p.k, p.p, uniform_for(r.seed, r.generated)
         on_gpu = torch.device(dev).type == "cuda"
-        if on_gpu and stage is None:
-            _, stage = self._pinned_pair(n)
-        host = stage[:4 * n] if on_gpu else torch.empty(4 * n, dtype=torch.float32)
+        host = self._pinned_parameters(n)[:4 * n] if on_gpu else torch.empty(4 * n, dtype=torch.float32)
         par = host.numpy().reshape(4, n)
         par[0], par[1].view(np.int32)[:], par[2], par[3] = temperature, top_k, top_p, uniform
         d = host
