@@ -98,6 +98,7 @@ class Kernels:
     instance's options, which never change, and its scratch memory."""
 
     name = "cuda-sm100a"
+    weights_ahead = False       # see with_weights_ahead()
 
     def __init__(self, lib_path: str, options: Optional[KernelOptions] = None):
         self.lib_path = lib_path
@@ -272,6 +273,14 @@ class Kernels:
         k.options = options if options is not None else dataclasses.replace(self.options, **changes)
         return k
 
+    def with_weights_ahead(self, ahead: bool = True) -> "Kernels":
+        """As ``with_options``, an instance whose caller promises that no kernel writes the matrices it hands to the products (a model's
+        parameters): the tensor-core and streamed products then read them while the kernels before them are still running. An instance
+        without the promise launches those products plainly, behind everything before them, so that W may be any kernel's result."""
+        k = self.with_options(self.options)
+        k.weights_ahead = ahead
+        return k
+
     def ensure_workspace(self, device) -> None:
         """Scratch memory that kernels share between launches (allocated once, outside any graph capture)."""
         if self._ws_scratch is None:
@@ -283,7 +292,9 @@ class Kernels:
 
     def linear(self, a, w, bias32, out, mode):
         """out[M,N] (=, +=) a[M,K] . w[N,K]^T (+ bias). mode: 'store' | 'add' (float out) | 'f32' (float out).
-        ``a`` may be a LazyNorm: the small-M kernel then applies the norm while it reads the residual stream."""
+        ``a`` may be a LazyNorm: the small-M kernel then applies the norm while it reads the residual stream. The products of few tokens
+        (small-M, and 32-bit ones) read ``w`` before they wait for the kernel before them: there it must not be what a kernel
+        launched just before writes; with more tokens that holds of an instance made by ``with_weights_ahead`` only."""
         lazy = a if isinstance(a, LazyNorm) else None
         dtype = a.dtype
         if lazy is None:
@@ -373,6 +384,8 @@ class Kernels:
         src = a if norm is None else norm.fold.x32
         if self._lib.nib_gemm_stream_supported(_ptr(src), _ptr(w), c_int(m), c_int(k), c_int(src.stride(0)), c_int(2 if norm is None else 4), c_int(splits)) != 1:
             return False
+        if not self.weights_ahead:
+            self._lib.nib_pdl_skip_next()
         self._check(self._lib.nib_gemm_stream(
             _ptr(src), _ptr(w), _ptr(bias32), _ptr(out), c_int(m), c_int(n), c_int(k), c_int(src.stride(0)), c_int(out.stride(0)), c_int(epi),
             c_int(splits), _ptr(None if norm is None else norm.fold.gain32), c_float(0.0 if norm is None else norm.fold.eps), glu, self._stream()),
@@ -427,6 +440,8 @@ class Kernels:
         if lazy is not None:
             a = lazy.resolve()
         if bf16 and self._lib.nib_gemm_tc_supported(_ptr(a), _ptr(w), c_int(k), c_int(a.stride(0))) == 1:
+            if not self.weights_ahead:
+                self._lib.nib_pdl_skip_next()
             if self._use_pair(m, w.shape[0], k, epi):
                 self._check(self._lib.nib_gemm_tc_pair(
                     _ptr(a), _ptr(w), _ptr(bias32), _ptr(out), c_int(m), c_int(n), c_int(k), c_int(a.stride(0)),
@@ -519,6 +534,8 @@ class Kernels:
                 raise KernelError("qkv_project: pages or block table do not fit")
             num_pages, bt_stride = k_pages.shape[0], block_table.stride(0)
         if fused_tc:
+            if not self.weights_ahead:
+                self._lib.nib_pdl_skip_next()
             self._check(self._lib.nib_gemm_tc_qkv(
                 _ptr(a), _ptr(w_qkv), _ptr(bias32), _ptr(qkv), c_int(m), c_int(heads), c_int(kv_heads), c_int(head_dim),
                 c_int(k), c_int(a.stride(0)), c_int(qkv.stride(0)), _ptr(positions), _ptr(req_index), _ptr(cos), _ptr(sin),

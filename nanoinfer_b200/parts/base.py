@@ -34,7 +34,9 @@ class Runtime:
     """Where and with what a part computes."""
     device: torch.device
     dtype: torch.dtype            # torch.bfloat16 or torch.float32: activations, matrices, cache
-    ops: object                   # the kernel library (csrc/lib.py: Kernels)
+    # The kernel library (csrc/lib.py: Kernels). An engine's reads the matrices given to its products ahead of the kernels before them: a
+    # part that multiplies with a matrix that a kernel writes takes ``ops.with_weights_ahead(False)`` for it, and more than 16 tokens.
+    ops: object
 
     def matrix(self, t: torch.Tensor) -> torch.Tensor:
         """A matrix operand: compute dtype, contiguous, on the device."""

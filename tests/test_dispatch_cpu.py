@@ -4,6 +4,7 @@ projection sizes of the 0.5B, 1.5B and 7B models; the test pins them for those s
 threshold shows up as a decision that moved. No GPU and no library are needed: the rules read nothing but
 their arguments, the object's options and its count of SMs."""
 import pytest
+import torch
 
 import dataclasses
 
@@ -110,3 +111,50 @@ def test_decode_attention_splits_of_short_contexts(rules):
     assert [rules.decode_splits(n, 2, 512, 0, True, 64) for n in (1, 4, 8, 9, 10, 16, 32)] == [4, 4, 4, 4, 1, 1, 1]
     assert [rules.decode_splits(n, 2, 1024, 0, True, 64) for n in (1, 4, 5, 8, 16, 18, 19, 32)] == [8, 8, 4, 4, 4, 4, 2, 2]
     assert [rules.decode_splits(n, 2, 512, 0, True, 128) for n in (1, 9, 10, 18, 19, 32)] == [8, 8, 4, 4, 2, 2]
+
+
+class Library:
+    """A library that takes everything and notes what it was asked for."""
+
+    def __init__(self, refuses=()):
+        self.calls, self.refuses = [], refuses
+
+    def __getattr__(self, name):
+        def entry(*args):
+            self.calls.append(name)
+            return 0 if name in self.refuses else 1 if name.endswith("_supported") else 0
+        return entry
+
+    def launches(self):
+        out = [c for c in self.calls if not c.endswith("_supported")]
+        self.calls.clear()
+        return out
+
+
+def host_side(rules, **changes):
+    """``rules`` with a library that launches nothing, on tensors of the host."""
+    k = rules.with_options(**changes) if changes else rules
+    k._lib, k.launches, k._op_events, k._bound_stream = Library(), 0, None, 0
+    k._ws_scratch = k._ws_counters = torch.zeros(1)
+    return k
+
+
+def operands(m, n, k, dual=False):
+    return torch.zeros(m, k, dtype=torch.bfloat16), torch.zeros(2 * n if dual else n, k, dtype=torch.bfloat16), torch.zeros(m, n, dtype=torch.bfloat16)
+
+
+def test_a_matrix_that_a_kernel_may_write_is_read_behind_it(rules):
+    """Unless the instance was promised parameters, the products whose kernels send for W before they wait are plain launches."""
+    k = host_side(rules)
+    ahead = k.with_weights_ahead()
+    assert ahead.weights_ahead and not k.weights_ahead and not ahead.with_options(gemm_route="tc").with_weights_ahead(False).weights_ahead
+    tokens = 17
+    for m, launch in ((tokens, "nib_gemm_tc_splitk"), (600, "nib_gemm_tc_pair")):
+        a, w, out = operands(m, 7168, 256)
+        for ops, plain in ((k, ["nib_pdl_skip_next"]), (ahead, []), (ahead.with_options(tc_splits=0), []), (ahead.with_weights_ahead(False), ["nib_pdl_skip_next"])):
+            ops._gemm(a, w, None, out, m, 7168, 256, _EPI["store"])
+            assert k._lib.launches() == plain + [launch]
+    a, w, out = operands(12, 512, 256, dual=True)
+    for ops, plain in ((k, ["nib_pdl_skip_next"]), (ahead, [])):
+        ops._gemm(a, w, None, out, 12, 512, 256, _EPI["swiglu"])
+        assert k._lib.launches() == plain + ["nib_gemm_stream"]

@@ -1124,3 +1124,26 @@ def test_sampling_from_gathered_elements_and_without(K):
                 torch.cuda.synchronize()
                 assert host.tolist() == few[r:r + 8].tolist(), (top_k, top_p, temperature, r)
             assert torch.equal(want, few), (top_k, top_p, temperature, (want != few).nonzero().flatten().tolist())
+
+
+@pytest.mark.parametrize("m", [17, 64, 128, 600])
+def test_a_product_with_a_matrix_that_the_product_before_it_writes(K, m):
+    """Without the promise that no kernel writes its matrix, a product reads it behind the kernels before it. (Small whole numbers: exact sums.)"""
+    n, k, inner = 2048, 1024, 256
+    small = lambda shape, seed: torch.randint(-1, 2, shape, generator=torch.Generator().manual_seed(seed)).to(torch.bfloat16).cuda()      # noqa: E731
+    left, right, a = small((n, inner), 1), small((k, inner), 2), small((m, k), 3)
+    want_w = (left.float() @ right.float().t()).to(torch.bfloat16)
+    want = (a.double() @ want_w.double().t()).float()
+    want_glu = torch.empty(12, n // 2, dtype=torch.bfloat16, device="cuda")
+    REF.linear_swiglu(a[:12].contiguous(), want_w, want_glu)
+    for turn in range(4):
+        w, out = torch.zeros(n, k, dtype=torch.bfloat16, device="cuda"), torch.empty(m, n, device="cuda")
+        torch.cuda.synchronize()
+        K.linear(left, right, None, w, "store")
+        K.linear(a, w, None, out, "f32")
+        assert torch.equal(w, want_w) and torch.equal(out, want)
+        w, glu = torch.zeros(n, k, dtype=torch.bfloat16, device="cuda"), torch.empty(12, n // 2, dtype=torch.bfloat16, device="cuda")
+        torch.cuda.synchronize()
+        K.linear(left, right, None, w, "store")
+        K.linear_swiglu(a[:12], w, glu)           # the streamed product
+        assert_close(glu, want_glu, torch.bfloat16, "gated, of a written matrix")
