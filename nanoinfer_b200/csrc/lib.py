@@ -24,6 +24,7 @@ class KernelError(RuntimeError):
 
 _DT = {torch.float32: 0, torch.bfloat16: 1}
 _EPI = {"store": 0, "add": 1, "f32": 2, "swiglu": 3, "glu": 5, "geglu": 6}
+_ADD = _EPI["add"]
 _DUAL = (3, 5, 6)       # the gated epilogues: two accumulators, gate rows and up rows
 _LAYOUT = {"interleaved": 0, "half": 1}     # which elements of a rotated vector make a pair
 
@@ -416,11 +417,12 @@ class Kernels:
         if lazy is not None and not self._foldable(lazy):
             a, lazy = lazy.resolve(), None
         bf16 = a.dtype == torch.bfloat16 and not self.options.force_simt_gemm
-        splits = self._use_stream(m, n, k, epi, lazy is not None) if bf16 and (lazy is None or epi in _DUAL) else 0
-        if splits and self._streamed(splits, a, lazy, w, bias32, out, m, n, k, epi, glu):
-            return
-        if lazy is not None and lazy.resolved is not None:
-            a, lazy = lazy.resolved, None
+        if m <= 16 and bf16 and (epi in _DUAL or (epi == _ADD and lazy is None)):      # (a prompt's products are not to pay for the question)
+            splits = self._use_stream(m, n, k, epi, lazy is not None)
+            if splits and self._streamed(splits, a, lazy, w, bias32, out, m, n, k, epi, glu):
+                return
+            if lazy is not None and lazy.resolved is not None:
+                a, lazy = lazy.resolved, None
         if bf16 and self.options.tc_token_tile == 0:
             kernel, fuse = self._route(m, w.shape[0], k, epi, lazy is not None)
             if lazy is not None and not fuse:

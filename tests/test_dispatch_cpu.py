@@ -158,3 +158,16 @@ def test_a_matrix_that_a_kernel_may_write_is_read_behind_it(rules):
     for ops, plain in ((k, ["nib_pdl_skip_next"]), (ahead, [])):
         ops._gemm(a, w, None, out, 12, 512, 256, _EPI["swiglu"])
         assert k._lib.launches() == plain + ["nib_gemm_stream"]
+
+
+def test_the_streamed_product_is_asked_only_where_it_could_be_meant(rules, monkeypatch):
+    """The host launches a prompt's step product by product: one of more than 16 tokens, or of another epilogue, costs no question."""
+    k = host_side(rules)
+    asked = []
+    monkeypatch.setattr(Kernels, "_use_stream", lambda self, *a: asked.append(a) or 0)
+    for m, epi, dual, question in ((17, "swiglu", True, False), (100, "add", False, False), (1, "store", False, False), (16, "f32", False, False),
+                                   (16, "swiglu", True, True), (1, "add", False, True), (16, "geglu", True, True)):
+        a, w, out = operands(m, 512, 256, dual)
+        k._gemm(a, w, None, out, m, 512, 256, _EPI[epi])
+        assert len(asked) == question, (m, epi)
+        asked.clear()
