@@ -60,6 +60,7 @@ struct QkvEpi {
     const int* positions; const int* req_index; const float* cos_t; const float* sin_t;
     const int* block_table; int bt_stride, page_size, num_pages;
     __nv_bfloat16* k_pages; __nv_bfloat16* v_pages; int writes;
+    int late;       // up to 16 tokens: the kernel behind this one is let in when the weights are read
 };
 
 // First rows of the two halves of row group `group` in the q/k/v form.
@@ -88,11 +89,14 @@ gemm_smallm_kernel(const void* __restrict__ A, const __nv_bfloat16* __restrict__
 
     // Up to 16 tokens the kernel behind this one may start only when this kernel's own loads are out (below), where that is one that
     // streams weights through registers: resident from this kernel's first instruction on it would take issue slots and bandwidth from
-    // it. Behind the output projection comes the gate/up product, which sends for its weights without either, and behind q/k/v the
-    // attention, which wants its keys and values on their way as early as can be: both are let in at once (us a step, 0.5B widths,
-    // one token at 777, 482 late and 475 at once, 16 at 1,000 715 and 707; 1.5B, 8 at 4,096 1,244 and 1,203, 4 at 500 1,021 and 994).
-    constexpr bool LATE_DEPENDENTS = NT <= 2 && EPI != EPI_ADD && EPI != EPI_QKV;
-    if (!LATE_DEPENDENTS) pdl_launch_dependents();
+    // it. Behind the output projection comes the gate/up product, which sends for its weights without either, and behind a decode
+    // step's q/k/v the attention, which wants its keys and values on their way as early as can be: both are let in at once (us a step,
+    // q/k/v late / at once: 0.5B widths, one token at 777 480 / 471, 16 at 4,000 909 / 893; 1.5B, 8 at 4,090 1,215 / 1,175). A prompt's
+    // attention has nothing to fetch that early, and what comes behind it takes bandwidth from this kernel (four layers of the 7B, late /
+    // at once: a prompt of 12 tokens 618 / 643, 16 behind 1,000 657 / 703): the host says which it is.
+    constexpr bool MAY_BE_LATE = NT <= 2 && EPI != EPI_ADD;
+    const bool late = MAY_BE_LATE && (EPI != EPI_QKV || qe.late);
+    if (!late) pdl_launch_dependents();
     bool waited = false;          // pdl_wait() comes after the first batch of weight loads has been issued
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     if (threadIdx.x == 0) nib_trace_mark(trace, trace_cap, NIB_TK_GEMM_SMALLM, EPI, 0);
@@ -241,7 +245,7 @@ gemm_smallm_kernel(const void* __restrict__ A, const __nv_bfloat16* __restrict__
             }
         }
     }
-    if (LATE_DEPENDENTS) pdl_launch_dependents();
+    if (late) pdl_launch_dependents();
     if (!waited) pdl_wait();      // before the first write (shared results, scratch, output)
     if (NORM) {
         // the four threads of a quad hold the same token's partial sums: add them (fixed order)
@@ -534,12 +538,13 @@ NIB_API int nib_gemm_smallm_qkv_supported(const void* A, const void* W, int toke
 // head_dim] = A . W^T + bias (A, gain, eps as in nib_gemm_smallm); query and key heads are rotated by
 // positions[token] (tables of rot/2 values per position; the first rot dimensions of a head, halves paired); the whole
 // row is stored to ``qkv``; with ``writes`` the rotated key and the value also go to the slot of the token's position
-// in its request's page (block_table[req_index[token]][position / page_size]; a negative entry is skipped).
+// in its request's page (block_table[req_index[token]][position / page_size]; a negative entry is skipped). ``late``: what comes
+// behind a product of up to 16 tokens is let in late (see the kernel).
 NIB_API int nib_gemm_smallm_qkv(const void* A, const void* W, const float* bias, void* qkv, int tokens, int heads,
                                 int kv_heads, int head_dim, int K, int lda, int ldq, const float* gain, float eps,
                                 const int* positions, const int* req_index, const float* cos_t, const float* sin_t,
                                 int rot, const int* block_table, int bt_stride, int page_size, void* k_pages,
-                                void* v_pages, int num_pages, int writes, cudaStream_t stream) {
+                                void* v_pages, int num_pages, int writes, int late, cudaStream_t stream) {
     const int N = (heads + 2 * kv_heads) * head_dim;
     NIB_REQUIRE(heads > 0 && kv_heads > 0 && lda >= K && ldq >= N, "gemm (small M, q/k/v): bad sizes heads=%d/%d head_dim=%d", heads, kv_heads, head_dim);
     NIB_REQUIRE(nib_gemm_smallm_qkv_supported(A, W, tokens, K, lda, gain ? 4 : 2, head_dim, rot),
@@ -551,7 +556,7 @@ NIB_API int nib_gemm_smallm_qkv(const void* A, const void* W, const float* bias,
     NIB_REQUIRE(gain == nullptr || (((uintptr_t)gain & 15) == 0), "gemm (small M, q/k/v): the gain must be 16-byte aligned");
     Args a{A, W, bias, qkv, tokens, N, K, lda, ldq, gain, eps, nullptr, nullptr, 1,
            QkvEpi{heads, kv_heads, head_dim, rot, positions, req_index, cos_t, sin_t, block_table, bt_stride, page_size,
-                  num_pages, (__nv_bfloat16*)k_pages, (__nv_bfloat16*)v_pages, writes}, NibGlu{}};
+                  num_pages, (__nv_bfloat16*)k_pages, (__nv_bfloat16*)v_pages, writes, late}, NibGlu{}};
     if (gain) return launch_tokens<true>(WARPS, EPI_QKV, a, stream);
     return launch_tokens<false>(WARPS, EPI_QKV, a, stream);
 }

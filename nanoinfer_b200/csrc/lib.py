@@ -551,7 +551,8 @@ class Kernels:
             c_int(k), c_int(src.stride(0)), c_int(qkv.stride(0)), _ptr(gain), c_float(lazy.fold.eps if lazy is not None else 0.0),
             _ptr(positions), _ptr(req_index), _ptr(cos), _ptr(sin), c_int(rot), _ptr(block_table if writes else None),
             c_int(bt_stride), c_int(page_size), _ptr(k_pages if writes else None), _ptr(v_pages if writes else None),
-            c_int(num_pages), c_int(1 if writes else 0), self._stream()), "q/k/v projection with rotation and page write")
+            c_int(num_pages), c_int(1 if writes else 0), c_int(0 if block_table is not None and block_table.shape[0] == m else 1),     # as many requests as tokens: decoding
+            self._stream()), "q/k/v projection with rotation and page write")
 
     def rope_store(self, qkv, heads, kv_heads, head_dim, positions, req_index, rotary, block_table,
                    page_size, k_pages, v_pages, writes):

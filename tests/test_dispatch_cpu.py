@@ -122,6 +122,7 @@ class Library:
     def __getattr__(self, name):
         def entry(*args):
             self.calls.append(name)
+            self.args = args
             return 0 if name in self.refuses else 1 if name.endswith("_supported") else 0
         return entry
 
@@ -171,3 +172,15 @@ def test_the_streamed_product_is_asked_only_where_it_could_be_meant(rules, monke
         k._gemm(a, w, None, out, m, 512, 256, _EPI[epi])
         assert len(asked) == question, (m, epi)
         asked.clear()
+
+
+@pytest.mark.parametrize("requests,late", [(12, 0), (1, 1), (3, 1)])
+def test_what_comes_behind_few_tokens_of_a_prompt_is_let_in_late(rules, monkeypatch, requests, late):
+    """The q/k/v product lets a decode step's attention in at once, and a prompt's only behind its weights."""
+    k, m = host_side(rules), 12
+    monkeypatch.setattr("nanoinfer_b200.csrc.lib._need", lambda *a, **kw: None)
+    a, w, qkv = operands(m, 256, 128)
+    table, pages = torch.zeros(requests, 2, dtype=torch.int32), torch.zeros(4, 1, 16, 64, dtype=torch.bfloat16)
+    k.qkv_project(a, w, None, qkv, 2, 1, 64, torch.zeros(m, dtype=torch.int32), torch.zeros(m, dtype=torch.int32), None, table, 16, pages, pages, True)
+    assert k._lib.launches() == ["nib_gemm_smallm_qkv"]
+    assert k._lib.args[-2].value == late
