@@ -417,7 +417,8 @@ class Kernels:
         if lazy is not None and not self._foldable(lazy):
             a, lazy = lazy.resolve(), None
         bf16 = a.dtype == torch.bfloat16 and not self.options.force_simt_gemm
-        if m <= 16 and bf16 and (epi in _DUAL or (epi == _ADD and lazy is None)):      # (a prompt's products are not to pay for the question)
+        if m <= 16 and bf16 and (epi in _DUAL or (epi == _ADD and lazy is None and (m == 1 or self.options.gemm_route == "stream"))):
+            # (the others are not to pay for the question)
             splits = self._use_stream(m, n, k, epi, lazy is not None)
             if splits and self._streamed(splits, a, lazy, w, bias32, out, m, n, k, epi, glu):
                 return

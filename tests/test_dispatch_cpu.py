@@ -166,7 +166,7 @@ def test_the_streamed_product_is_asked_only_where_it_could_be_meant(rules, monke
     k = host_side(rules)
     asked = []
     monkeypatch.setattr(Kernels, "_use_stream", lambda self, *a: asked.append(a) or 0)
-    for m, epi, dual, question in ((17, "swiglu", True, False), (100, "add", False, False), (1, "store", False, False), (16, "f32", False, False),
+    for m, epi, dual, question in ((17, "swiglu", True, False), (100, "add", False, False), (1, "store", False, False), (16, "f32", False, False), (2, "add", False, False),
                                    (16, "swiglu", True, True), (1, "add", False, True), (16, "geglu", True, True)):
         a, w, out = operands(m, 512, 256, dual)
         k._gemm(a, w, None, out, m, 512, 256, _EPI[epi])
