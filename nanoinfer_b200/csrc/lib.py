@@ -359,17 +359,32 @@ class Kernels:
 
     def _use_stream(self, m: int, n: int, k: int, epi: int, has_norm: bool) -> int:
         """Into how many CTAs' stretches of K the streamed product (weights copied into shared memory ahead of everything) cuts
-        this product of at most 16 tokens; 0: another kernel takes it. Measured as whole decode steps at the widths of the
-        0.5B, 1.5B and 7B models: gate/up behind its norm wins for every number of tokens up to 16 (us a step without / with: one token 565 /
-        498, 1,060 / 1,005, 585 / 560; 8 tokens 640 / 571, 1,176 / 1,106; 16 tokens of the 0.5B 814 / 699); up to 8 tokens of an input
-        that is normed already the small-M product is as good (5,632 x 2,048: 11.2 us and 11.6). The down projection wins for one
+        this product of at most 16 tokens; 0: another kernel takes it. Measured as whole decode steps at the widths of the 0.5B,
+        1.5B and 7B models, and as chains of feed-forwards with weights from memory (us a layer, the other kernel / this one).
+
+        Gate/up. Up to 8 tokens it wins behind a norm, which it computes itself (one token 565 / 498, 1,060 / 1,005, 585 / 560 a step; a
+        layer of 256 x 1,024 6.2 / 4.3, of 2,048 x 14,336 33.2 / 31.5); of an input that is normed already the small-M product is as good (5,632 x 2,048:
+        11.2 and 11.6). With 9 to 16 the norm is a kernel of its own either way. The small-M product, which takes weights up to 12 MB, is the
+        better one there (16 tokens, 1,024 x 2,816 10.1 / 10.3, 512 x 2,048 8.0 / 8.9); above, this one wins while every SM's share is one turn of at
+        most 64 features (1,024 x 3,072 14.7 / 10.6, 896 x 4,864 14.4 / 12.5, 2,048 x 9,344 30.1 / 26.6), loses with two (1,024 x 9,600 16.8 / 18.3,
+        3,584 x 18,944 at 9 tokens 72.0 / 75.9) and wins with three, where the tcgen05 product's tiles of 128 features are more than the SMs
+        (1,024 x 19,200 29.0 / 28.8 and at 9 tokens 28.5 / 26.0; 28,416 36.3 / 34.6), and not with four (28,672: 36.6 / 37.4). Several turns go through a ring in
+        what the activations leave of the shared memory: from 24,576 of them on they lose (16 tokens, 2,048 x 22,528 55.5 / 59.7; 8 tokens, 3,584 x
+        18,944 72.4 / 73.3; 12 tokens, 2,048 x 22,528 55.3 / 51.8).
+
+        The down projection wins for one
         token while a CTA of eight that share K holds its weights whole (498 / 474; two tokens 507 / 503, 8 at 4,096 640 / 661; 1.5B, one
         token 1,005 / 1,094)."""
         o = self.options
         if o.gemm_route not in (None, "stream") or o.tc_token_tile or o.tc_splits or o.smallm_ksplit or o.smallm_cross or m > 16 or k % 64:
             return 0
         if epi in _DUAL:
-            return 1 if has_norm or m > 8 or o.gemm_route == "stream" else 0
+            if o.gemm_route == "stream":
+                return 1
+            turns = -(-n // (64 * self.sm_count))
+            if turns > 1 and m * k > 24576:
+                return 0
+            return 1 if (has_norm if m <= 8 else 4 * n * k > 12e6 and turns in (1, 3)) else 0
         if epi != _EPI["add"]:
             return 0
         if o.gemm_route == "stream":

@@ -155,9 +155,9 @@ def test_a_matrix_that_a_kernel_may_write_is_read_behind_it(rules):
         for ops, plain in ((k, ["nib_pdl_skip_next"]), (ahead, []), (ahead.with_options(tc_splits=0), []), (ahead.with_weights_ahead(False), ["nib_pdl_skip_next"])):
             ops._gemm(a, w, None, out, m, 7168, 256, _EPI["store"])
             assert k._lib.launches() == plain + [launch]
-    a, w, out = operands(12, 512, 256, dual=True)
+    a, w, out = operands(12, 4096, 1024, dual=True)
     for ops, plain in ((k, ["nib_pdl_skip_next"]), (ahead, [])):
-        ops._gemm(a, w, None, out, 12, 512, 256, _EPI["swiglu"])
+        ops._gemm(a, w, None, out, 12, 4096, 1024, _EPI["swiglu"])
         assert k._lib.launches() == plain + ["nib_gemm_stream"]
 
 
@@ -184,3 +184,27 @@ def test_what_comes_behind_few_tokens_of_a_prompt_is_let_in_late(rules, monkeypa
     k.qkv_project(a, w, None, qkv, 2, 1, 64, torch.zeros(m, dtype=torch.int32), torch.zeros(m, dtype=torch.int32), None, table, 16, pages, pages, True)
     assert k._lib.launches() == ["nib_gemm_smallm_qkv"]
     assert k._lib.args[-2].value == late
+
+
+def test_gated_products_of_up_to_16_tokens(rules):
+    """Streamed behind a norm up to 8 tokens; with more, above the small-M product's weights, where every SM has one turn of features
+    or the tcgen05 product's tiles are more than the SMs."""
+    def streamed(m, hidden, inter, normed=True):
+        return rules._use_stream(m, inter, hidden, _EPI["swiglu"], normed)
+    for m in (1, 2, 8):
+        for hidden, inter in ((64, 100), (896, 4864), (1536, 8960), (2048, 14336)):
+            assert streamed(m, hidden, inter) == 1 and streamed(m, hidden, inter, False) == 0
+    for m in (9, 12, 16):
+        for normed in (True, False):
+            for hidden, inter in ((896, 4864), (1536, 8960), (1024, 4224), (1024, 3072), (1024, 9472), (1024, 18945), (1024, 28416)):
+                assert streamed(m, hidden, inter, normed) == 1, (m, hidden, inter)
+            for hidden, inter in ((1024, 2816), (512, 2048), (2048, 1024), (1024, 9473), (1024, 18944), (3584, 18944), (1024, 28417)):
+                assert streamed(m, hidden, inter, normed) == 0, (m, hidden, inter)
+    assert streamed(17, 896, 4864) == 0 and streamed(8, 900, 4864) == 0
+    assert [streamed(m, 3584, 18944) for m in (1, 6, 7, 8)] == [1, 1, 0, 0]         # several turns: the activations take the ring's room
+    assert [streamed(m, 2048, 22528) for m in (12, 13, 16)] == [1, 0, 0]
+    rules.options = dataclasses.replace(rules.options, gemm_route="stream")
+    assert streamed(16, 512, 2048, False) == 1
+    for change in (dict(gemm_route="tc"), dict(gemm_route="smallm"), dict(gemm_route=None, tc_token_tile=16), dict(gemm_route=None, smallm_cross=2)):
+        rules.options = dataclasses.replace(rules.options, **change)
+        assert streamed(4, 896, 4864) == 0

@@ -1129,13 +1129,14 @@ def test_sampling_from_gathered_elements_and_without(K):
 @pytest.mark.parametrize("m", [17, 64, 128, 600])
 def test_a_product_with_a_matrix_that_the_product_before_it_writes(K, m):
     """Without the promise that no kernel writes its matrix, a product reads it behind the kernels before it. (Small whole numbers: exact sums.)"""
-    n, k, inner = 2048, 1024, 256
+    n, k, inner = 8192, 1024, 256           # (12 tokens, gated, of so many weights: the streamed product)
     small = lambda shape, seed: torch.randint(-1, 2, shape, generator=torch.Generator().manual_seed(seed)).to(torch.bfloat16).cuda()      # noqa: E731
     left, right, a = small((n, inner), 1), small((k, inner), 2), small((m, k), 3)
     want_w = (left.float() @ right.float().t()).to(torch.bfloat16)
     want = (a.double() @ want_w.double().t()).float()
     want_glu = torch.empty(12, n // 2, dtype=torch.bfloat16, device="cuda")
     REF.linear_swiglu(a[:12].contiguous(), want_w, want_glu)
+    assert K._use_stream(12, n // 2, k, 3, False) == 1
     for turn in range(4):
         w, out = torch.zeros(n, k, dtype=torch.bfloat16, device="cuda"), torch.empty(m, n, device="cuda")
         torch.cuda.synchronize()
@@ -1145,5 +1146,5 @@ def test_a_product_with_a_matrix_that_the_product_before_it_writes(K, m):
         w, glu = torch.zeros(n, k, dtype=torch.bfloat16, device="cuda"), torch.empty(12, n // 2, dtype=torch.bfloat16, device="cuda")
         torch.cuda.synchronize()
         K.linear(left, right, None, w, "store")
-        K.linear_swiglu(a[:12], w, glu)           # the streamed product
+        K.linear_swiglu(a[:12], w, glu)
         assert_close(glu, want_glu, torch.bfloat16, "gated, of a written matrix")
