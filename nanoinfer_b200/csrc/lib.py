@@ -372,9 +372,10 @@ class Kernels:
         what the activations leave of the shared memory: from 24,576 of them on they lose (16 tokens, 2,048 x 22,528 55.5 / 59.7; 8 tokens, 3,584 x
         18,944 72.4 / 73.3; 12 tokens, 2,048 x 22,528 55.3 / 51.8).
 
-        The down projection wins for one
-        token while a CTA of eight that share K holds its weights whole (498 / 474; two tokens 507 / 503, 8 at 4,096 640 / 661; 1.5B, one
-        token 1,005 / 1,094)."""
+        The down projection wins for one token while a CTA of eight that share K holds its weights whole, which is one chunk of at most 64
+        features in 100 KB (a step 498 / 474; two tokens 507 / 503, 8 at 4,096 640 / 661; 1.5B, one token 1,005 / 1,094. A layer: 896 x 4,864 8.8 /
+        8.5, 1,024 x 5,632 10.3 / 9.6, 1,152 x 5,632 11.9 / 11.2; not whole, 1,024 x 8,192 12.4 / 13.4; two chunks, 1,280 x 5,120 12.9 / 15.2, 1,536 x
+        2,560 9.0 / 9.4, 2,048 x 2,304 9.5 / 9.4)."""
         o = self.options
         if o.gemm_route not in (None, "stream") or o.tc_token_tile or o.tc_splits or o.smallm_ksplit or o.smallm_cross or m > 16 or k % 64:
             return 0
@@ -389,7 +390,9 @@ class Kernels:
             return 0
         if o.gemm_route == "stream":
             return 8 if k > 2048 else 1
-        return 8 if m == 1 and 2048 < k <= 8192 and 2 * n * k <= 9 << 20 else 0
+        share = max(1, self.sm_count // 8)          # CTAs along n
+        rows, blocks = -(-n // share), -(-k // 512)
+        return 8 if m == 1 and 2048 < k <= 8192 and rows <= 64 and (rows + 1) * blocks * 128 <= 92 << 10 else 0
 
     def _streamed(self, splits, a, lazy, w, bias32, out, m, n, k, epi, glu) -> bool:
         """The streamed product if it takes these operands. From 9 tokens on every CTA's reading the 32-bit stream for the norm costs more

@@ -208,3 +208,13 @@ def test_gated_products_of_up_to_16_tokens(rules):
     for change in (dict(gemm_route="tc"), dict(gemm_route="smallm"), dict(gemm_route=None, tc_token_tile=16), dict(gemm_route=None, smallm_cross=2)):
         rules.options = dataclasses.replace(rules.options, **change)
         assert streamed(4, 896, 4864) == 0
+
+
+def test_the_down_projection_of_one_token(rules):
+    """Streamed while a CTA of eight that share K holds its weights whole: one chunk of features, within a CTA's room."""
+    def streamed(m, hidden, inter):
+        return rules._use_stream(m, hidden, inter, _EPI["add"], False)
+    for hidden, inter in ((896, 4864), (512, 8192), (1024, 4224), (1024, 5632), (1152, 5632)):
+        assert streamed(1, hidden, inter) == 8 and streamed(2, hidden, inter) == 0
+    for hidden, inter in ((1536, 8960), (3584, 18944), (1024, 8192), (1153, 3584), (1536, 2560), (2048, 2304), (896, 2048), (256, 16384), (896, 4900)):
+        assert streamed(1, hidden, inter) == 0, (hidden, inter)

@@ -26,8 +26,9 @@ def rnd(shape, seed, scale=1.0, dtype=BF16):
     return x
 
 
-# features an SM: 1, 7 (a tile of its own), 17, 34 (an odd tile over the halves), 64, and 65 (two chunks of 33)
-@pytest.mark.parametrize("n,k", [(5, 64), (896, 4864), (1000, 192), (2500, 1536), (4900, 320), (9472, 128), (9500, 704)])
+# features an SM: 1, 7 (a tile of its own), 17, 34 (an odd tile over the halves), 64, and 65 (two chunks of 33). From 2,048 k on eight CTAs
+# share them: 50 and 64 features each, held whole; two chunks through the ring; the same with a last stretch of k that is shorter
+@pytest.mark.parametrize("n,k", [(5, 64), (896, 4864), (1152, 5632), (1536, 2560), (2048, 2304), (1000, 192), (2500, 1536), (4900, 320), (9472, 128), (9500, 704)])
 @pytest.mark.parametrize("m", [1, 3, 8, 9, 16])
 def test_streamed_sum(K, m, n, k):
     a, w, bias = rnd((m, k), 1), rnd((n, k), 2, k ** -0.5), rnd((n,), 3, dtype=torch.float32)
