@@ -73,6 +73,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_w, const StreamArgs p
     constexpr bool TWO = epi_dual(EPI);
     constexpr int HALVES = WARPS / KG, TT = TW * HALVES, TOK = NT * 8;               // row tiles of a chunk
     static_assert(TWO ? KG == 4 : EPI == EPI_ADD && !NORM, "gated, half of the warps on the gate rows and half on the up rows, or a sum");
+    static_assert(!NORM || NT == 1, "from 9 tokens on the norm is a kernel of its own");
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* a_s = smem + (size_t)p.stages * p.w_stage;               // [tokens][a_pitch]
@@ -446,8 +447,7 @@ int launch_plan(const Plan& plan, const void* W, const StreamArgs& p, int grid, 
 template <int EPI>
 int launch_epi(const Plan& plan, const void* W, const StreamArgs& p, int grid, cudaStream_t stream) {
     if constexpr (epi_dual(EPI)) {
-        if (p.gain != nullptr)
-            return p.tokens <= 8 ? launch_plan<1, EPI, true>(plan, W, p, grid, stream) : launch_plan<2, EPI, true>(plan, W, p, grid, stream);
+        if (p.gain != nullptr) return launch_plan<1, EPI, true>(plan, W, p, grid, stream);
     }
     return p.tokens <= 8 ? launch_plan<1, EPI, false>(plan, W, p, grid, stream) : launch_plan<2, EPI, false>(plan, W, p, grid, stream);
 }
@@ -471,7 +471,7 @@ NIB_API int nib_gemm_stream_error() {
     return v;
 }
 
-// Operands as nib_gemm_smallm, the gated epilogues (with a norm before them if ``gain`` is there) and EPI_ADD. ``splits``: CTAs that share
+// Operands as nib_gemm_smallm, the gated epilogues (with a norm of up to 8 tokens before them if ``gain`` is there) and EPI_ADD. ``splits``: CTAs that share
 // K (EPI_ADD only: their sums meet in memory, in any order).
 NIB_API int nib_gemm_stream(const void* A, const void* W, const float* bias, void* out, int tokens, int N, int K, int lda, int ldo, int epi,
                             int splits, const float* gain, float eps, const NibGlu* glu, cudaStream_t stream) {
@@ -480,7 +480,8 @@ NIB_API int nib_gemm_stream(const void* A, const void* W, const float* bias, voi
     NIB_REQUIRE(!epi_dual(epi) || bias == nullptr, "gemm (streamed): the gated epilogues take no bias");
     NIB_REQUIRE(epi != EPI_GLU || glu != nullptr, "gemm (streamed): the gated epilogue needs its constants");
     NIB_REQUIRE(splits == 1 || epi == EPI_ADD, "gemm (streamed): only sums are split along K");
-    NIB_REQUIRE(gain == nullptr || (((uintptr_t)gain & 15) == 0 && epi_dual(epi)), "gemm (streamed): no norm before this epilogue, or a gain that is not 16-byte aligned");
+    NIB_REQUIRE(gain == nullptr || (((uintptr_t)gain & 15) == 0 && epi_dual(epi) && tokens <= 8),
+                "gemm (streamed): no norm before this epilogue or %d tokens, or a gain that is not 16-byte aligned", tokens);
     const int sms = nib_sm_count();
     NIB_REQUIRE(sms > 0 && splits <= sms, "gemm (streamed): no device, or too many splits");
     const Plan plan = plan_of(N, K / 64, epi_dual(epi), splits, sms);
