@@ -137,8 +137,9 @@ class Kernels:
                      "nib_rmsnorm_add", "nib_moe_route", "nib_moe_max_tiles", "nib_moe_group", "nib_moe_gemm_simt", "nib_moe_combine",
                      "nib_moe_tc_supported", "nib_moe_tc_error", "nib_moe_gather_rows", "nib_moe_gemm_tc", "nib_moe_step", "nib_moe_step_supported", "nib_moe_identity", "nib_stream_mix", "nib_grouped_state_scan", "nib_grouped_state_error", "nib_pdl_skip_next", "nib_memory_gates", "nib_layernorm",
                      "nib_decay_state_scan", "nib_decay_state_chunks_supported",
-                     "nib_gemm_stream", "nib_gemm_stream_supported", "nib_gemm_stream_error", "nib_sample_rows"):
+                     "nib_gemm_stream", "nib_gemm_stream_supported", "nib_gemm_stream_error", "nib_sample_rows", "nib_sample_rows_most"):
             getattr(self._lib, name).restype = c_int
+        self.sample_rows_most = int(self._lib.nib_sample_rows_most())      # rows whose parameters a launch takes by value
         self._lib.nib_grouped_state_scratch.restype = self._lib.nib_decay_state_scratch.restype = c_longlong
 
     # ---- plumbing ---------------------------------------------------------------------------
@@ -1694,8 +1695,6 @@ class Kernels:
         rows, vocab = logits.shape
         self._check(self._lib.nib_sample(_ptr(logits), c_int(rows), c_int(vocab), _ptr(temperature), _ptr(top_k),
                                          _ptr(top_p), _ptr(uniform), _ptr(out), self._stream()), "sample")
-
-    sample_rows_most = 64       # rows whose parameters a launch takes by value
 
     def sample_rows(self, logits, rows, out):
         """The same for up to ``sample_rows_most`` rows of (temperature, top_k, top_p, first, seed, counter), numbers of the host
