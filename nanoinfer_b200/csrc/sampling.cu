@@ -573,7 +573,11 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
         const unsigned long long limit = (unsigned long long)((double)tp * (double)FIX_ONE);
         unsigned prefix = 0u;
         unsigned long long above0 = 0ull;
-        const auto mass_of = [&](float x) { return (unsigned long long)(weight(x - mx) * fix_over_z); };
+        // (nothing for an undefined value: the histograms hold 42 bits of a mass, and a NaN's 2^63 is none of them)
+        const auto mass_of = [&](float x) {
+            const float m = weight(x - mx) * fix_over_z;
+            return m > 0.f ? (unsigned long long)m : 0ull;
+        };
         const auto choose = [&]() {
             // the lowest non-empty bin whose "mass above" (the bins above it, and what earlier passes left
             // above) is still within the limit; the very first (largest) element always stays, so if even

@@ -1148,3 +1148,37 @@ def test_a_product_with_a_matrix_that_the_product_before_it_writes(K, m):
         K.linear(left, right, None, w, "store")
         K.linear_swiglu(a[:12], w, glu)
         assert_close(glu, want_glu, torch.bfloat16, "gated, of a written matrix")
+
+
+def test_sampling_of_rows_with_undefined_and_infinite_logits(K):
+    """The select over a list and the one without take the same token of a row that holds NaN or infinities; all in range."""
+    vocab = 20000
+    base = 2.0 * torch.randn(16, vocab, generator=torch.Generator().manual_seed(9))
+    nan, inf = float("nan"), float("inf")
+    minus = torch.tensor([-1], dtype=torch.int32).view(torch.float32)[0]        # a NaN whose sign is set
+    base[0, 77] = nan
+    base[1, 78] = minus
+    base[2, 5] = inf
+    base[3, [9, 15000]] = inf
+    base[4, ::2] = nan
+    base[5, 1::2] = minus
+    base[6] = nan
+    base[7] = minus
+    base[8] = -inf
+    base[9, 3], base[9, 4], base[9, 5] = nan, minus, inf
+    base[10, :19000] = -inf
+    base[11, 40], base[11, 41:] = minus, -inf
+    base[12, 100:2000] = nan
+    base[13, 100:2000] = inf
+    base[14, 100:2000] = minus
+    rows = base.repeat(3, 1).cuda().contiguous()
+    n = rows.shape[0]
+    for top_k, top_p in ((0, 0.9), (0, 1.0), (0, 0.0), (40, 0.9), (40, 1.0), (5000, 0.8), (19999, 0.999)):
+        par = [torch.full((n,), v, dtype=t, device="cuda") for v, t in ((0.8, torch.float32), (top_k, torch.int32), (top_p, torch.float32))]
+        uniform = torch.tensor([(0.37 * i) % 1.0 for i in range(n)], device="cuda")
+        many, few = (torch.empty(n, dtype=torch.int32, device="cuda") for _ in range(2))
+        K.sample(rows, *par, uniform, many)
+        for r in range(0, n, 16):
+            K.sample(rows[r:r + 16], *(p[r:r + 16].clone() for p in par), uniform[r:r + 16].clone(), few[r:r + 16])
+        assert torch.equal(many, few), (top_k, top_p, [(i % 16, a, b) for i, (a, b) in enumerate(zip(many.tolist(), few.tolist())) if a != b])
+        assert bool(((many >= 0) & (many < vocab)).all())
