@@ -213,7 +213,7 @@ class Sampler:
         for i, r in enumerate(rows):
             p = r.params
             if not p.greedy:
-                temperature[i], top_k[i], top_p[i], uniform[i] = p.temperature, p.k, p.p, uniform_for(r.seed, r.generated)
+                temperature[i], top_k[i], top_p[i], uniform[i] = p.temperature, min(p.k, 0x7FFFFFFF), p.p, uniform_for(r.seed, r.generated)
         on_gpu = torch.device(dev).type == "cuda"
         host = self._pinned_parameters(n)[:4 * n] if on_gpu else torch.empty(4 * n, dtype=torch.float32)
         par = host.numpy().reshape(4, n)

@@ -107,4 +107,7 @@ def test_parameters_by_value_are_what_the_arrays_hold():
     by_value = Sampler._row_parameters([SampleRow(SamplingParams(**k), None, 3, seed=-1) for k in kinds])
     assert [r[:3] for r in by_value] == [(1e-3, 5, 1.0), (3.3e38, 0, 1.0), (float("inf"), 0, 0.5), (float("inf"), 0, 1.0), (1.0, 1, 1.0),
                                          (1.0, 0x7FFFFFFF, 1.0), (1.0, 0, 0.0)]
+    arrays = Sampler(FakeOps(), "cpu")._device_parameters([SampleRow(SamplingParams(**k), None, 3, seed=-1) for k in kinds], "cpu")
+    for row, *par in zip(by_value, *(a.tolist() for a in arrays)):         # the same beyond the rows that go by value
+        assert torch.tensor(row[:3], dtype=torch.float32).tolist() == torch.tensor(par[:3], dtype=torch.float32).tolist()
     assert by_value[0][3:] == (0, (1 << 64) - 1, 3) and by_value[4][3:] == (1, 0, 0)
