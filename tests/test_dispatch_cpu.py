@@ -1,5 +1,5 @@
 """Which kernel a matrix product and a decode attention go to is decided on the host from sizes alone
-(``Kernels._route``, ``_use_pair``, ``decode_splits``). These rules were fitted to measurements at the
+(``Kernels._use_stream``, which is asked first up to 16 tokens, ``_route``, ``_use_pair``, ``decode_splits``). These rules were fitted to measurements at the
 projection sizes of the 0.5B, 1.5B and 7B models; the test pins them for those sizes so that a change of a
 threshold shows up as a decision that moved. No GPU and no library are needed: the rules read nothing but
 their arguments, the object's options and its count of SMs."""
@@ -36,11 +36,15 @@ def projections(shape):
     }
 
 
-def test_decode_products_of_the_small_model_stream_through_the_small_m_kernel(rules):
+def test_decode_products_of_the_small_model(rules):
+    """q/k/v and the output projection by the small-M kernel, gate/up and one token's down projection streamed; where the streamed
+    kernel refuses its operands, gate/up goes on to the small-M kernel and the down projection to the tcgen05 one."""
     p = projections("0.5b")
     for m in (1, 8):
         assert rules._route(m, *p["qkv"]) == ("smallm", True)           # the norm folded in
-        assert rules._route(m, *p["o"]) == ("smallm", False)
+        assert rules._route(m, *p["o"]) == ("smallm", False) and rules._use_stream(m, 896, 896, _EPI["add"], False) == 0
+        assert rules._use_stream(m, 4864, 896, _EPI["swiglu"], True) == 1
+        assert rules._use_stream(m, 896, 4864, _EPI["add"], False) == (8 if m == 1 else 0)
         assert rules._route(m, *p["gate_up"]) == ("smallm", False)      # wide output: the norm runs alone
         assert rules._route(m, *p["down"]) == ("tc", False)             # long K: split over CTAs on tcgen05
     assert rules._route(64, *p["qkv"]) == ("smallm", False)
@@ -50,8 +54,9 @@ def test_decode_products_of_the_small_model_stream_through_the_small_m_kernel(ru
 def test_decode_products_of_the_large_model_go_to_tcgen05_where_the_weights_are_large(rules):
     p = projections("7b")
     assert rules._route(8, *p["qkv"])[0] == "smallm"
+    assert rules._use_stream(4, 18944, 3584, _EPI["swiglu"], True) == 1 and rules._use_stream(8, 18944, 3584, _EPI["swiglu"], True) == 0
     assert rules._route(8, *p["gate_up"])[0] == "tc"
-    assert rules._route(8, *p["down"])[0] == "tc"
+    assert rules._use_stream(1, 3584, 18944, _EPI["add"], False) == 0 and rules._route(8, *p["down"])[0] == "tc"
     lm_head = (152064, 3584, _EPI["f32"], True)
     assert rules._route(1, *lm_head) == ("tc", False)
 

@@ -1182,3 +1182,32 @@ def test_sampling_of_rows_with_undefined_and_infinite_logits(K):
             K.sample(rows[r:r + 16], *(p[r:r + 16].clone() for p in par), uniform[r:r + 16].clone(), few[r:r + 16])
         assert torch.equal(many, few), (top_k, top_p, [(i % 16, a, b) for i, (a, b) in enumerate(zip(many.tolist(), few.tolist())) if a != b])
         assert bool(((many >= 0) & (many < vocab)).all())
+
+
+@pytest.mark.parametrize("seed", [0, 1, -1, -(1 << 62), (1 << 63) - 1, 1 << 63, (1 << 64) - 1, 0x9E3779B97F4A7C15])
+def test_uniform_numbers_made_on_the_device_are_the_hosts(K, seed):
+    """Of many equal logits one is drawn: which one is the uniform number times the vocabulary."""
+    from nanoinfer_b200.sampling import SampleRow, SamplingParams
+    from nanoinfer_b200.sampling.sampler import Sampler, uniform_for
+    vocab = 8192            # (sums of ones are exact)
+    counters = [0, 1, 2, 1000, (1 << 31) - 1, 1 << 31, (1 << 32) + 5, (1 << 63) - 1] + list(range(7, 63))
+    rows = [SampleRow(SamplingParams(temperature=1.0), None, c, seed=seed) for c in counters]
+    assert len(rows) == 64
+    logits = torch.zeros(65, vocab, device="cuda")
+    sampler = Sampler(K, "cuda:0")
+    want = [int(uniform_for(seed, c) * vocab) for c in counters]
+    assert sampler.sample(logits[:64].contiguous(), rows) == want                     # by value
+    assert sampler.sample(logits, rows + [rows[0]])[:64] == want                      # by arrays
+    assert sampler.sample_async(logits[:64].contiguous(), rows).wait() == want
+    out = [sampler.sample_async(logits[:8].contiguous(), rows[:8])] + [sampler.sample(logits[:3].contiguous(), rows[5 + i:8 + i]) for i in range(6)]
+    assert out[0].wait() == want[:8] and out[1:] == [want[5 + i:8 + i] for i in range(6)]
+
+
+@pytest.mark.parametrize("m", [17, 40, 48, 49, 64])
+def test_gated_products_of_17_to_64_tokens(K, m):
+    """Tiles of 16 tokens up to 48 (three by 38 feature tiles are one turn of the SMs), of 32 and 64 above; the last one ragged."""
+    a, w = rnd((m, 896), torch.bfloat16, 1), rnd((2 * 4864, 896), torch.bfloat16, 2, 896 ** -0.5)
+    out, ref = (torch.empty(m, 4864, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    K.linear_swiglu(a, w, out)
+    REF.linear_swiglu(a, w, ref)
+    assert_close(out, ref, torch.bfloat16, "gated")
