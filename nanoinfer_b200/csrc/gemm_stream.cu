@@ -1,12 +1,12 @@
-// Matrix product for a decode step of up to 16 tokens over wide weights: out[tokens, N] = A[tokens, K] . W[N, K]^T, bfloat16
-// operands, 32-bit sums. What bounds it is reading the weights once and the chain from the kernel before it to its own result.
+// Matrix product for a decode step of up to 16 tokens (whose activations are at most 64 KB) over wide weights: out[tokens, N] =
+// A[tokens, K] . W[N, K]^T, bfloat16 operands, 32-bit sums. What bounds it is reading the weights once and the chain from the kernel before it to its own result.
 //
 // One CTA an SM, every SM the same number of output features (RB = ceil(N / SMs), in several chunks where that is more than 64):
 // no last wave. (With 16 features a CTA the 4,864 features of the 0.5B widths are 304 CTAs, two an SM and eight over, and those eight
 // start when the first 296 are done.) One warp sends for the weights by tensor-map copies, BEFORE the wait for the kernel before this
 // one (they are nobody's output): all of them at once where they fit, else through a ring of stages. The copies cost no registers and
-// no issue slots of whatever runs meanwhile, and every kernel lets the next one in at its first instruction, so the weights of
-// the products that follow are on their way while a chain of small kernels waits for itself.
+// no issue slots of whatever runs meanwhile, and the kernels before this one (attention, output projection) let the next one in at their
+// first instruction, so the weights of the products that follow are on their way while a chain of small kernels waits for itself.
 //
 // Behind the wait a CTA reads all activations into shared memory, warp w the w-th eighth of every token, and where a norm stands
 // before the product it computes that itself: bfloat16(x * gain) as the operand, the sum of x^2 beside it, and 1 / sqrt(mean(x^2)

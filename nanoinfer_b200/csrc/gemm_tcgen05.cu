@@ -277,8 +277,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     __syncthreads();
     tc_fence_after();
     const unsigned tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
-    // The weights of the first item's stages are sent for before the wait: no kernel writes them, and this CTA is here only since
-    // nobody else's shared memory is in its way.
+    // The weights of the first item's stages are sent for before the wait: no kernel writes them (what the host promises, or the launch is
+    // a plain one), and this CTA is here only since nobody else's shared memory is in its way. Four layers of the 7B widths, us without /
+    // with: 24 decoded tokens 705 / 685, a prompt of 64 741 / 721, 100 729 / 716, 200 979 / 967.
     const auto send_w = [&](int s, int kb, int f0) {
         unsigned char* st = smem + s * C::STAGE_BYTES;
         mbar_expect_tx(&full_bar[s], C::STAGE_BYTES);
@@ -937,8 +938,11 @@ NIB_API int nib_gemm_tc_splitk(const void* A, const void* W, const float* bias, 
         if (tok_tile == 64 && 2LL * f_tiles <= sm_count() && (epi != EPI_ADD || 2LL * N * K <= (16LL << 20))) tok_tile = 32;
         // The gated product's feature tiles are twice as many rows: tiles of 16 tokens while they are one turn of the SMs and the
         // weights are few, so that a tile's weights read once more come from L2 (us alone, by 32 and by 16: 4,864 x 896, 24 tokens 8.1 and
-        // 7.6, 40 8.7 and 7.8; 64 would be two turns, 8.7 and 11.6; 8,960 x 1,536, 24 tokens 13.3 and 14.6).
-        const long long sixteens = (long long)f_tiles * ceil_div(tokens, 16);      // (so many that K is not split besides)
+        // 7.6, 40 8.7 and 7.8; 64 would be two turns, 8.7 and 11.6; 8,960 x 1,536, 24 tokens 13.3 and 14.6). Tiles that are at most half
+        // of the SMs leave it to K: split among CTAs with tiles of 32 it uses the SMs too and reads the weights once (a feed-forward's
+        // layer by 32 and by 16, 17 and 32 tokens: 4,224 x 1,024 12.9 and 14.3, 14.1 and 14.7; 4,736 x 896 12.5 and 14.0, 13.6 and 15.2; one
+        // feature tile more is the other way round, 4,864 x 896 12.8 and 12.6, 13.8 and 13.0).
+        const long long sixteens = (long long)f_tiles * ceil_div(tokens, 16);
         if (epi_dual(epi) && tokens > 16 && tokens <= 64 && sixteens <= sm_count() && 2 * sixteens > sm_count() && 4LL * N * K <= (32LL << 20)) tok_tile = 16;
     }
     NIB_REQUIRE(ceil_div(tokens, tok_tile) <= 65535, "gemm (tensor cores): too many token tiles");

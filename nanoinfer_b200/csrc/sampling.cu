@@ -4,9 +4,9 @@
 // repetition penalty on the raw logits -> greedy (first index of the maximum) when temperature is 0
 // -> logits / temperature -> top-k (ties at the k-th value stay) -> top-p (a token is dropped iff the
 // probability of those before it, in descending order, exceeds p; the first stays) -> softmax ->
-// draw. The draw is an inverse CDF in vocabulary order with a uniform number that the host derives
-// from (seed, number of tokens generated), so a request's tokens do not depend on the batch it
-// was sampled in. The reference samples on the host (cpp/python/ni/scheduler.py:89-147).
+// draw. The draw is an inverse CDF in vocabulary order with a uniform number made from (seed, number of
+// tokens generated), here up to 64 rows and by the host beyond, the same one: a request's tokens do not depend on
+// the batch it was sampled in. The reference samples on the host (cpp/python/ni/scheduler.py:89-147).
 #include "pipeline.cuh"
 
 // ---------------------------------------------------------------------------------- penalty
@@ -844,10 +844,10 @@ static int launch_sample(const float* logits, int rows, int vocab, const float* 
     const int per = (ceil_div(vocab, CS * ST) + 3) & ~3;
     // Up to 32 rows all CTAs are at work at once, two an SM, and a row's time is what counts: 512 threads, and the slice kept in
     // shared memory if two of them fit an SM's (else for the 12 rows that one an SM holds). More rows: as many CTAs an SM as there can
-    // be (five), and the slice kept only where it is small. Measured with another top-p select, at a vocabulary of 151,936, top-p 0.9, us: 1 row 47 (68 with 256
-    // threads and nothing kept), 12 rows 49 (70), 16 rows 64 (82; 93 with one CTA an SM), 32 rows 69 (85; 143), 34 rows 97 (with 512
-    // threads, which are two turns then, 99), 64 rows 122 (131); 32,000: 34 rows 35 (51 with 512 threads), 64 rows 41 (64; 53 with
-    // nothing kept).
+    // be (five), and the slice kept only where it is small. Measured, us with 512 / 256 threads, at a vocabulary of 151,936: top-p 0.9, 1 row
+    // 38 / 68, 12 rows 46 / 75, 16 51 / 86, 32 58 / 90; top-k 40, 32 rows 35 / 52; neither, 30 / 33. From 34 rows on 512 threads are two turns: 34
+    // rows, top-p 80 / 104, top-k 52 / 55, neither 41 / 33; 64 rows 110 / 131, 65 / 67, 54 / 41; at 32,000, 34 rows 39 / 37, 31 / 22, 21 / 14, 64 rows 49 /
+    // 44, 37 / 25, 25 / 15 (one kernel takes all rows of a call, whatever each asks for).
     const size_t slice = sizeof(float) * (size_t)ST * per;
     const auto room = [&](int copies) { return sizeof(unsigned) * 4 * copies * BINS + slice; };
     const bool wide = rows <= 32;
